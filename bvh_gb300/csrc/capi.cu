@@ -52,6 +52,7 @@ struct bvh_ctx {
   void* eval_buf = nullptr;               // bvh_evaluate scratch
   size_t eval_bytes = 0;
   void* heat_buf = nullptr;               // bvh_heatmap scratch (heatmap_scratch_bytes())
+  TracePool trace_pool;                   // the packed traversal's records
   StageEvents evs;
   bvh_timing last{};
   int last_algo = -1;
@@ -107,6 +108,7 @@ extern "C" bvh_status bvh_ctx_create(bvh_ctx** out, int device) {
   bvh_ctx* c = new (std::nothrow) bvh_ctx();
   if (!c) return BVH_ERR_OUT_OF_MEMORY;
   c->device = device;
+  c->trace_pool.device = device;
   for (int k = 0; k < 8; ++k)
     if (cudaEventCreate(&c->evs.ev[k]) != cudaSuccess) { delete c; return BVH_ERR_DEVICE; }
   c->evs.use = true;
@@ -132,6 +134,7 @@ extern "C" bvh_status bvh_ctx_destroy(bvh_ctx* ctx) {
   workspace_free(ctx->ws);
   cudaFree(ctx->eval_buf);
   cudaFree(ctx->heat_buf);
+  trace_pool_free(ctx->trace_pool);
   for (int k = 0; k < 8; ++k) cudaEventDestroy(ctx->evs.ev[k]);
   cudaFreeHost(ctx->h_status);
   cudaFree(ctx->hash_buf);
@@ -910,7 +913,7 @@ extern "C" bvh_status bvh_trace(bvh_ctx* ctx, const bvh_node* nodes, uint32_t n_
   rp.d[0] = rays->dx; rp.d[1] = rays->dy; rp.d[2] = rays->dz;
   HitOut ho{hits->t, hits->prim, hits->nodes_visited, hits->aabb_tests, hits->tri_tests};
   return from_cuda(trace_rays(reinterpret_cast<const Node*>(nodes), (int)n_nodes, mesh_ptrs(mesh), mesh->n, rp,
-                              rays->n, ho, reinterpret_cast<cudaStream_t>(stream)));
+                              rays->n, ho, &ctx->trace_pool, reinterpret_cast<cudaStream_t>(stream)));
 }
 
 // The camera as the kernels take it; generateRay's basis is derived on the device, per ray.
@@ -936,7 +939,7 @@ extern "C" bvh_status bvh_trace_pinhole(bvh_ctx* ctx, const bvh_node* nodes, uin
   cudaSetDevice(ctx->device);
   HitOut ho{hits->t, hits->prim, hits->nodes_visited, hits->aabb_tests, hits->tri_tests};
   return from_cuda(trace_pinhole(reinterpret_cast<const Node*>(nodes), (int)n_nodes, mesh_ptrs(mesh), mesh->n, b, ho,
-                                 reinterpret_cast<cudaStream_t>(stream)));
+                                 &ctx->trace_pool, reinterpret_cast<cudaStream_t>(stream)));
 }
 
 extern "C" bvh_status bvh_pinhole_rays(const bvh_camera* cam, int32_t width, int32_t height, float* ox, float* oy,

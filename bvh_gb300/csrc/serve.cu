@@ -234,7 +234,7 @@ static cudaError_t launch_one(bvh_server* sv, Slot& s) {
   float* ht = reinterpret_cast<float*>(s.hits);
   int32_t* hi = reinterpret_cast<int32_t*>(s.hits);
   HitOut ho{ht, hi + s.ray_cap, hi + 2 * s.ray_cap, hi + 3 * s.ray_cap, hi + 4 * s.ray_cap};
-  if ((e = trace_rays(s.ws.nodes, (int)(2 * n - 1), m, n, rp, nr, ho, s.stream)) != cudaSuccess) return e;
+  if ((e = trace_rays(s.ws.nodes, (int)(2 * n - 1), m, n, rp, nr, ho, nullptr, s.stream)) != cudaSuccess) return e;
   void* dst[5] = {r.hits.t, r.hits.prim, r.hits.nodes_visited, r.hits.aabb_tests, r.hits.tri_tests};
   for (int k = 0; k < 5; ++k)
     if (nr && dst[k] &&

@@ -33,8 +33,18 @@ struct ShadeIn {
   const int32_t* vis;
 };
 
+// Stream-ordered scratch of the packed traversal (see trace.cu): a pool of the context's own, made at
+// its first use, which keeps at most one trace's records between calls.
+struct TracePool {
+  int device = 0;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = 0;  // the pool's release threshold: the largest trace so far
+};
+void trace_pool_free(TracePool& p);
+
+// `pool` (may be NULL) lets a trace of enough rays repack the tree first; the hits are the same.
 cudaError_t trace_rays(const Node* nodes, int n_nodes, const MeshPtrs& m, uint32_t n_tris, const RayPtrs& rays,
-                       uint32_t nr, const HitOut& out, cudaStream_t st);
+                       uint32_t nr, const HitOut& out, TracePool* pool, cudaStream_t st);
 
 // Rays of many requests traced in one launch against a batched build (each request's tree at
 // node_base, its triangles at tri_base of the concatenated mesh, child and primitive indices
@@ -59,7 +69,7 @@ struct CopyDesc {
 inline uint32_t copy_pieces(uint32_t n) { return (n + kCopyPiece - 1) / kCopyPiece; }
 cudaError_t copy_many(const CopyDesc* d_descs, uint32_t count, uint32_t total_pieces, cudaStream_t st);
 cudaError_t trace_pinhole(const Node* nodes, int n_nodes, const MeshPtrs& m, uint32_t n_tris, const PinholeCam& cam,
-                          const HitOut& out, cudaStream_t st);
+                          const HitOut& out, TracePool* pool, cudaStream_t st);
 cudaError_t pinhole_rays(const PinholeCam& cam, float* ox, float* oy, float* oz, float* dx, float* dy, float* dz,
                          cudaStream_t st);
 // kRenderKernel's shading of traced pinhole pixels (mode 0 normal, 1 depth, 2 diffuse, 3 visits).
