@@ -21,6 +21,12 @@ namespace bvhgb {
 
 constexpr int kTlMax = 7;
 constexpr float kTlInf = 1e30f;
+// Minimum of three; as fminf, a NaN operand never wins.
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 }  // namespace bvhgb
 #include "treelet_dp_unrolled.cuh"
 namespace bvhgb {
@@ -248,7 +254,7 @@ __device__ void treelet_rebuild(Node* nodes, int32_t root, LaneTreelet& T) {
 // key bits plus 32) fall back to the climb-ordered kernel above.
 // ---------------------------------------------------------------------------------------
 constexpr int kTlMaxHeight = 254;
-constexpr int kLvThreads = 32;  // one warp per block; its DP tables are 20 KB of shared memory
+constexpr int kLvThreads = 32;  // one warp per block; its DP table is 16 KB of shared memory
 
 // A lane's treelet in registers (all indexing below is unrolled to constant indices).
 struct RegTreelet {
@@ -402,13 +408,32 @@ __device__ __forceinline__ void reg_areas(const RegTreelet& T, int nv, float* A)
 }
 
 // Subset DP (:119-165) by one lane for up to nv leaves, straight-line code with the costs in
-// registers (treelet_dp_unrolled.cuh); best splits into this lane's column P.
+// registers (treelet_dp_unrolled.cuh); this lane's column C holds the areas and receives the costs.
+// Costs only, the splits looked up afterwards for the subsets that the rebuild visits: the 10M pass's
+// heights from 4 on 2.53 -> 1.99 ms, three passes 21.1 -> 19.0 ms (carrying every subset's split
+// took 4 operations per split in a serial chain and a store per subset).
+// *of: the leaf count whose full set's best split is returned.
 template <int NVMAX = kTlMax>
-__device__ __forceinline__ void reg_dp(int nv, const float* A, uint8_t* P) {
-  if (NVMAX <= 4 || nv <= 4) dp_unrolled_4(A, P);
-  else if (NVMAX <= 5 || nv == 5) dp_unrolled_5(A, P);
-  else if (NVMAX <= 6 || nv == 6) dp_unrolled_6(A, P);
-  else dp_unrolled_7(A, P);
+__device__ __forceinline__ uint32_t reg_dp(int nv, float* C, int* of) {
+  *of = std::min(NVMAX, std::max(nv, 4));
+  if (NVMAX <= 4 || nv <= 4) return dp_unrolled_4(C);
+  if (NVMAX <= 5 || nv == 5) return dp_unrolled_5(C);
+  if (NVMAX <= 6 || nv == 6) return dp_unrolled_6(C);
+  return dp_unrolled_7(C);
+}
+
+// The best split of `mask` from the costs in this lane's column: the first minimum over the nonempty
+// subsets of mask without its lowest member in increasing order; 0 where no split is finite.
+__device__ __forceinline__ uint32_t best_split(const float* C, uint32_t mask) {
+  const uint32_t delta = mask & (mask - 1u);
+  uint32_t p = delta & (0u - delta), bp = 0u;
+  float b = kTlInf;
+  do {
+    const float v = __fadd_rn(C[p * 32u], C[(mask ^ p) * 32u]);
+    if (v < b) { b = v; bp = p; }
+    p = (p - delta) & delta;
+  } while (p);
+  return bp;
 }
 
 // Id reuse (:167-191): the treelet's internal nodes in DFS order from the root, right child
@@ -444,46 +469,51 @@ __device__ __forceinline__ int reg_avail(const Node* nodes, int32_t root, const 
   return n_avail;
 }
 
-// Rebuild (:194-246) from the partitions P (this lane's column, stride 32), breadth-first,
-// handing out the reused ids in order.  A subset with no finite split (NaN areas) leaves the
-// treelet unchanged.
-template <int PSTRIDE>
-__device__ __forceinline__ void reg_build(Node* nodes, const RegTreelet& T, const uint8_t* P, const int* avail,
-                                          int n_avail) {
+// Rebuild (:194-246) breadth-first, handing out the reused ids in order: the j-th subset of the queue
+// gets the j-th id.  split(mask): the best split of a subset.  A subset with no finite split (NaN
+// areas) leaves the treelet unchanged.  The queues are bytes of 64-bit words, so nothing is indexed
+// through local memory.
+template <typename Split>
+__device__ __forceinline__ void reg_build(Node* nodes, const RegTreelet& T, Split split, const int* avail, int n_avail) {
   const int n = T.n;
-  const uint32_t full = (1u << n) - 1u;
-  {
-    int vm[kTlMax], vh = 0, vt = 0;
-    vm[vt++] = (int)full;
-    while (vh < vt) {
-      const int mask = vm[vh++];
-      const int lm = P[mask * PSTRIDE], rm = mask ^ lm;
-      if (lm == 0 || rm == 0 || (lm & ~mask)) return;
-      if (__popc(lm) > 1) { if (vt >= kTlMax) return; vm[vt++] = lm; }
-      if (__popc(rm) > 1) { if (vt >= kTlMax) return; vm[vt++] = rm; }
-    }
-    if (n_avail != n - 1) return;
+  if (n_avail != n - 1) return;
+  unsigned long long masks = (1u << n) - 1u, lefts = 0;
+  int qt = 1;
+#pragma unroll
+  for (int j = 0; j < kTlMax - 1; ++j) {
+    if (j >= n - 1) break;
+    const uint32_t mask = (uint32_t)(masks >> (8 * j)) & 255u;
+    const uint32_t lm = split(mask), rm = mask ^ lm;
+    if (lm == 0 || rm == 0 || (lm & ~mask)) return;
+    lefts |= (unsigned long long)lm << (8 * j);
+    if (__popc(lm) > 1) masks |= (unsigned long long)lm << (8 * qt++);
+    if (__popc(rm) > 1) masks |= (unsigned long long)rm << (8 * qt++);
   }
-  int qm[kTlMax], qn[kTlMax];
-  int qh = 0, qt = 0, used = 1;
-  qm[qt] = (int)full;
-  qn[qt++] = avail[0];
-  while (qh < qt) {
-    const int mask = qm[qh], cur = qn[qh];
-    qh++;
-    const int lm = P[mask * PSTRIDE], rm = mask ^ lm;
-    int li, ri;
-    if (__popc(lm) == 1) li = reg_id(T, __ffs(lm) - 1);
-    else { li = avail[used++]; qm[qt] = lm; qn[qt++] = li; }
-    if (__popc(rm) == 1) ri = reg_id(T, __ffs(rm) - 1);
-    else { ri = avail[used++]; qm[qt] = rm; qn[qt++] = ri; }
-    const Box b = reg_union(T, (uint32_t)mask);
+  int used = 1;
+#pragma unroll
+  for (int j = 0; j < kTlMax - 1; ++j) {
+    if (j >= n - 1) break;
+    const uint32_t mask = (uint32_t)(masks >> (8 * j)) & 255u, lm = (uint32_t)(lefts >> (8 * j)) & 255u;
+    const int cur = avail[j];
+    int child[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const uint32_t cm = s ? mask ^ lm : lm;
+      child[s] = reg_id(T, __ffs(cm) - 1);
+      if (__popc(cm) > 1) {
+#pragma unroll
+        for (int k = 1; k < kTlMax - 1; ++k)
+          if (k == used) child[s] = avail[k];
+        used++;
+      }
+    }
+    const Box b = reg_union(T, mask);
     float4* p = reinterpret_cast<float4*>(nodes + cur);
     __stcg(p, b.lo);
     __stcg(p + 1, b.hi);
-    __stcg(reinterpret_cast<int2*>(&nodes[cur].left), make_int2(li, ri));
-    __stcg(&nodes[li].aux0, cur);
-    __stcg(&nodes[ri].aux0, cur);
+    __stcg(reinterpret_cast<int2*>(&nodes[cur].left), make_int2(child[0], child[1]));
+    __stcg(&nodes[child[0]].aux0, cur);
+    __stcg(&nodes[child[1]].aux0, cur);
   }
 }
 
@@ -632,12 +662,12 @@ __global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(Node* __restrict__ 
 }
 
 // One lane's treelet q of the current height (act: a real one): leaf ids and boxes from its
-// descriptor and the nodes, subset areas and the DP in this lane's shared-memory columns C and
-// P (stride 32), then the rebuild.  The warp runs the DP variant of its largest treelet, at most
+// descriptor and the nodes, subset areas and the DP in this lane's shared-memory column C
+// (stride 32), then the rebuild.  The warp runs the DP variant of its largest treelet, at most
 // NVMAX leaves.  Called by all 32 lanes together.
 template <int NVMAX>
 __device__ __forceinline__ void lane_dp(Node* nodes, const uint32_t* desc, uint32_t stride, uint32_t q, bool act,
-                                        float* C, uint8_t* P) {
+                                        float* C) {
   const uint32_t w0 = act ? __ldcg(desc + q) : 0u;
   RegTreelet T;
   T.n = (int)(w0 & 255u);
@@ -650,12 +680,14 @@ __device__ __forceinline__ void lane_dp(Node* nodes, const uint32_t* desc, uint3
   const int nv = (int)__reduce_max_sync(0xffffffffu, (uint32_t)T.n);
   if (nv < 2) return;
   reg_areas<NVMAX>(T, nv, C);
-  reg_dp<NVMAX>(nv, C, P);
+  int of;
+  const uint32_t top = reg_dp<NVMAX>(nv, C, &of);
   if (T.n >= 2) {
     int avail[kTlMax];
 #pragma unroll
     for (int i = 0; i < kTlMax - 1; ++i) avail[i] = (int)__ldcg(desc + (size_t)(8 + i) * stride + q);
-    reg_build<32>(nodes, T, P, avail, na);
+    const uint32_t full = (1u << of) - 1u;
+    reg_build(nodes, T, [&](uint32_t mask) { return mask == full ? top : best_split(C, mask); }, avail, na);
   }
 }
 
@@ -665,9 +697,8 @@ template <int NVMAX>
 __global__ void __launch_bounds__(kLvThreads) k_tl_dp(Node* __restrict__ nodes, const uint32_t* __restrict__ off,
                                                       const uint32_t* __restrict__ ctl,
                                                       const uint32_t* __restrict__ desc, uint32_t stride) {
-  // per-lane columns of 2^NVMAX costs and partitions (the narrow path below uses 768 words)
+  // per-lane columns of 2^NVMAX areas, then costs (the narrow path below uses 768 words)
   __shared__ float s_cost[std::max((1 << NVMAX) * 32, 1024)];
-  __shared__ uint8_t s_part[(1 << NVMAX) * 32];
   if (__ldcg(ctl) != 0u) return;
   const uint32_t h = __ldcg(ctl + 2);
   const uint32_t b = __ldcg(off + h), e = __ldcg(off + h + 1);
@@ -703,18 +734,17 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dp(Node* __restrict__ nodes, 
         int avail[kTlMax];
 #pragma unroll
         for (int i = 0; i < kTlMax - 1; ++i) avail[i] = (int)__ldcg(desc + (size_t)(8 + i) * stride + q);
-        reg_build<1>(nodes, T, S.part, avail, (int)(w0 >> 8));
+        reg_build(nodes, T, [&](uint32_t mask) { return (uint32_t)S.part[mask]; }, avail, (int)(w0 >> 8));
       }
       __syncwarp();
     }
     return;
   }
   float* C = s_cost + lane;
-  uint8_t* P = s_part + lane;
   // warp-uniform loop: the warp runs the DP variant of its largest treelet
   for (uint32_t kb = b + blockIdx.x * kLvThreads; kb < e; kb += gridDim.x * kLvThreads) {
     const uint32_t k = kb + lane;
-    lane_dp<NVMAX>(nodes, desc, stride, k - b, k < e, C, P);
+    lane_dp<NVMAX>(nodes, desc, stride, k - b, k < e, C);
   }
 }
 
@@ -729,7 +759,6 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dpc(Node* __restrict__ nodes,
                                                        const uint32_t* __restrict__ desc, uint32_t stride) {
   constexpr int R = 8;
   __shared__ float s_cost[(1 << NV) * 32];
-  __shared__ uint8_t s_part[(1 << NV) * 32];
   __shared__ uint32_t s_list[32 * R];
   if (__ldcg(ctl) != 0u) return;
   const uint32_t h = __ldcg(ctl + 2);
@@ -737,7 +766,6 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dpc(Node* __restrict__ nodes,
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
   float* C = s_cost + lane;
-  uint8_t* P = s_part + lane;
   const uint32_t rounds = max(1u, min((uint32_t)R, div_up(e - b, 32u * gridDim.x)));
   for (uint32_t chunk = b + blockIdx.x * (32u * rounds); chunk < e; chunk += gridDim.x * (32u * rounds)) {
     uint32_t cnt = 0;
@@ -752,7 +780,7 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dpc(Node* __restrict__ nodes,
     __syncwarp();
     for (uint32_t i = 0; i < cnt; i += 32) {
       const bool act = i + (uint32_t)lane < cnt;
-      lane_dp<NV>(nodes, desc, stride, act ? s_list[i + lane] : 0u, act, C, P);
+      lane_dp<NV>(nodes, desc, stride, act ? s_list[i + lane] : 0u, act, C);
     }
     __syncwarp();  // the list is refilled by the next chunk
   }
@@ -821,7 +849,7 @@ __global__ void __launch_bounds__(kNarrowThreads) k_tl_narrow(Node* __restrict__
             T.id[i] = W.S.act[i];
             T.b[i] = leaf_box(W.S, i);
           }
-          reg_build<1>(nodes, T, W.S.part, W.avail, W.na);
+          reg_build(nodes, T, [&](uint32_t mask) { return (uint32_t)W.S.part[mask]; }, W.avail, W.na);
         }
       }
       __syncwarp();
