@@ -610,7 +610,7 @@ def run_ours(args):
         "e2e": e2e,
         # PLOC's and LBVH+'s loops run on the device: those builds report their own launches
         "gpu_launches": args.steps * (build_launches if algo in ("ploc", "lbvh_plus") and build_launches > 0
-                                      else kernels_per_build(algo, bits, rounds, ploc_iters, tree_height)),
+                                      else kernels_per_build(algo, bits, rounds, ploc_iters, tree_height) + 1),  # + k_finish
         "clocks": clk.summary(),
         "autotune": tuning,
     }
@@ -785,7 +785,7 @@ def measure_batched(steps, warmup, local=0, rank=0, autotune=True, algo="lbvh", 
            "stage_ms": stages,
            "e2e": {"value": round(n / (e2e_ms / 1e3) / 1e6, 2), "unit": "Mtris/s", "h2d_bytes_per_step": 36 * n,
                    "d2h_bytes_per_step": 48 * n_nodes + 4 * n, "ms_per_step": round(e2e_ms, 3)},
-           "gpu_launches": steps * batched_kernels_per_build(count, iters if algo == "ploc" else -1),
+           "gpu_launches": steps * (batched_kernels_per_build(count, iters if algo == "ploc" else -1) + 1),
            "clocks": clk.summary(), "autotune": tuning}
     if algo == "ploc":
         out["ploc"] = {"iterations": iters, "cluster_sum": csum, "radius": radius}

@@ -29,6 +29,7 @@ __device__ __forceinline__ void atomic_fmax(float* a, float v) {
 }
 
 __global__ void k_seg_init(float* __restrict__ mbox, uint32_t count, uint32_t* __restrict__ scratch, ScratchLayout L) {
+  stage_stamp(reinterpret_cast<unsigned long long*>(scratch + L.stamps), 0);
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
   for (uint32_t m = gtid; m < count; m += gsz) {
     float4* b = reinterpret_cast<float4*>(mbox + 8 * (size_t)m);
@@ -106,6 +107,8 @@ __global__ void __launch_bounds__(256) k_seg_morton(MeshPtrs m, const SegItem* _
   __shared__ uint32_t s_hist[kMaxPasses][256];
   __shared__ float s_scene[6];
   for (int k = threadIdx.x; k < kMaxPasses * 256; k += blockDim.x) (&s_hist[0][0])[k] = 0;
+  let_next_start();
+  stage_stamp(reinterpret_cast<unsigned long long*>(scratch + L.stamps), 1);
   for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
     const SegItem w = items[it];
     __syncthreads();
@@ -171,11 +174,11 @@ cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_
   if ((e = epoch_tick(ws, st)) != cudaSuccess) return e;
   k_seg_init<<<152 * 4, 256, 0, st>>>(d_mbox, count, ws.scratch, L);
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(n_items, 152 * 8));
+  // launched plainly: started early, these grids of 8 blocks per SM settle where the one before them leaves
+  // room first, and their static shares of the items then run unevenly (k_seg_morton 647 -> 680 us at 29M)
   k_seg_bounds<<<grid, 256, 0, st>>>(m, d_items, n_items, d_mbox);
-  if (evs && evs->use) cudaEventRecord(evs->ev[1], st);
   k_seg_morton<<<grid, 256, 0, st>>>(m, d_items, n_items, d_mbox, passes, shift0,
                                      reinterpret_cast<uint32_t*>(ws.keys[0]), lows, ws.boxes, ws.scratch, L);
-  if (evs && evs->use) cudaEventRecord(evs->ev[2], st);
   int fb = 0;
   if ((e = run_sort_u32(ws, n, passes, st, L, &fb)) != cudaSuccess) return e;
   const uint32_t* hkeys = reinterpret_cast<const uint32_t*>(ws.keys[fb]);
@@ -185,7 +188,6 @@ cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_
                                reinterpret_cast<uint32_t*>(ws.delta), ws.scratch + L.counters + kLongRunCounter,
                                nullptr, st)) != cudaSuccess)
     return e;
-  if (evs && evs->use) cudaEventRecord(evs->ev[3], st);
   out->fb = fb;
   out->shift0 = shift0;
   out->lows = lows;
@@ -201,19 +203,18 @@ cudaError_t batched_build(Workspace& ws, const MeshPtrs& m, uint32_t n, const ui
   ScratchLayout L = scratch_layout(ws.cap_n);
   const int fb = bs.fb;
   const uint32_t* hkeys = reinterpret_cast<const uint32_t*>(ws.keys[fb]);
-  k_delta_seg_split<<<div_up(n, 256), 256, 0, st>>>(hkeys, ws.vals[fb], bs.lows, d_offsets, bs.shift0, ws.delta, n);
+  if ((e = launch_after(k_delta_seg_split, div_up(n, 256), 256, 0, st, hkeys, ws.vals[fb], bs.lows, d_offsets, bs.shift0,
+                        ws.delta, n)) != cudaSuccess)
+    return e;
   uint32_t* fcount = ws.scratch + L.counters + kFrontierCounter;
   uint2* frontier = reinterpret_cast<uint2*>(ws.keys[fb ^ 1]);  // the sort's other key buffer
   const SegBatch seg{hkeys, d_offsets, 30 - bs.shift0};
-  k_emit<SegBatch, false, kEmitTile><<<div_up(n, kEmitTile), kEmitTile, 0, st>>>(
-      ws.delta, nullptr, ws.vals[fb], ws.boxes, ws.nodes, n, seg, d_indices, frontier, fcount, kEmitMaxSteps);
-  k_emit_climb<SegBatch, false><<<std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st>>>(
-      ws.delta, ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount);
-  if (evs && evs->use) {
-    cudaEventRecord(evs->ev[4], st);
-    cudaEventRecord(evs->ev[5], st);
-  }
-  return cudaGetLastError();
+  if ((e = launch_after(k_emit<SegBatch, false, kEmitTile>, div_up(n, kEmitTile), kEmitTile, 0, st, ws.delta, nullptr,
+                        ws.vals[fb], ws.boxes, ws.nodes, n, seg, d_indices, frontier, fcount, kEmitMaxSteps,
+                        reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps))) != cudaSuccess)
+    return e;
+  return launch_after(k_emit_climb<SegBatch, false>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st, ws.delta,
+                      ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount);
 }
 
 }  // namespace bvhgb

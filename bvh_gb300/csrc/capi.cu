@@ -64,7 +64,7 @@ struct bvh_ctx {
   cudaStream_t last_stream = nullptr;
   // bvh_build_host: a second stream that copies the indices and leaves out while the build ends
   cudaStream_t dl_stream = nullptr;
-  cudaEvent_t ev_leaves = nullptr, ev_dl = nullptr;
+  cudaEvent_t ev_sorted = nullptr, ev_leaves = nullptr, ev_dl = nullptr;
 };
 
 static bvh_status from_cuda(cudaError_t e) {
@@ -129,6 +129,7 @@ extern "C" bvh_status bvh_ctx_destroy(bvh_ctx* ctx) {
   if (ctx->bgraph.exec) cudaGraphExecDestroy(ctx->bgraph.exec);
   if (ctx->capture_stream) cudaStreamDestroy(ctx->capture_stream);
   if (ctx->dl_stream) cudaStreamDestroy(ctx->dl_stream);
+  if (ctx->ev_sorted) cudaEventDestroy(ctx->ev_sorted);
   if (ctx->ev_leaves) cudaEventDestroy(ctx->ev_leaves);
   if (ctx->ev_dl) cudaEventDestroy(ctx->ev_dl);
   workspace_free(ctx->ws);
@@ -228,6 +229,7 @@ static bvh_status build_impl(bvh_ctx* ctx, const bvh_mesh_soa* mesh, const bvh_p
   ctx->ws.no_cooperative = params->reserved[2] == BVH_NO_COOPERATIVE;
   apply_tuning(ctx, params->algo, n);
   ctx->have_timing = false;
+  ctx->evs.split = false;
   ctx->last = bvh_timing{};
   ctx->last_algo = params->algo;
   ctx->last_stream = st;
@@ -249,12 +251,12 @@ static bvh_status build_impl(bvh_ctx* ctx, const bvh_mesh_soa* mesh, const bvh_p
                    params->reserved[1] == BVH_HOST_DRIVEN_LOOPS);
     if (e != cudaSuccess) return from_cuda(e);
   }
-  ScratchLayout L = scratch_layout(ctx->ws.cap_n);
-  cudaMemcpyAsync(ctx->h_status, ctx->ws.scratch + L.status, 4, cudaMemcpyDeviceToHost, st);
-  if (params->algo == BVH_ALGO_PLOC)  // iterations and live-cluster sum, read at bvh_sync
-    cudaMemcpyAsync(ctx->h_status + 4, ctx->ws.scratch + L.ploc, 20 * 4, cudaMemcpyDeviceToHost, st);
-  if (params->algo == BVH_ALGO_LBVH_PLUS && params->treelet_rounds > 0 && n > 1)  // tree height, read at bvh_sync
-    cudaMemcpyAsync(ctx->h_status + 4, ctx->ws.scratch + L.hist + kTlCtlWord, 3 * 4, cudaMemcpyDeviceToHost, st);
+  // with the status word: PLOC's iterations and live-cluster sum, or LBVH+'s tree height (read at bvh_sync)
+  const ScratchLayout L = scratch_layout(ctx->ws.cap_n);
+  const bool plus = params->algo == BVH_ALGO_LBVH_PLUS && params->treelet_rounds > 0 && n > 1;
+  const int words = params->algo == BVH_ALGO_PLOC ? 20 : plus ? 3 : 0;
+  if ((e = finish_build(ctx->ws, plus ? L.hist + kTlCtlWord : L.ploc, words, ctx->h_status, st)) != cudaSuccess)
+    return from_cuda(e);
   cudaEventRecord(ctx->evs.ev[6], st);
   out->nodes = reinterpret_cast<const bvh_node*>(ctx->ws.nodes);
   out->indices = idx;
@@ -300,13 +302,13 @@ extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {
     const uint32_t* w = ctx->h_status + 4;
     ctx->last.ploc_iterations = (int32_t)w[kPlocIterWord];
     ctx->last.ploc_cluster_sum = (uint64_t)w[kPlocSumWord + 1] << 32 | w[kPlocSumWord];
-    // bounds, Morton, 4 sort passes, cluster init; 4 per iteration run as separate launches; the
+    // bounds, Morton, 4 sort passes, cluster init, the final report; 4 per iteration run as separate launches; the
     // middle-iterations and tail kernels (each one launch, whatever it ran); the root fix
     const int32_t one_launch_its = (int32_t)(w[16] + w[17]);
     ctx->last.kernel_launches = ctx->last_n == 0   ? 0  // batched: the caller counts
-                                : ctx->last_n > 1 ? 7 + 4 * (ctx->last.ploc_iterations - one_launch_its) +
+                                : ctx->last_n > 1 ? 8 + 4 * (ctx->last.ploc_iterations - one_launch_its) +
                                                       (int32_t)w[18] + (int32_t)w[19] + 1
-                                                  : 7;
+                                                  : 8;
   } else if (ctx->last_algo == BVH_ALGO_LBVH_PLUS) {
     ctx->last.tree_height = (int32_t)ctx->h_status[5];
     // LBVH kernels, then per treelet pass: heights, counts, offsets, grouping, the fallback
@@ -317,7 +319,7 @@ extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {
     int32_t loop_h;
     if (ctx->last_host_loops) loop_h = c[0] ? 0 : std::max(0, (int32_t)c[1] - 3);
     else loop_h = c[0] ? 1 : std::max(1, (ctx->ws.tl_narrow ? (int32_t)c[2] : (int32_t)c[1] + 1) - 4);
-    const int32_t lbvh = 2 + 4 + (ctx->last_bits != 30 ? 2 : 0) + 2;
+    const int32_t lbvh = 2 + 4 + (ctx->last_bits != 30 ? 2 : 0) + 2 + 1;  // the last: the final report
     ctx->last.kernel_launches =
         ctx->last_n > 1 ? lbvh + ctx->last_rounds * (5 + 11 + 3 * loop_h + (ctx->ws.tl_narrow ? 1 : 0)) : lbvh;
   }
@@ -330,13 +332,17 @@ extern "C" bvh_status bvh_last_timing(bvh_ctx* ctx, bvh_timing* out) {
   bvh_timing t = ctx->last;
   if (ctx->have_timing) {
     cudaEvent_t* ev = ctx->evs.ev;
-    float a = 0;
-    if (cudaEventElapsedTime(&a, ev[0], ev[1]) == cudaSuccess) t.bounds_ms = a;
-    if (cudaEventElapsedTime(&a, ev[1], ev[2]) == cudaSuccess) t.morton_ms = a;
-    if (cudaEventElapsedTime(&a, ev[2], ev[3]) == cudaSuccess) t.sort_ms = a;
-    if (cudaEventElapsedTime(&a, ev[3], ev[4]) == cudaSuccess) t.emit_ms = a;
-    if (cudaEventElapsedTime(&a, ev[4], ev[5]) == cudaSuccess) t.optimize_ms = a;
-    if (cudaEventElapsedTime(&a, ev[0], ev[5]) == cudaSuccess) t.total_ms = a;
+    unsigned long long at[4];  // stage start times in ns: bounds, Morton, sort, emission
+    memcpy(at, ctx->h_status + 24, sizeof(at));
+    const auto ms = [&](int a, int b) { return at[b] > at[a] ? (float)((double)(at[b] - at[a]) * 1e-6) : 0.0f; };
+    float end = 0, total = 0;
+    if (cudaEventElapsedTime(&total, ev[0], ev[6]) == cudaSuccess) t.total_ms = total;
+    if (!ctx->evs.split || cudaEventElapsedTime(&end, ev[0], ev[4]) != cudaSuccess) end = t.total_ms;
+    t.optimize_ms = t.total_ms - end;
+    t.bounds_ms = ms(0, 1);
+    t.morton_ms = ms(1, 2);
+    t.sort_ms = ms(2, 3);
+    t.emit_ms = std::max(0.0f, end - t.bounds_ms - t.morton_ms - t.sort_ms);
   }
   *out = t;
   return s;
@@ -397,18 +403,20 @@ extern "C" bvh_status bvh_build_host(bvh_ctx* ctx, const bvh_mesh_soa* mesh, con
   const bool early = params->algo == BVH_ALGO_LBVH && n > 1;
   if (early && !ctx->dl_stream) {
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->dl_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_sorted, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_leaves, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_dl, cudaEventDisableTiming);
     if (e != cudaSuccess) return from_cuda(e);
   }
   bvh_tree tree;
+  ws.indices_ready = early ? ctx->ev_sorted : nullptr;
   ws.leaves_ready = early ? ctx->ev_leaves : nullptr;
   bvh_status s = build_impl(ctx, &dm, params, st, &tree);
-  ws.leaves_ready = nullptr;
+  ws.indices_ready = ws.leaves_ready = nullptr;
   if (s != BVH_OK) return s;
   if (early) {
     cudaStream_t dl = ctx->dl_stream;
-    cudaError_t e = cudaStreamWaitEvent(dl, ctx->evs.ev[3], 0);  // sort (and run fix-up) done
+    cudaError_t e = cudaStreamWaitEvent(dl, ctx->ev_sorted, 0);  // sort (and run fix-up) done
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_indices, tree.indices, (size_t)n * 4, cudaMemcpyDeviceToHost, dl);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(dl, ctx->ev_leaves, 0);
     if (e == cudaSuccess)
@@ -513,6 +521,7 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
   ctx->have_timing = false;
   ctx->last = bvh_timing{};
   ctx->last_n = 0;
+  ctx->evs.split = false;
   ctx->last_algo = params->algo;
   apply_tuning(ctx, params->algo + 256, n);
   const uint32_t n_items = count_items(batch->offsets, count);
@@ -571,14 +580,11 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
     cudaEventRecord(ctx->evs.ev[0], st);
     if ((e = epoch_tick(ws, st)) != cudaSuccess) return from_cuda(e);  // the graph bumps the epoch
     if ((e = cudaGraphLaunch(g.exec, st)) != cudaSuccess) return from_cuda(e);
-    for (int k = 1; k <= 5; ++k) cudaEventRecord(ctx->evs.ev[k], st);
   } else {
     if ((e = enqueue_batch(ctx, m, n, count, words, params, st, true)) != cudaSuccess) return from_cuda(e);
   }
-  ScratchLayout L = scratch_layout(ws.cap_n);
-  cudaMemcpyAsync(ctx->h_status, ws.scratch + L.status, 4, cudaMemcpyDeviceToHost, st);
-  if (ploc)  // iterations and live-cluster sum, read at bvh_sync
-    cudaMemcpyAsync(ctx->h_status + 4, ws.scratch + L.ploc, 20 * 4, cudaMemcpyDeviceToHost, st);
+  const ScratchLayout L = scratch_layout(ws.cap_n);
+  if ((e = finish_build(ws, L.ploc, ploc ? 20 : 0, ctx->h_status, st)) != cudaSuccess) return from_cuda(e);
   cudaEventRecord(ctx->evs.ev[6], st);
   ctx->last_stream = st;
   ctx->have_timing = true;

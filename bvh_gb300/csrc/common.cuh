@@ -224,6 +224,27 @@ __device__ __forceinline__ bool grid_sync(uint32_t* bar, uint32_t target, uint32
   return *s_ok != 0;
 }
 
+// Programmatic dependent launch.  A kernel launched with launch_after (lbvh.cuh) may start while the one
+// before it in the stream still runs, so its launch latency and its shared-memory set-up overlap that
+// kernel's end; every block must pass after_previous() before it touches global memory.  It then allows
+// the same to the next kernel, which starts once all blocks here have got that far: the overlap is of
+// two kernels at most, so whatever a kernel reads is two kernel starts away from any older use of it.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// The first kernel of a build, launched the plain way.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Start time of a build stage (0 bounds, 1 Morton, 2 sort, 3 emission), written by its first block.
+__device__ __forceinline__ void stage_stamp(unsigned long long* stamps, int stage) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    stamps[stage] = t;
+  }
+}
+
 __host__ __device__ inline uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 }  // namespace bvhgb

@@ -89,6 +89,7 @@ static __global__ void __launch_bounds__(256)
     k_delta_seg_split(const uint32_t* __restrict__ hk, const uint32_t* __restrict__ vals,
                       const uint32_t* __restrict__ lows, const uint32_t* __restrict__ offsets, int shift0,
                       uint8_t* __restrict__ D, uint32_t n) {
+  after_previous();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k + 1 >= n) return;
   const uint32_t a = __ldg(hk + k), b = __ldg(hk + k + 1);
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
                                             const Box* __restrict__ tri_boxes, Node* __restrict__ nodes,
                                             uint32_t n, Seg seg, uint32_t* __restrict__ out_idx,
                                             uint2* __restrict__ frontier, uint32_t* __restrict__ frontier_count,
-                                            uint32_t max_steps) {
+                                            uint32_t max_steps, unsigned long long* __restrict__ stamps) {
   // D of positions bbase-1 .. bbase+T-1 (0 outside [0, n-1) : a segment boundary)
   __shared__ uint8_t s_D[T + 1];
   // KEYS30: keys and values of positions bbase-1 .. bbase+T
@@ -148,6 +149,9 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   const uint32_t tid = threadIdx.x;
   const uint32_t i = blockIdx.x * T + tid;
   const uint32_t bbase = blockIdx.x * T;  // sorted position of thread 0
+  s_flag[tid] = 0;
+  after_previous();
+  stage_stamp(stamps, 3);
   bool active = i < n;
   uint32_t off = 0, cnt = 1, nb = 0;
   Climb c;
@@ -157,7 +161,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   c.my = 0;
   if (active) {
     seg.get(i, off, cnt, nb);
-    const uint32_t prim_g = __ldg(vals + i);
+    const uint32_t prim_g = __ldcg(vals + i);
     const uint32_t prim = prim_g - off;  // original index within the mesh
     if (out_idx) out_idx[i] = prim;
     const float4* bp = reinterpret_cast<const float4*>(tri_boxes + prim_g);
@@ -167,18 +171,18 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     store_node(nodes, nb + (uint32_t)c.my, c.box, (int32_t)(prim | kLeafBit), -1, -1);
     if (cnt == 1) active = false;  // a one-triangle mesh: the leaf is the root
     if (KEYS30) {
-      s_k[tid + 1] = __ldg(keys30 + i);
+      s_k[tid + 1] = __ldcg(keys30 + i);
       s_v[tid + 1] = prim_g;
     }
   }
   if (KEYS30) {
     if (tid == 0 && bbase > 0) {
-      s_k[0] = __ldg(keys30 + bbase - 1);
-      s_v[0] = __ldg(vals + bbase - 1);
+      s_k[0] = __ldcg(keys30 + bbase - 1);
+      s_v[0] = __ldcg(vals + bbase - 1);
     }
     if (tid == T - 1 && bbase + T < n) {
-      s_k[T + 1] = __ldg(keys30 + bbase + T);
-      s_v[T + 1] = __ldg(vals + bbase + T);
+      s_k[T + 1] = __ldcg(keys30 + bbase + T);
+      s_v[T + 1] = __ldcg(vals + bbase + T);
     }
     __syncthreads();
     // s_D[k] = D[bbase - 1 + k]; position j and j + 1 sit at s_k[k], s_k[k + 1]
@@ -200,7 +204,6 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
       s_D[T] = jl + 1 < n ? __ldg(D + jl) : (uint8_t)0;
     }
   }
-  s_flag[tid] = 0;
   __syncthreads();
   // ---- climb inside the block: the second child to reach a split completes the parent ----
   // A node [f, l] with both ends in this block reads D[f-1] and D[l] from s_D; its parent's
@@ -288,6 +291,7 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
                                                     const uint32_t* epoch_word, uint32_t n, Seg seg,
                                                     const uint2* __restrict__ frontier,
                                                     const uint32_t* __restrict__ frontier_count) {
+  after_previous();
   const uint32_t count = __ldcg(frontier_count);
   const unsigned long long tag = (unsigned long long)__ldcg(epoch_word) << 32;
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {

@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(256, 4) k_fixrun_split_short(const uint32_t* _
                                                             uint8_t* __restrict__ D, uint32_t* __restrict__ long_list,
                                                             uint32_t* __restrict__ long_count) {
   constexpr unsigned long long kNoH = ~0ull;
+  after_previous();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
   unsigned long long hw[8];
@@ -288,6 +289,7 @@ __global__ void __launch_bounds__(kFixThreads) k_fixrun_split_long(const uint32_
   __shared__ uint32_t s_off[256];
   __shared__ uint32_t s_w[8];
   __shared__ uint32_t s_e;
+  after_previous();
   const uint32_t count = __ldcg(long_count);
   const int t = threadIdx.x;
   for (uint32_t li = blockIdx.x; li < count; li += gridDim.x) {
@@ -358,16 +360,11 @@ cudaError_t sort_fix_runs_split(const uint32_t* hkeys, uint32_t* vals, const uin
                                 uint32_t* long_list, uint32_t* long_count, uint8_t* D, cudaStream_t st) {
   if (n < 2) return cudaSuccess;
   const uint32_t grid = div_up(div_up(n, 4u), 256u);
-  if (D) {
-    k_fixrun_split_short<true><<<grid, 256, 0, st>>>(hkeys, vals, lows, n, lbits, D, long_list, long_count);
-    k_fixrun_split_long<true><<<152, kFixThreads, 0, st>>>(hkeys, vals, lows, n, lbits, scratch_a, scratch_b, tvals,
-                                                           D, long_list, long_count);
-  } else {
-    k_fixrun_split_short<false><<<grid, 256, 0, st>>>(hkeys, vals, lows, n, lbits, D, long_list, long_count);
-    k_fixrun_split_long<false><<<152, kFixThreads, 0, st>>>(hkeys, vals, lows, n, lbits, scratch_a, scratch_b, tvals,
-                                                            D, long_list, long_count);
-  }
-  return cudaGetLastError();
+  cudaError_t e = launch_after(D ? k_fixrun_split_short<true> : k_fixrun_split_short<false>, grid, 256, 0, st, hkeys, vals,
+                               lows, n, lbits, D, long_list, long_count);
+  if (e != cudaSuccess) return e;
+  return launch_after(D ? k_fixrun_split_long<true> : k_fixrun_split_long<false>, 152, kFixThreads, 0, st, hkeys, vals,
+                      lows, n, lbits, scratch_a, scratch_b, tvals, D, long_list, long_count);
 }
 
 }  // namespace bvhgb

@@ -36,6 +36,8 @@ ScratchLayout scratch_layout(uint32_t n) {
   o = (o + 3) & ~size_t(3);
   L.scene = o; o += 8;
   L.ploc = o; o += 20;
+  o = (o + 1) & ~size_t(1);
+  L.stamps = o; o += 8;
   L.partials = o; o += (size_t)kBoundsBlocks * 8;
   o = (o + 3) & ~size_t(3);
   L.zero_begin = o;
@@ -72,6 +74,8 @@ __device__ __forceinline__ void tri_box_acc(float a0, float a1, float a2, float&
 
 __global__ void __launch_bounds__(256) k_bounds(MeshPtrs m, uint32_t n, int vec4, uint32_t* __restrict__ scratch,
                                                 ScratchLayout L) {
+  let_next_start();
+  stage_stamp(reinterpret_cast<unsigned long long*>(scratch + L.stamps), 0);
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gsz = gridDim.x * blockDim.x;
   // zero the current build's histograms, tile counters and look-back descriptors
@@ -198,6 +202,8 @@ __global__ void __launch_bounds__(256) k_morton(MeshPtrs m, uint32_t n, int vec4
   __shared__ uint32_t s_hist[P][256];
   for (int i = threadIdx.x; i < P * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0;
   __shared__ float s_scene[8];
+  after_previous();
+  stage_stamp(reinterpret_cast<unsigned long long*>(scratch + L.stamps), 1);
   if (threadIdx.x < 8) s_scene[threadIdx.x] = __ldcg(reinterpret_cast<const float*>(scratch + L.scene) + threadIdx.x);
   __syncthreads();
   const float* smn = s_scene;
@@ -338,9 +344,11 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(const K* __restrict_
 
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int shift = 8 * pass;  // digit `pass` of the key
-  if (tid == 0) *s_tile = atomicAdd(scratch + L.counters + pass, 1u);
   for (int b = tid; b < NW * BINS; b += THREADS) s_whist[b] = 0;
   for (int b = tid; b < NW * kMatchWords; b += THREADS) s_match[b] = 0;
+  after_previous();
+  if (pass == 0) stage_stamp(reinterpret_cast<unsigned long long*>(scratch + L.stamps), 2);
+  if (tid == 0) *s_tile = atomicAdd(scratch + L.counters + pass, 1u);
   __syncthreads();
   const uint32_t tile = *s_tile;
   const uint32_t base = tile * (uint32_t)TILE;
@@ -483,7 +491,17 @@ static cudaError_t run_sort(Workspace& ws, uint32_t n, int passes, cudaStream_t 
     ScratchLayout Lc = L;
     void* args[] = {(void*)&kin, (void*)&vin, (void*)&kout, (void*)&vout, (void*)&n, (void*)&p, (void*)&scratch,
                     (void*)&Lc, (void*)&tiles};
-    cudaError_t e = cudaLaunchKernel(sv.fn, dim3(tiles), dim3(kSortThreads), args, sv.smem, st);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles);
+    cfg.blockDim = dim3(kSortThreads);
+    cfg.dynamicSmemBytes = sv.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelExC(&cfg, sv.fn, args);
     if (e != cudaSuccess) return e;
     cur ^= 1;
   }
@@ -586,6 +604,28 @@ cudaError_t wait_selftest(uint32_t limit, uint32_t* status_out) {
 }
 
 // ---------------------------------------------------------------------------------------
+// end of a build
+// ---------------------------------------------------------------------------------------
+// One warp writes what the host reads after a build straight to page-locked memory (a copy of the status
+// word through the copy engine, with an event on each side, took 4 to 6 us of every build).
+__global__ void k_finish(const uint32_t* __restrict__ scratch, size_t status, size_t first, int words, size_t stamps,
+                         uint32_t* __restrict__ host) {
+  after_previous();
+  const int t = threadIdx.x;
+  if (t == 0) host[0] = __ldcg(scratch + status);
+  if (t < words) host[4 + t] = __ldcg(scratch + first + t);
+  if (t >= 24) host[t] = __ldcg(scratch + stamps + (t - 24));
+}
+
+cudaError_t finish_build(const Workspace& ws, size_t first, int words, uint32_t* host, cudaStream_t st) {
+  const ScratchLayout L = scratch_layout(ws.cap_n);
+  uint32_t* dev = nullptr;
+  cudaError_t e = cudaHostGetDevicePointer(&dev, host, 0);
+  if (e != cudaSuccess) return e;
+  return launch_after(k_finish, 1, 32, 0, st, ws.scratch, L.status, first, words, L.stamps, dev);
+}
+
+// ---------------------------------------------------------------------------------------
 // workspace
 // ---------------------------------------------------------------------------------------
 void workspace_free(Workspace& ws) {
@@ -667,8 +707,8 @@ static inline uint32_t* split_long_list(const Workspace& ws, uint32_t n) {
 }
 
 template <int BITS, typename K>
-static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, StageEvents* evs,
-                               const ScratchLayout& L, int* final_buf) {
+static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, const ScratchLayout& L,
+                               int* final_buf) {
   uint32_t* lows = sizeof(K) == 8 ? split_lows(ws) : nullptr;
   const int vec4 = all_aligned16(m) && (reinterpret_cast<uintptr_t>(lows) & 15) == 0 ? 1 : 0;
   // zero only the descriptors the current build's passes use (the passes sort 32-bit keys)
@@ -677,13 +717,13 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
                                              (uint32_t)sort_variant_tile(ws.sort_variant)) * 256;
   cudaError_t et = epoch_tick(ws, st);
   if (et != cudaSuccess) return et;
-  k_bounds<<<kBoundsBlocks, 256, 0, st>>>(m, n, vec4, ws.scratch, Lz);
-  rec(evs, 1, st);
   const uint32_t work = vec4 ? div_up(n, 4) : n;
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(div_up(work, 256), 152 * 8));
-  k_morton<BITS, K><<<grid, 256, 0, st>>>(m, n, vec4, reinterpret_cast<uint32_t*>(ws.keys[0]), lows, ws.boxes,
-                                          ws.scratch, L);
-  rec(evs, 2, st);
+  // (the bounds partials and the last block's arrival count grow with the grid: no idle blocks)
+  k_bounds<<<std::min<uint32_t>(grid, kBoundsBlocks), 256, 0, st>>>(m, n, vec4, ws.scratch, Lz);
+  if ((et = launch_after(k_morton<BITS, K>, grid, 256, 0, st, m, n, vec4, reinterpret_cast<uint32_t*>(ws.keys[0]), lows,
+                         ws.boxes, ws.scratch, L)) != cudaSuccess)
+    return et;
   // 4 passes sort the 32-bit keys: the whole 30-bit code, or the high 32 bits of a 60/63-bit
   // code; then each run of equal high halves is ordered by its low bits.
   cudaError_t e = run_sort(ws, n, 4, st, L, final_buf);
@@ -695,31 +735,33 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
                             ws.vals[fb ^ 1], split_long_list(ws, n), ws.scratch + L.counters + kLongRunCounter,
                             ws.delta, st);
   }
-  rec(evs, 3, st);
+  if (e == cudaSuccess && ws.indices_ready) e = cudaEventRecord(ws.indices_ready, st);
   return e;
 }
 
-cudaError_t prefix_sort30(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, StageEvents* evs,
-                          uint32_t** sorted_idx) {
+cudaError_t prefix_sort30(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, uint32_t** sorted_idx) {
   ScratchLayout L = scratch_layout(ws.cap_n);
   int fb = 0;
-  cudaError_t e = lbvh_prefix<30, uint32_t>(ws, m, n, st, evs, L, &fb);
+  cudaError_t e = lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb);
   *sorted_idx = ws.vals[fb];
   return e;
 }
 
 template <int BITS, bool PARENTS>
-static void launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchLayout& L, cudaStream_t st) {
+static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchLayout& L, cudaStream_t st) {
   const uint32_t* keys = reinterpret_cast<const uint32_t*>(ws.keys[fb]);
   const uint32_t* epoch = ws.scratch + L.epoch;
   uint32_t* fcount = ws.scratch + L.counters + kFrontierCounter;
   uint2* frontier = reinterpret_cast<uint2*>(ws.keys[fb ^ 1]);  // the sort's other key buffer, 8 B per position
   // delta bytes: computed by k_emit from the 30-bit keys, written by the run fix-up for 60/63 bits
-  k_emit<SegSingle, PARENTS, kEmitTile, BITS == 30><<<div_up(n, kEmitTile), kEmitTile, 0, st>>>(
-      ws.delta, keys, ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier, fcount, kEmitMaxSteps);
+  unsigned long long* stamps = reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps);
+  cudaError_t e = launch_after(k_emit<SegSingle, PARENTS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
+                               ws.delta, keys, ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier,
+                               fcount, kEmitMaxSteps, stamps);
+  if (e != cudaSuccess) return e;
   if (ws.leaves_ready && !PARENTS) cudaEventRecord(ws.leaves_ready, st);
-  k_emit_climb<SegSingle, PARENTS><<<std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st>>>(
-      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount);
+  return launch_after(k_emit_climb<SegSingle, PARENTS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
+                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount);
 }
 
 cudaError_t run_sort_u32(Workspace& ws, uint32_t n, int passes, cudaStream_t st, const ScratchLayout& L,
@@ -736,27 +778,22 @@ cudaError_t lbvh_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int bits, i
   int fb = 0;
   const bool parents = treelet_rounds > 0;
   if (bits == 30) {
-    e = lbvh_prefix<30, uint32_t>(ws, m, n, st, evs, L, &fb);
-    if (e != cudaSuccess) return e;
-    if (parents) launch_emit<30, true>(ws, fb, n, L, st);
-    else launch_emit<30, false>(ws, fb, n, L, st);
+    if ((e = lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
+    e = parents ? launch_emit<30, true>(ws, fb, n, L, st) : launch_emit<30, false>(ws, fb, n, L, st);
   } else if (bits == 60) {
-    e = lbvh_prefix<60, unsigned long long>(ws, m, n, st, evs, L, &fb);
-    if (e != cudaSuccess) return e;
-    if (parents) launch_emit<60, true>(ws, fb, n, L, st);
-    else launch_emit<60, false>(ws, fb, n, L, st);
+    if ((e = lbvh_prefix<60, unsigned long long>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
+    e = parents ? launch_emit<60, true>(ws, fb, n, L, st) : launch_emit<60, false>(ws, fb, n, L, st);
   } else {
-    e = lbvh_prefix<63, unsigned long long>(ws, m, n, st, evs, L, &fb);
-    if (e != cudaSuccess) return e;
-    if (parents) launch_emit<63, true>(ws, fb, n, L, st);
-    else launch_emit<63, false>(ws, fb, n, L, st);
+    if ((e = lbvh_prefix<63, unsigned long long>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
+    e = parents ? launch_emit<63, true>(ws, fb, n, L, st) : launch_emit<63, false>(ws, fb, n, L, st);
   }
-  rec(evs, 4, st);
+  if (e != cudaSuccess) return e;
   if (treelet_rounds > 0 && n >= 2) {
+    rec(evs, 4, st);
+    if (evs) evs->split = evs->use;
     e = treelet_rounds_run(ws, n, treelet_rounds, st, fb, host_loops);
     if (e != cudaSuccess) return e;
   }
-  rec(evs, 5, st);
   *out_indices = ws.vals[fb];
   return cudaGetLastError();
 }

@@ -69,9 +69,10 @@ struct Workspace {
   float* bat_mbox = nullptr;          // device, count * 8
   uint32_t* bat_indices = nullptr;    // device, n (mesh-local original indices)
   uint32_t bat_count_cap = 0, bat_n_cap = 0;
-  // recorded (when set) between the LBVH emission and its frontier climb: from there on the leaf
-  // nodes [n-1, 2n-1) of a plain LBVH are final and can be copied out while the climb runs
-  cudaEvent_t leaves_ready = nullptr;
+  // recorded (when set) after the LBVH sort, when the indices are final, and between the emission and
+  // its frontier climb: from there on the leaf nodes [n-1, 2n-1) of a plain LBVH are final; both can
+  // be copied out while the rest of the build runs
+  cudaEvent_t indices_ready = nullptr, leaves_ready = nullptr;
 };
 
 // First epoch value; every build adds kEpochStride (emission uses E, treelet round r uses E+1+r).
@@ -91,6 +92,7 @@ struct ScratchLayout {
   size_t desc;       // passes * tiles * 256
   size_t partials;   // bounds partials, kBoundsBlocks * 8
   size_t ploc;       // PLOC control words (20)
+  size_t stamps;     // 8 words, four 64-bit stage start times
   size_t zero_begin; // first word zeroed at the start of each build
   size_t zero_end;
   size_t total;
@@ -111,11 +113,35 @@ void sort_variant_describe(int v, int* ipt, int* window, int* minb);
 // Times every onesweep variant on `n` pseudo-random 32-bit keys and keeps the fastest in ws.
 cudaError_t autotune_sort(Workspace& ws, uint32_t n, cudaStream_t st, float* ms_out /* per variant */);
 
-// Builds stage events: [0] start, [1] bounds, [2] morton, [3] sort, [4] emit, [5] optimise.
+// Stage times of a build.  [0] start, [4] before the treelet passes or the clustering loop, [6] end; the
+// stages before that are told apart by the start times the kernels leave in the scratch (an event between
+// two kernels costs the stream about 2 us each and keeps the second from starting early).
 struct StageEvents {
   cudaEvent_t ev[8];
   bool use = false;
+  bool split = false;  // [4] was recorded: a treelet pass or a clustering loop follows it
 };
+
+// A kernel that may start before its predecessor in the stream has ended (it calls after_previous()).
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
+                                A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// The end of a build: writes its status word, `words` control words from scratch + first and the stage
+// start times to page-locked host memory (32 words: [0] status, [4..] control words, [24..] times).
+cudaError_t finish_build(const Workspace& ws, size_t first, int words, uint32_t* host, cudaStream_t st);
 
 // LBVH over device-resident SoA input; result in ws.nodes / ws.vals[final].
 // morton_bits: 30, 60 or 63.  treelet_rounds > 0 selects LBVH+.
@@ -132,8 +158,7 @@ constexpr int kPlocIterWord = 6;
 constexpr int kPlocSumWord = 8;
 
 // Shared pieces used by PLOC: bounds + Morton-30 + sort (indices sorted by code).
-cudaError_t prefix_sort30(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, StageEvents* evs,
-                          uint32_t** sorted_idx);
+cudaError_t prefix_sort30(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, uint32_t** sorted_idx);
 
 // Runs the sort's bounded look-back wait against a predecessor that never publishes, giving up
 // after `limit` polls; *status_out = the status word it left (kStatusSortTimeout expected).

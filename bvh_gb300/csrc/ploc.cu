@@ -58,7 +58,9 @@ struct PlocSeg {
 };
 
 __global__ void k_ploc_init(const uint32_t* __restrict__ sidx, const Box* __restrict__ tri_boxes, PlocBufs B, uint32_t n,
-                            uint32_t cap, uint32_t tail, uint32_t grid_at) {
+                            uint32_t cap, uint32_t tail, uint32_t grid_at,
+                            unsigned long long* __restrict__ stamps) {
+  stage_stamp(stamps, 3);
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
     B.ctrl[0] = n;
@@ -715,7 +717,9 @@ __global__ void __launch_bounds__(256) k_ploc_seg(PlocBufs B, PlocSeg S, uint32_
 __global__ void __launch_bounds__(256) k_ploc_init_seg(const uint32_t* __restrict__ sidx,
                                                        const Box* __restrict__ tri_boxes, PlocBufs B, PlocSeg S,
                                                        const SegItem* __restrict__ items, uint32_t n_items,
-                                                       uint32_t n, uint32_t cap, uint32_t* __restrict__ d_indices) {
+                                                       uint32_t n, uint32_t cap, uint32_t* __restrict__ d_indices,
+                                                       unsigned long long* __restrict__ stamps) {
+  stage_stamp(stamps, 3);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     B.ctrl[0] = n;
     B.ctrl[1] = n;
@@ -1422,10 +1426,14 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
   }
   if (evs && evs->use) cudaEventRecord(evs->ev[0], st);
   uint32_t* sidx = nullptr;
-  if ((e = prefix_sort30(ws, m, n, st, evs, &sidx)) != cudaSuccess) return e;
+  if ((e = prefix_sort30(ws, m, n, st, &sidx)) != cudaSuccess) return e;
   *out_indices = sidx;
-  k_ploc_init<<<div_up(n, 256), 256, 0, st>>>(sidx, ws.boxes, B, n, cap, tail, grid_at);
-  if (evs && evs->use) cudaEventRecord(evs->ev[4], st);
+  k_ploc_init<<<div_up(n, 256), 256, 0, st>>>(sidx, ws.boxes, B, n, cap, tail, grid_at,
+                                              reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps));
+  if (evs && evs->use) {
+    cudaEventRecord(evs->ev[4], st);
+    evs->split = true;
+  }
   if (loop && host_loop) {
     for (uint32_t it = 0; it < cap; ++it) {
       enqueue_iteration<false, false>(B, none, n, radius, sh, st, cudaGraphConditionalHandle{});
@@ -1475,7 +1483,6 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
     if (tail) k_ploc_tail<<<1, kTailThreads, tail_smem(), st>>>(B, radius);
     k_ploc_root<<<1, 256, 0, st>>>(ws.nodes, 2 * n - 1, B.ctrl);
   }
-  if (evs && evs->use) cudaEventRecord(evs->ev[5], st);
   return cudaGetLastError();
 }
 
@@ -1529,8 +1536,12 @@ cudaError_t batched_ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, con
   BatchedSort bs;
   if ((e = batched_prefix(ws, m, n, count, d_items, n_items, d_mbox, st, evs, &bs)) != cudaSuccess) return e;
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(n_items, 152 * 8));
-  k_ploc_init_seg<<<grid, 256, 0, st>>>(ws.vals[bs.fb], ws.boxes, B, S, d_items, n_items, n, cap, d_indices);
-  if (evs && evs->use) cudaEventRecord(evs->ev[4], st);
+  k_ploc_init_seg<<<grid, 256, 0, st>>>(ws.vals[bs.fb], ws.boxes, B, S, d_items, n_items, n, cap, d_indices,
+                                       reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps));
+  if (evs && evs->use) {
+    cudaEventRecord(evs->ev[4], st);
+    evs->split = true;
+  }
   if (loop && host_loop) {
     for (uint32_t it = 0; it < cap; ++it) {
       enqueue_iteration<true, false>(B, S, n, radius, sh, st, cudaGraphConditionalHandle{});
@@ -1575,7 +1586,6 @@ cudaError_t batched_ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, con
     }
   }
   if (loop) k_ploc_root_seg<<<grid, 256, 0, st>>>(ws.nodes, d_items, n_items, S, B.ctrl);
-  if (evs && evs->use) cudaEventRecord(evs->ev[5], st);
   return cudaGetLastError();
 }
 
