@@ -113,6 +113,7 @@ extern "C" bvh_status bvh_ctx_create(bvh_ctx** out, int device) {
     if (cudaEventCreate(&c->evs.ev[k]) != cudaSuccess) { delete c; return BVH_ERR_DEVICE; }
   c->evs.use = true;
   if (cudaMallocHost(&c->h_status, 128) != cudaSuccess) { delete c; return BVH_ERR_OUT_OF_MEMORY; }
+  if (cudaHostGetDevicePointer(&c->ws.report, c->h_status, 0) != cudaSuccess) { delete c; return BVH_ERR_DEVICE; }
   if (prepare_kernels() != cudaSuccess) { delete c; return BVH_ERR_DEVICE; }
   if (cudaStreamCreateWithFlags(&c->capture_stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete c;
@@ -230,6 +231,7 @@ static bvh_status build_impl(bvh_ctx* ctx, const bvh_mesh_soa* mesh, const bvh_p
   apply_tuning(ctx, params->algo, n);
   ctx->have_timing = false;
   ctx->evs.split = false;
+  ctx->ws.reported = false;
   ctx->last = bvh_timing{};
   ctx->last_algo = params->algo;
   ctx->last_stream = st;
@@ -255,7 +257,7 @@ static bvh_status build_impl(bvh_ctx* ctx, const bvh_mesh_soa* mesh, const bvh_p
   const ScratchLayout L = scratch_layout(ctx->ws.cap_n);
   const bool plus = params->algo == BVH_ALGO_LBVH_PLUS && params->treelet_rounds > 0 && n > 1;
   const int words = params->algo == BVH_ALGO_PLOC ? 20 : plus ? 3 : 0;
-  if ((e = finish_build(ctx->ws, plus ? L.hist + kTlCtlWord : L.ploc, words, ctx->h_status, st)) != cudaSuccess)
+  if ((e = finish_build(ctx->ws, plus ? L.hist + kTlCtlWord : L.ploc, words, st)) != cudaSuccess)
     return from_cuda(e);
   cudaEventRecord(ctx->evs.ev[6], st);
   out->nodes = reinterpret_cast<const bvh_node*>(ctx->ws.nodes);
@@ -302,13 +304,14 @@ extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {
     const uint32_t* w = ctx->h_status + 4;
     ctx->last.ploc_iterations = (int32_t)w[kPlocIterWord];
     ctx->last.ploc_cluster_sum = (uint64_t)w[kPlocSumWord + 1] << 32 | w[kPlocSumWord];
-    // bounds, Morton, 4 sort passes, cluster init, the final report; 4 per iteration run as separate launches; the
+    // bounds, Morton, 4 sort passes (one kernel for a small mesh), cluster init, the final report; 4 per iteration run as separate launches; the
     // middle-iterations and tail kernels (each one launch, whatever it ran); the root fix
     const int32_t one_launch_its = (int32_t)(w[16] + w[17]);
+    const int32_t prefix = one_block_build(ctx->last_n) ? 1 : 6;
     ctx->last.kernel_launches = ctx->last_n == 0   ? 0  // batched: the caller counts
-                                : ctx->last_n > 1 ? 8 + 4 * (ctx->last.ploc_iterations - one_launch_its) +
+                                : ctx->last_n > 1 ? prefix + 2 + 4 * (ctx->last.ploc_iterations - one_launch_its) +
                                                       (int32_t)w[18] + (int32_t)w[19] + 1
-                                                  : 8;
+                                                  : prefix + 2;
   } else if (ctx->last_algo == BVH_ALGO_LBVH_PLUS) {
     ctx->last.tree_height = (int32_t)ctx->h_status[5];
     // LBVH kernels, then per treelet pass: heights, counts, offsets, grouping, the fallback
@@ -319,7 +322,8 @@ extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {
     int32_t loop_h;
     if (ctx->last_host_loops) loop_h = c[0] ? 0 : std::max(0, (int32_t)c[1] - 3);
     else loop_h = c[0] ? 1 : std::max(1, (ctx->ws.tl_narrow ? (int32_t)c[2] : (int32_t)c[1] + 1) - 4);
-    const int32_t lbvh = 2 + 4 + (ctx->last_bits != 30 ? 2 : 0) + 2 + 1;  // the last: the final report
+    // the LBVH (one kernel for a small mesh) and the final report
+    const int32_t lbvh = one_block_build(ctx->last_n) ? 1 + 1 : 2 + 4 + (ctx->last_bits != 30 ? 2 : 0) + 2 + 1;
     ctx->last.kernel_launches =
         ctx->last_n > 1 ? lbvh + ctx->last_rounds * (5 + 11 + 3 * loop_h + (ctx->ws.tl_narrow ? 1 : 0)) : lbvh;
   }
@@ -400,7 +404,7 @@ extern "C" bvh_status bvh_build_host(bvh_ctx* ctx, const bvh_mesh_soa* mesh, con
   // A plain LBVH's indices are final after the sort and its leaves after the emission kernel:
   // a second stream copies those out while the rest of the build runs; the internal nodes
   // follow on the build's stream.  The copies use the link the whole time, which bounds the call.
-  const bool early = params->algo == BVH_ALGO_LBVH && n > 1;
+  const bool early = params->algo == BVH_ALGO_LBVH && !one_block_build(n);
   if (early && !ctx->dl_stream) {
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->dl_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_sorted, cudaEventDisableTiming);
@@ -522,6 +526,7 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
   ctx->last = bvh_timing{};
   ctx->last_n = 0;
   ctx->evs.split = false;
+  ws.reported = false;
   ctx->last_algo = params->algo;
   apply_tuning(ctx, params->algo + 256, n);
   const uint32_t n_items = count_items(batch->offsets, count);
@@ -584,7 +589,7 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
     if ((e = enqueue_batch(ctx, m, n, count, words, params, st, true)) != cudaSuccess) return from_cuda(e);
   }
   const ScratchLayout L = scratch_layout(ws.cap_n);
-  if ((e = finish_build(ws, L.ploc, ploc ? 20 : 0, ctx->h_status, st)) != cudaSuccess) return from_cuda(e);
+  if ((e = finish_build(ws, L.ploc, ploc ? 20 : 0, st)) != cudaSuccess) return from_cuda(e);
   cudaEventRecord(ctx->evs.ev[6], st);
   ctx->last_stream = st;
   ctx->have_timing = true;

@@ -16,6 +16,7 @@
 //                 + kRefitHierarchy_nt :243-274).  The node ids are exactly Karras's.
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 
 #include "emit.cuh"
 #include "lbvh.cuh"
@@ -427,6 +428,10 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(const K* __restrict_
   }
 }
 
+}  // namespace bvhgb
+#include "small.cuh"
+namespace bvhgb {
+
 // Onesweep variants (items per thread, look-back window, minimum blocks per SM); the autotuner
 // (bvh_autotune) times them and each context keeps the fastest per key width.
 struct SortVariant {
@@ -471,7 +476,7 @@ cudaError_t prepare_kernels() {
     cudaError_t e = cudaFuncSetAttribute(sv.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sv.smem);
     if (e != cudaSuccess) return e;
   }
-  return cudaSuccess;
+  return prepare_small();
 }
 
 // `passes` stable 8-bit passes over the 32-bit keys in ws.keys[0] (values: the original index).
@@ -617,12 +622,10 @@ __global__ void k_finish(const uint32_t* __restrict__ scratch, size_t status, si
   if (t >= 24) host[t] = __ldcg(scratch + stamps + (t - 24));
 }
 
-cudaError_t finish_build(const Workspace& ws, size_t first, int words, uint32_t* host, cudaStream_t st) {
+cudaError_t finish_build(const Workspace& ws, size_t first, int words, cudaStream_t st) {
+  if (ws.reported) return cudaSuccess;
   const ScratchLayout L = scratch_layout(ws.cap_n);
-  uint32_t* dev = nullptr;
-  cudaError_t e = cudaHostGetDevicePointer(&dev, host, 0);
-  if (e != cudaSuccess) return e;
-  return launch_after(k_finish, 1, 32, 0, st, ws.scratch, L.status, first, words, L.stamps, dev);
+  return launch_after(k_finish, 1, 32, 0, st, ws.scratch, L.status, first, words, L.stamps, ws.report);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -742,7 +745,8 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
 cudaError_t prefix_sort30(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, uint32_t** sorted_idx) {
   ScratchLayout L = scratch_layout(ws.cap_n);
   int fb = 0;
-  cudaError_t e = lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb);
+  cudaError_t e = n <= kSmallMax ? small_build(ws, m, n, 30, kSmallSort, st, L, nullptr)
+                                 : lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb);
   *sorted_idx = ws.vals[fb];
   return e;
 }
@@ -764,6 +768,8 @@ static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchL
                       ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount);
 }
 
+bool one_block_build(uint32_t n) { return n <= kSmallMax; }
+
 cudaError_t run_sort_u32(Workspace& ws, uint32_t n, int passes, cudaStream_t st, const ScratchLayout& L,
                          int* final_buf) {
   return run_sort(ws, n, passes, st, L, final_buf);
@@ -777,7 +783,10 @@ cudaError_t lbvh_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int bits, i
   rec(evs, 0, st);
   int fb = 0;
   const bool parents = treelet_rounds > 0;
-  if (bits == 30) {
+  if (n <= kSmallMax) {
+    e = small_build(ws, m, n, bits, parents ? kSmallLbvhPlus : kSmallLbvh, st, L, parents ? nullptr : ws.report);
+    ws.reported = e == cudaSuccess && ws.report && !parents;
+  } else if (bits == 30) {
     if ((e = lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
     e = parents ? launch_emit<30, true>(ws, fb, n, L, st) : launch_emit<30, false>(ws, fb, n, L, st);
   } else if (bits == 60) {

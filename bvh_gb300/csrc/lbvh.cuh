@@ -73,6 +73,10 @@ struct Workspace {
   // its frontier climb: from there on the leaf nodes [n-1, 2n-1) of a plain LBVH are final; both can
   // be copied out while the rest of the build runs
   cudaEvent_t indices_ready = nullptr, leaves_ready = nullptr;
+  // the report of a build (see finish_build): where it goes (page-locked, or NULL), and whether the
+  // build's own kernel has written it
+  uint32_t* report = nullptr;
+  bool reported = false;
 };
 
 // First epoch value; every build adds kEpochStride (emission uses E, treelet round r uses E+1+r).
@@ -140,8 +144,11 @@ inline cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t bl
 }
 
 // The end of a build: writes its status word, `words` control words from scratch + first and the stage
-// start times to page-locked host memory (32 words: [0] status, [4..] control words, [24..] times).
-cudaError_t finish_build(const Workspace& ws, size_t first, int words, uint32_t* host, cudaStream_t st);
+// start times to ws.report (32 words: [0] status, [4..] control words, [24..] times).
+cudaError_t finish_build(const Workspace& ws, size_t first, int words, cudaStream_t st);
+
+// Meshes of at most this many triangles are built (for PLOC: sorted) by one block in one launch.
+bool one_block_build(uint32_t n);
 
 // LBVH over device-resident SoA input; result in ws.nodes / ws.vals[final].
 // morton_bits: 30, 60 or 63.  treelet_rounds > 0 selects LBVH+.
