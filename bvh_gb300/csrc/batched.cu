@@ -211,10 +211,10 @@ cudaError_t batched_build(Workspace& ws, const MeshPtrs& m, uint32_t n, const ui
   const SegBatch seg{hkeys, d_offsets, 30 - bs.shift0};
   if ((e = launch_after(k_emit<SegBatch, false, kEmitTile>, div_up(n, kEmitTile), kEmitTile, 0, st, ws.delta, nullptr,
                         ws.vals[fb], ws.boxes, ws.nodes, n, seg, d_indices, frontier, fcount, kEmitMaxSteps,
-                        reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps))) != cudaSuccess)
+                        reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps), nullptr)) != cudaSuccess)
     return e;
   return launch_after(k_emit_climb<SegBatch, false>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st, ws.delta,
-                      ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount);
+                      ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount, nullptr);
 }
 
 }  // namespace bvhgb

@@ -21,8 +21,8 @@ struct __align__(16) Node {
   float4 hi;
   int32_t left;
   int32_t right;
-  int32_t aux0;  // parent index while building (unspecified for users of BVHNode)
-  int32_t aux1;
+  int32_t aux0;  // LBVH+: the areas of the left and the right child's box while building, as bits
+  int32_t aux1;  // (unspecified for users of BVHNode)
 };
 static_assert(sizeof(Box) == 32, "AABB_cw is 32 bytes");
 static_assert(sizeof(Node) == 48, "BVHNode is 48 bytes");

@@ -108,35 +108,76 @@ static __global__ void __launch_bounds__(256)
   D[k] = (uint8_t)(d + 1);
 }
 
-template <bool PARENTS>
-__device__ __forceinline__ void write_internal(Node* nodes, uint32_t nb, int32_t my, const Box& box, int32_t lc,
-                                               int32_t rc) {
-  store_node(nodes, nb + (uint32_t)my, box, lc, rc, -1);
-  if (PARENTS) {
-    __stcg(&nodes[nb + lc].aux0, my);
-    __stcg(&nodes[nb + rc].aux0, my);
-  }
-}
-
-// Climb state of one lane: the node it currently owns covers sorted positions [f, l].
+// Climb state of one lane: the node it currently owns covers sorted positions [f, l].  al, ar (its
+// children's areas) and h (its height) are kept for LBVH+ alone.
 struct Climb {
   uint32_t f, l;
   Box box;
   int32_t lc, rc, my;
+  float al, ar;
+  uint32_t h;
   bool internal;
 };
+
+// PLUS: what the treelet passes read of a node besides its box -- the children's areas beside their ids
+// (one 16-byte load when a treelet grows through the node) and its height.
+template <bool PLUS>
+__device__ __forceinline__ void write_internal(Node* nodes, uint8_t* hgt, uint32_t nb, int32_t my, const Climb& c) {
+  if (!PLUS) {
+    store_node(nodes, nb + (uint32_t)my, c.box, c.lc, c.rc, -1);
+    return;
+  }
+  float4* p = reinterpret_cast<float4*>(nodes + nb + (uint32_t)my);
+  __stcg(p, c.box.lo);
+  __stcg(p + 1, c.box.hi);
+  __stcg(reinterpret_cast<int4*>(p + 2), make_int4(c.lc, c.rc, __float_as_int(c.al), __float_as_int(c.ar)));
+  __stcg(hgt + nb + (uint32_t)my, (uint8_t)min(c.h, 255u));
+}
+
+// The lane's node becomes the parent of itself and its sibling `sib` (height hs), the right one when is_left.
+// PLUS: the first treelet pass turns the children of a node of height 1 round (its two-leaf treelet's
+// only split puts the second leaf left; not where the area is NaN); here they are written that way at once.
+template <bool PLUS>
+__device__ __forceinline__ void climb_merge(Climb& c, bool is_left, int32_t sib_id, const Box& sib, uint32_t hs) {
+  if (PLUS) {
+    const float mine = box_area(c.box), other = box_area(sib);
+    c.al = is_left ? mine : other;
+    c.ar = is_left ? other : mine;
+  }
+  if (is_left) {
+    c.lc = c.my;
+    c.rc = sib_id;
+    c.box = box_union(c.box, sib);
+  } else {
+    c.lc = sib_id;
+    c.rc = c.my;
+    c.box = box_union(sib, c.box);
+  }
+  if (PLUS) {
+    c.h = 1u + max(c.h, hs);
+    if (c.h == 1u && box_area(c.box) > -1.0f) {
+      const int32_t t = c.lc;
+      c.lc = c.rc;
+      c.rc = t;
+      const float u = c.al;
+      c.al = c.ar;
+      c.ar = u;
+    }
+  }
+}
 
 // T sorted positions per block, one thread each (a larger block leaves fewer nodes whose sibling
 // lies in another block to the frontier pass).
 // KEYS30: the tile's delta bytes are computed here from the sorted 30-bit keys (the delta_nt
 // rule, as k_delta) and written to D for k_emit_climb; otherwise they are read from D.
-template <typename Seg, bool PARENTS, uint32_t T = 256, bool KEYS30 = false>
+template <typename Seg, bool PLUS, uint32_t T = 256, bool KEYS30 = false>
 __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, const uint32_t* __restrict__ keys30,
                                             const uint32_t* __restrict__ vals,
                                             const Box* __restrict__ tri_boxes, Node* __restrict__ nodes,
                                             uint32_t n, Seg seg, uint32_t* __restrict__ out_idx,
                                             uint2* __restrict__ frontier, uint32_t* __restrict__ frontier_count,
-                                            uint32_t max_steps, unsigned long long* __restrict__ stamps) {
+                                            uint32_t max_steps, unsigned long long* __restrict__ stamps,
+                                            uint8_t* __restrict__ hgt) {
   // D of positions bbase-1 .. bbase+T-1 (0 outside [0, n-1) : a segment boundary)
   __shared__ uint8_t s_D[T + 1];
   // KEYS30: keys and values of positions bbase-1 .. bbase+T
@@ -146,6 +187,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   __shared__ uint32_t s_flag[T];
   __shared__ float4 s_lo[2][T];
   __shared__ float4 s_hi[2][T];
+  __shared__ uint8_t s_h[2][PLUS ? T : 1];  // the child's height
   const uint32_t tid = threadIdx.x;
   const uint32_t i = blockIdx.x * T + tid;
   const uint32_t bbase = blockIdx.x * T;  // sorted position of thread 0
@@ -159,6 +201,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   c.lc = c.rc = -1;
   c.internal = false;
   c.my = 0;
+  c.h = 0;
   if (active) {
     seg.get(i, off, cnt, nb);
     const uint32_t prim_g = __ldcg(vals + i);
@@ -213,7 +256,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     const int dl = (int)s_D[c.f - bbase] - 1;
     const int dr = (int)s_D[c.l - bbase + 1] - 1;
     if (dl < 0 && dr < 0) {  // segment root
-      write_internal<PARENTS>(nodes, nb, 0, c.box, c.lc, c.rc);
+      write_internal<PLUS>(nodes, hgt, nb, 0, c);
       break;
     }
     const bool is_left = dr > dl;
@@ -223,35 +266,30 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     // sibling starts outside the block, or the climb has gone max_steps levels: the node
     // continues in k_emit_climb, so that one long chain does not hold the block
     if (step >= max_steps || (is_left ? gamma + 1 >= bbase + T : gamma < bbase)) {
-      if (pending) write_internal<PARENTS>(nodes, nb, c.my, c.box, c.lc, c.rc);
+      if (pending) write_internal<PLUS>(nodes, hgt, nb, c.my, c);
       to_frontier = true;
       break;
     }
-    // with parent links the node is written before the rendezvous, so that the parent's later
-    // write of its aux0 lands last
-    if (PARENTS && pending) write_internal<PARENTS>(nodes, nb, c.my, c.box, c.lc, c.rc);
     const uint32_t k = gamma - bbase;
     const int side = is_left ? 0 : 1;
     s_lo[side][k] = make_float4(c.box.lo.x, c.box.lo.y, c.box.lo.z, __int_as_float(c.my));
     s_hi[side][k] = make_float4(c.box.hi.x, c.box.hi.y, c.box.hi.z, __uint_as_float(is_left ? c.f : c.l));
+    if (PLUS) s_h[side][k] = (uint8_t)c.h;  // (at most T)
     // release: the slot is visible before the flag bit; acquire: the sibling's slot is read after
     const uint32_t prev = atom_or_acq_rel_cta(&s_flag[k], 1u << side);
-    if (!PARENTS && pending) write_internal<PARENTS>(nodes, nb, c.my, c.box, c.lc, c.rc);
+    if (pending) write_internal<PLUS>(nodes, hgt, nb, c.my, c);
     if (prev == 0u) break;  // first to arrive
     const float4 a = s_lo[side ^ 1][k], b = s_hi[side ^ 1][k];
     Box sb;
     sb.lo = make_float4(a.x, a.y, a.z, 0.f);
     sb.hi = make_float4(b.x, b.y, b.z, 0.f);
+    const uint32_t hs = PLUS ? s_h[side ^ 1][k] : 0u;
     if (is_left) {
-      c.lc = c.my;
-      c.rc = __float_as_int(a.w);
       c.l = __float_as_uint(b.w);
-      c.box = box_union(c.box, sb);
+      climb_merge<PLUS>(c, true, __float_as_int(a.w), sb, hs);
     } else {
-      c.lc = __float_as_int(a.w);
-      c.rc = c.my;
       c.f = __float_as_uint(b.w);
-      c.box = box_union(sb, c.box);
+      climb_merge<PLUS>(c, false, __float_as_int(a.w), sb, hs);
     }
     c.internal = true;
   }
@@ -285,12 +323,13 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
 
 // Climb from every frontier node (a finished node whose parent needs a sibling built by
 // another block) through the rendezvous words; the second child to arrive completes the parent.
-template <typename Seg, bool PARENTS>
+template <typename Seg, bool PLUS>
 __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ D, Node* __restrict__ nodes,
                                                     unsigned long long* __restrict__ slots,
                                                     const uint32_t* epoch_word, uint32_t n, Seg seg,
                                                     const uint2* __restrict__ frontier,
-                                                    const uint32_t* __restrict__ frontier_count) {
+                                                    const uint32_t* __restrict__ frontier_count,
+                                                    uint8_t* __restrict__ hgt) {
   after_previous();
   const uint32_t count = __ldcg(frontier_count);
   const unsigned long long tag = (unsigned long long)__ldcg(epoch_word) << 32;
@@ -307,6 +346,7 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
     uint32_t gamma = is_left ? c.l : c.f - 1;
     c.my = c.f == c.l ? (int32_t)(cnt - 1 + (c.f - off)) : (int32_t)((is_left ? c.l : c.f) - off);
     c.box = load_node_box(nodes, nb + (uint32_t)c.my);
+    c.h = PLUS && c.f != c.l ? __ldcg(hgt + nb + (uint32_t)c.my) : 0u;
     while (true) {
       const uint32_t far = is_left ? c.f : c.l;
       const unsigned long long old = atom_exch_acq_rel(slots + gamma, tag | far);
@@ -316,27 +356,25 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
       int32_t sib;
       if (is_left) {
         sib = (other == gamma + 1) ? (int32_t)cnt + g : g + 1;
-        c.lc = c.my;
-        c.rc = sib;
+        const uint32_t hs = PLUS && other != gamma + 1 ? __ldcg(hgt + nb + (uint32_t)sib) : 0u;
         c.l = other;
-        c.box = box_union(c.box, load_node_box(nodes, nb + (uint32_t)sib));
+        climb_merge<PLUS>(c, true, sib, load_node_box(nodes, nb + (uint32_t)sib), hs);
       } else {
         sib = (other == gamma) ? (int32_t)cnt - 1 + g : g;
-        c.lc = sib;
-        c.rc = c.my;
+        const uint32_t hs = PLUS && other != gamma ? __ldcg(hgt + nb + (uint32_t)sib) : 0u;
         c.f = other;
-        c.box = box_union(load_node_box(nodes, nb + (uint32_t)sib), c.box);
+        climb_merge<PLUS>(c, false, sib, load_node_box(nodes, nb + (uint32_t)sib), hs);
       }
       dl = c.f == 0 ? -1 : (int)__ldg(D + c.f - 1) - 1;
       dr = c.l + 1 >= n ? -1 : (int)__ldg(D + c.l) - 1;
       if (dl < 0 && dr < 0) {
-        write_internal<PARENTS>(nodes, nb, 0, c.box, c.lc, c.rc);
+        write_internal<PLUS>(nodes, hgt, nb, 0, c);
         break;
       }
       is_left = dr > dl;
       gamma = is_left ? c.l : c.f - 1;
       c.my = (int32_t)((is_left ? c.l : c.f) - off);
-      write_internal<PARENTS>(nodes, nb, c.my, c.box, c.lc, c.rc);
+      write_internal<PLUS>(nodes, hgt, nb, c.my, c);
     }
   }
 }

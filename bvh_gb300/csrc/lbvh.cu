@@ -34,6 +34,7 @@ ScratchLayout scratch_layout(uint32_t n) {
   L.status = o; o += 1;
   L.ticket = o; o += 1;
   L.epoch = o; o += 1;
+  L.wild = o; o += 1;
   o = (o + 3) & ~size_t(3);
   L.scene = o; o += 8;
   L.ploc = o; o += 20;
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(256) k_bounds(MeshPtrs m, uint32_t n, int vec4
     for (size_t w = L.zero_begin + words4 * 4 + gtid; w < L.zero_end; w += gsz) scratch[w] = 0;
     if (gtid == 0) {
       scratch[L.status] = 0;
+      scratch[L.wild] = 0;
       uint32_t e = scratch[L.epoch] + kEpochStride;
       scratch[L.epoch] = e < kEpochStride ? kEpochStride : e;
     }
@@ -191,9 +193,19 @@ __device__ __forceinline__ K tri_code(float x0, float y0, float z0, float x1, fl
   return (K)morton_code<BITS>(nx, ny, nz);
 }
 
+// A box whose coordinates are finite and at most 1e13 in magnitude.  Where all are, every area is a number
+// below 1e28, every treelet has a split that costs less than the subset DP's infinity, and a node's box is
+// the union of its leaves' however they are grouped, so LBVH+ need not refit it.
+__device__ __forceinline__ bool tame_box(const Box& b) {
+  constexpr float kTame = 1e13f;
+  return fabsf(b.lo.x) <= kTame && fabsf(b.lo.y) <= kTame && fabsf(b.lo.z) <= kTame && fabsf(b.hi.x) <= kTame &&
+         fabsf(b.hi.y) <= kTame && fabsf(b.hi.z) <= kTame;
+}
+
 // Codes of more than 32 bits are written split: keys = the high 32 bits (code >> (BITS - 32)),
 // which the radix passes sort, and lows = the rest, in input order.
-template <int BITS, typename K>
+// PLUS: whether some box is not tame goes to the scratch (6 compares per triangle: 2% of the kernel).
+template <int BITS, typename K, bool PLUS>
 __global__ void __launch_bounds__(256) k_morton(MeshPtrs m, uint32_t n, int vec4, uint32_t* __restrict__ keys,
                                                 uint32_t* __restrict__ lows, Box* __restrict__ boxes,
                                                 uint32_t* __restrict__ scratch, ScratchLayout L) {
@@ -212,6 +224,7 @@ __global__ void __launch_bounds__(256) k_morton(MeshPtrs m, uint32_t n, int vec4
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gsz = gridDim.x * blockDim.x;
   uint32_t done = 0;
+  bool wild = false;
   if (vec4) {
     const uint32_t n4 = n >> 2;
     const float4* p[9];
@@ -237,6 +250,7 @@ __global__ void __launch_bounds__(256) k_morton(MeshPtrs m, uint32_t n, int vec4
       for (int e = 0; e < 4; ++e) {
         bp[2 * e] = b[e].lo;
         bp[2 * e + 1] = b[e].hi;
+        if (PLUS) wild |= !tame_box(b[e]);
 #pragma unroll
         for (int p2 = 0; p2 < P; ++p2) atomicAdd(&s_hist[p2][(uint32_t)(c[e] >> (S0 + 8 * p2)) & 255u], 1u);
       }
@@ -250,10 +264,12 @@ __global__ void __launch_bounds__(256) k_morton(MeshPtrs m, uint32_t n, int vec4
     keys[i] = (uint32_t)(c >> S0);
     if constexpr (sizeof(K) == 8) lows[i] = (uint32_t)(c & kLowMask);
     boxes[i] = b;
+    if (PLUS) wild |= !tame_box(b);
 #pragma unroll
     for (int p2 = 0; p2 < P; ++p2) atomicAdd(&s_hist[p2][(uint32_t)(c >> (S0 + 8 * p2)) & 255u], 1u);
   }
-  __syncthreads();
+  const int any = PLUS ? __syncthreads_or(wild) : (__syncthreads(), 0);
+  if (PLUS && any && threadIdx.x == 0) atomicOr(scratch + L.wild, 1u);
   uint32_t* gh = scratch + L.hist;
   for (int i = threadIdx.x; i < P * 256; i += blockDim.x) {
     uint32_t c = (&s_hist[0][0])[i];
@@ -635,11 +651,13 @@ void workspace_free(Workspace& ws) {
   cudaFree(ws.keys[0]); cudaFree(ws.keys[1]);
   cudaFree(ws.vals[0]); cudaFree(ws.vals[1]);
   cudaFree(ws.boxes); cudaFree(ws.nodes); cudaFree(ws.slots); cudaFree(ws.scratch); cudaFree(ws.delta);
+  cudaFree(ws.heights);
   if (ws.ploc_exec) cudaGraphExecDestroy(ws.ploc_exec);
   if (ws.ploc_seg_exec) cudaGraphExecDestroy(ws.ploc_seg_exec);
   if (ws.aux_stream) cudaStreamDestroy(ws.aux_stream);
   if (ws.ploc_host) cudaFreeHost(ws.ploc_host);
-  if (ws.tl_exec) cudaGraphExecDestroy(ws.tl_exec);
+  for (cudaGraphExec_t x : ws.tl_exec)
+    if (x) cudaGraphExecDestroy(x);
   cudaFree(ws.cbox[0]); cudaFree(ws.cbox[1]); cudaFree(ws.cid[0]); cudaFree(ws.cid[1]); cudaFree(ws.nbr);
   cudaFree(ws.mesh_dev);
   cudaFree(ws.bat_offsets); cudaFreeHost(ws.bat_offsets_h); cudaFree(ws.bat_mbox); cudaFree(ws.bat_indices);
@@ -665,8 +683,9 @@ cudaError_t workspace_reserve(Workspace& ws, uint32_t n, cudaStream_t st) {
   uint32_t cap = std::max<uint32_t>(n, 1024);
   cudaFree(ws.keys[0]); cudaFree(ws.keys[1]); cudaFree(ws.vals[0]); cudaFree(ws.vals[1]);
   cudaFree(ws.boxes); cudaFree(ws.nodes); cudaFree(ws.slots); cudaFree(ws.scratch); cudaFree(ws.delta);
+  cudaFree(ws.heights);
   ws.keys[0] = ws.keys[1] = nullptr; ws.vals[0] = ws.vals[1] = nullptr;
-  ws.boxes = nullptr; ws.nodes = nullptr; ws.slots = nullptr; ws.scratch = nullptr; ws.delta = nullptr;
+  ws.boxes = nullptr; ws.nodes = nullptr; ws.slots = nullptr; ws.scratch = nullptr; ws.delta = nullptr; ws.heights = nullptr;
   ws.cap_n = 0;
   cudaError_t e;
   if ((e = cudaMalloc(&ws.keys[0], (size_t)cap * 8)) != cudaSuccess) return e;
@@ -677,6 +696,7 @@ cudaError_t workspace_reserve(Workspace& ws, uint32_t n, cudaStream_t st) {
   if ((e = cudaMalloc(&ws.nodes, (2 * (size_t)cap) * sizeof(Node))) != cudaSuccess) return e;
   if ((e = cudaMalloc(&ws.slots, (size_t)cap * 8)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&ws.delta, (size_t)cap + 16)) != cudaSuccess) return e;
+  if ((e = cudaMalloc(&ws.heights, (size_t)cap + 16)) != cudaSuccess) return e;
   ScratchLayout L = scratch_layout(cap);
   if ((e = cudaMalloc(&ws.scratch, L.total * 4)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(ws.slots, 0, (size_t)cap * 8, st)) != cudaSuccess) return e;
@@ -711,7 +731,7 @@ static inline uint32_t* split_long_list(const Workspace& ws, uint32_t n) {
 
 template <int BITS, typename K>
 static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, const ScratchLayout& L,
-                               int* final_buf) {
+                               int* final_buf, bool plus) {
   uint32_t* lows = sizeof(K) == 8 ? split_lows(ws) : nullptr;
   const int vec4 = all_aligned16(m) && (reinterpret_cast<uintptr_t>(lows) & 15) == 0 ? 1 : 0;
   // zero only the descriptors the current build's passes use (the passes sort 32-bit keys)
@@ -724,7 +744,7 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(div_up(work, 256), 152 * 8));
   // (the bounds partials and the last block's arrival count grow with the grid: no idle blocks)
   k_bounds<<<std::min<uint32_t>(grid, kBoundsBlocks), 256, 0, st>>>(m, n, vec4, ws.scratch, Lz);
-  if ((et = launch_after(k_morton<BITS, K>, grid, 256, 0, st, m, n, vec4, reinterpret_cast<uint32_t*>(ws.keys[0]), lows,
+  if ((et = launch_after(plus ? k_morton<BITS, K, true> : k_morton<BITS, K, false>, grid, 256, 0, st, m, n, vec4, reinterpret_cast<uint32_t*>(ws.keys[0]), lows,
                          ws.boxes, ws.scratch, L)) != cudaSuccess)
     return et;
   // 4 passes sort the 32-bit keys: the whole 30-bit code, or the high 32 bits of a 60/63-bit
@@ -746,12 +766,12 @@ cudaError_t prefix_sort30(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStre
   ScratchLayout L = scratch_layout(ws.cap_n);
   int fb = 0;
   cudaError_t e = n <= kSmallMax ? small_build(ws, m, n, 30, kSmallSort, st, L, nullptr)
-                                 : lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb);
+                                 : lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb, false);
   *sorted_idx = ws.vals[fb];
   return e;
 }
 
-template <int BITS, bool PARENTS>
+template <int BITS, bool PLUS>
 static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchLayout& L, cudaStream_t st) {
   const uint32_t* keys = reinterpret_cast<const uint32_t*>(ws.keys[fb]);
   const uint32_t* epoch = ws.scratch + L.epoch;
@@ -759,13 +779,13 @@ static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchL
   uint2* frontier = reinterpret_cast<uint2*>(ws.keys[fb ^ 1]);  // the sort's other key buffer, 8 B per position
   // delta bytes: computed by k_emit from the 30-bit keys, written by the run fix-up for 60/63 bits
   unsigned long long* stamps = reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps);
-  cudaError_t e = launch_after(k_emit<SegSingle, PARENTS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
+  cudaError_t e = launch_after(k_emit<SegSingle, PLUS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
                                ws.delta, keys, ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier,
-                               fcount, kEmitMaxSteps, stamps);
+                               fcount, kEmitMaxSteps, stamps, ws.heights);
   if (e != cudaSuccess) return e;
-  if (ws.leaves_ready && !PARENTS) cudaEventRecord(ws.leaves_ready, st);
-  return launch_after(k_emit_climb<SegSingle, PARENTS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
-                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount);
+  if (ws.leaves_ready && !PLUS) cudaEventRecord(ws.leaves_ready, st);
+  return launch_after(k_emit_climb<SegSingle, PLUS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
+                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount, ws.heights);
 }
 
 bool one_block_build(uint32_t n) { return n <= kSmallMax; }
@@ -782,22 +802,22 @@ cudaError_t lbvh_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int bits, i
   ScratchLayout L = scratch_layout(ws.cap_n);
   rec(evs, 0, st);
   int fb = 0;
-  const bool parents = treelet_rounds > 0;
+  const bool plus = treelet_rounds > 0 && n >= 2;
   if (n <= kSmallMax) {
-    e = small_build(ws, m, n, bits, parents ? kSmallLbvhPlus : kSmallLbvh, st, L, parents ? nullptr : ws.report);
-    ws.reported = e == cudaSuccess && ws.report && !parents;
+    e = small_build(ws, m, n, bits, plus ? kSmallLbvhPlus : kSmallLbvh, st, L, plus ? nullptr : ws.report);
+    ws.reported = e == cudaSuccess && ws.report && !plus;
   } else if (bits == 30) {
-    if ((e = lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
-    e = parents ? launch_emit<30, true>(ws, fb, n, L, st) : launch_emit<30, false>(ws, fb, n, L, st);
+    if ((e = lbvh_prefix<30, uint32_t>(ws, m, n, st, L, &fb, plus)) != cudaSuccess) return e;
+    e = plus ? launch_emit<30, true>(ws, fb, n, L, st) : launch_emit<30, false>(ws, fb, n, L, st);
   } else if (bits == 60) {
-    if ((e = lbvh_prefix<60, unsigned long long>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
-    e = parents ? launch_emit<60, true>(ws, fb, n, L, st) : launch_emit<60, false>(ws, fb, n, L, st);
+    if ((e = lbvh_prefix<60, unsigned long long>(ws, m, n, st, L, &fb, plus)) != cudaSuccess) return e;
+    e = plus ? launch_emit<60, true>(ws, fb, n, L, st) : launch_emit<60, false>(ws, fb, n, L, st);
   } else {
-    if ((e = lbvh_prefix<63, unsigned long long>(ws, m, n, st, L, &fb)) != cudaSuccess) return e;
-    e = parents ? launch_emit<63, true>(ws, fb, n, L, st) : launch_emit<63, false>(ws, fb, n, L, st);
+    if ((e = lbvh_prefix<63, unsigned long long>(ws, m, n, st, L, &fb, plus)) != cudaSuccess) return e;
+    e = plus ? launch_emit<63, true>(ws, fb, n, L, st) : launch_emit<63, false>(ws, fb, n, L, st);
   }
   if (e != cudaSuccess) return e;
-  if (treelet_rounds > 0 && n >= 2) {
+  if (plus) {
     rec(evs, 4, st);
     if (evs) evs->split = evs->use;
     e = treelet_rounds_run(ws, n, treelet_rounds, st, fb, host_loops);

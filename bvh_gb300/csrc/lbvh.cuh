@@ -29,6 +29,7 @@ struct Workspace {
   unsigned long long* slots = nullptr;  // n-1 rendezvous words (epoch << 32 | endpoint)
   uint32_t* scratch = nullptr;          // histograms, look-back descriptors, counters
   uint8_t* delta = nullptr;             // n-1 adjacent common-prefix lengths (+1)
+  uint8_t* heights = nullptr;           // LBVH+: n-1 inner nodes' heights (at most 255)
   size_t scratch_words = 0;
   // PLOC buffers
   Box* cbox[2] = {nullptr, nullptr};
@@ -37,7 +38,8 @@ struct Workspace {
   uint32_t ploc_cap = 0;
   cudaGraphExec_t ploc_exec = nullptr;  // clustering loop graph, valid for the key below
   uint32_t* ploc_host = nullptr;        // pinned words for the host-driven loops
-  cudaGraphExec_t tl_exec = nullptr;    // LBVH+ loop over heights, valid for the key below
+  // LBVH+ loop over heights, valid for the key below: [1] keeps the heights for a further pass
+  cudaGraphExec_t tl_exec[2] = {nullptr, nullptr};
   uint32_t tl_key_n = 0;
   const void* tl_key_nodes = nullptr;
   const void* tl_key_list = nullptr;
@@ -90,6 +92,7 @@ struct ScratchLayout {
   size_t status;     // 1 word, device status bits
   size_t ticket;     // 1 word, bounds-reduction arrival counter (self-resetting)
   size_t epoch;      // 1 word, rendezvous tag of the current build (bumped by 64 per build)
+  size_t wild;       // 1 word, nonzero: some triangle's box is not tame (see tame_box)
   size_t scene;      // 8 words, SceneParams
   size_t counters;   // 16 words, per-pass tile counters
   size_t hist;       // passes * 256

@@ -38,6 +38,7 @@ struct SmallShared {
     struct {
       float4 lo[2][CAP], hi[2][CAP];  // a child's box with its id (lo.w) and far end (hi.w), by side and split
       uint32_t flag[CAP];
+      uint8_t h[2][CAP];  // the child's height (LBVH+)
     } climb;
   };
 };
@@ -112,7 +113,7 @@ __device__ __forceinline__ void small_pass(SmallShared<K, IPT>& S, K (&key)[IPT]
 template <int BITS, int MODE, int IPT>
 __global__ void __launch_bounds__(kSmallThreads, 1)
     k_small(MeshPtrs m, uint32_t n, uint32_t* __restrict__ vals, Box* __restrict__ boxes, Node* __restrict__ nodes,
-            uint32_t* __restrict__ scratch, ScratchLayout L, uint32_t* __restrict__ host) {
+            uint32_t* __restrict__ scratch, ScratchLayout L, uint32_t* __restrict__ host, uint8_t* __restrict__ hgt) {
   using K = typename std::conditional<BITS == 30, uint32_t, unsigned long long>::type;
   using Shared = SmallShared<K, IPT>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   stage_stamp(stamps, 1);
   K key[IPT];
   uint32_t val[IPT];
+  bool wild = false;
 #pragma unroll
   for (int k = 0; k < IPT; ++k) {
     const uint32_t i = (uint32_t)w * 32u * IPT + (uint32_t)k * 32u + lane;
@@ -169,6 +171,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       Box b;
       key[k] = tri_code<BITS, K>(v[k][0], v[k][1], v[k][2], v[k][3], v[k][4], v[k][5], v[k][6], v[k][7], v[k][8], S.scene,
                                  S.scene + 3, b);
+      if (MODE == kSmallLbvhPlus) wild |= !tame_box(b);
       if (MODE == kSmallSort) {
         boxes[i] = b;
       } else {
@@ -176,6 +179,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
         S.box[3][i] = b.hi.x; S.box[4][i] = b.hi.y; S.box[5][i] = b.hi.z;
       }
     }
+  }
+  if (MODE == kSmallLbvhPlus) {
+    wild = __syncthreads_or(wild);
+    if (t == 0) scratch[L.wild] = wild ? 1u : 0u;
   }
   // ---- sort ----
   stage_stamp(stamps, 2);
@@ -201,13 +208,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   for (uint32_t k = t; k < n; k += kSmallThreads) S.climb.flag[k] = 0;
   __syncthreads();
   // ---- climb: as k_emit, every rendezvous inside the block ----
-  constexpr bool PARENTS = MODE == kSmallLbvhPlus;
+  constexpr bool PLUS = MODE == kSmallLbvhPlus;
   for (uint32_t i = t; i < n; i += kSmallThreads) {
     const uint32_t prim = S.val[i];
     Climb c;
     c.f = c.l = i;
     c.lc = c.rc = -1;
     c.internal = false;
+    c.h = 0;
     c.box.lo = make_float4(S.box[0][prim], S.box[1][prim], S.box[2][prim], 0.f);
     c.box.hi = make_float4(S.box[3][prim], S.box[4][prim], S.box[5][prim], 0.f);
     c.my = (int32_t)(n - 1 + i);
@@ -215,35 +223,26 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     while (true) {
       const int dl = (int)S.D[c.f] - 1, dr = (int)S.D[c.l + 1] - 1;
       if (dl < 0 && dr < 0) {  // the root (a one-triangle mesh: its leaf)
-        if (c.internal) write_internal<PARENTS>(nodes, 0, 0, c.box, c.lc, c.rc);
+        if (c.internal) write_internal<PLUS>(nodes, hgt, 0, 0, c);
         break;
       }
       const bool is_left = dr > dl, pending = c.internal;
       const uint32_t gamma = is_left ? c.l : c.f - 1;
       if (pending) c.my = (int32_t)(is_left ? c.l : c.f);
-      // with parent links the node is written before the rendezvous, so that its parent's link lands last
-      if (PARENTS && pending) write_internal<PARENTS>(nodes, 0, c.my, c.box, c.lc, c.rc);
       const int side = is_left ? 0 : 1;
       S.climb.lo[side][gamma] = make_float4(c.box.lo.x, c.box.lo.y, c.box.lo.z, __int_as_float(c.my));
       S.climb.hi[side][gamma] = make_float4(c.box.hi.x, c.box.hi.y, c.box.hi.z, __uint_as_float(is_left ? c.f : c.l));
+      if (PLUS) S.climb.h[side][gamma] = (uint8_t)c.h;  // (at most 95: the code's bits and 32)
       const uint32_t prev = atom_or_acq_rel_cta(&S.climb.flag[gamma], 1u << side);
-      if (!PARENTS && pending) write_internal<PARENTS>(nodes, 0, c.my, c.box, c.lc, c.rc);
+      if (pending) write_internal<PLUS>(nodes, hgt, 0, c.my, c);
       if (prev == 0u) break;  // first to arrive
       const float4 a = S.climb.lo[side ^ 1][gamma], b = S.climb.hi[side ^ 1][gamma];
       Box sib;
       sib.lo = make_float4(a.x, a.y, a.z, 0.f);
       sib.hi = make_float4(b.x, b.y, b.z, 0.f);
-      if (is_left) {
-        c.lc = c.my;
-        c.rc = __float_as_int(a.w);
-        c.l = __float_as_uint(b.w);
-        c.box = box_union(c.box, sib);
-      } else {
-        c.lc = __float_as_int(a.w);
-        c.rc = c.my;
-        c.f = __float_as_uint(b.w);
-        c.box = box_union(sib, c.box);
-      }
+      climb_merge<PLUS>(c, is_left, __float_as_int(a.w), sib, PLUS ? S.climb.h[side ^ 1][gamma] : 0u);
+      if (is_left) c.l = __float_as_uint(b.w);
+      else c.f = __float_as_uint(b.w);
       c.internal = true;
     }
   }
@@ -280,7 +279,7 @@ static cudaError_t small_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int
   const void* fn = small_kernel(bits, mode, n, &smem);
   MeshPtrs mp = m;
   ScratchLayout Lc = L;
-  void* args[] = {&mp, &n, &ws.vals[0], &ws.boxes, &ws.nodes, &ws.scratch, &Lc, &host};
+  void* args[] = {&mp, &n, &ws.vals[0], &ws.boxes, &ws.nodes, &ws.scratch, &Lc, &host, &ws.heights};
   return cudaLaunchKernel(fn, dim3(1), dim3(kSmallThreads), args, smem, st);
 }
 

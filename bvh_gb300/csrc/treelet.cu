@@ -42,6 +42,25 @@ __device__ __forceinline__ int2 ldcg_children(const Node* nodes, int32_t idx) {
   return __ldcg(reinterpret_cast<const int2*>(&nodes[idx].left));
 }
 
+// What a treelet's growth reads of an inner node: its children and their areas.  Every inner node carries the
+// areas of its children's boxes as they are (see write_internal; the passes below keep them so), so a
+// treelet grows through one 16-byte load per expanded node instead of two 48-byte children.
+struct Links {
+  int32_t l, r;
+  float al, ar;
+};
+__device__ __forceinline__ Links ldcg_links(const Node* nodes, int32_t idx) {
+  const int4 v = __ldcg(reinterpret_cast<const int4*>(&nodes[idx].left));
+  return Links{v.x, v.y, __int_as_float(v.z), __int_as_float(v.w)};
+}
+__device__ __forceinline__ void stcg_links(Node* nodes, int32_t idx, const Links& k) {
+  __stcg(reinterpret_cast<int4*>(&nodes[idx].left), make_int4(k.l, k.r, __float_as_int(k.al), __float_as_int(k.ar)));
+}
+// Height of node idx (leaves, from first_leaf on: 0).
+__device__ __forceinline__ uint32_t node_height(const uint8_t* hgt, int32_t first_leaf, int32_t idx) {
+  return idx < first_leaf ? (uint32_t)__ldcg(hgt + idx) : 0u;
+}
+
 // Subsets of {0..6} with 2..7 members, by size, increasing within a size.  For a treelet of
 // n < 7 leaves the subsets of its full mask are the entries <= (1 << n) - 1, in the same order.
 __constant__ uint8_t c_subsets[120] = {
@@ -80,18 +99,6 @@ __device__ __forceinline__ void set_leaf(LaneTreelet& T, int i, int32_t id, cons
   T.chr[i] = ch.y;
 }
 
-// pdep of the low bits of m into the set bits of mask (m-th nonempty subset of mask in
-// increasing numeric order, m >= 1).
-__device__ __forceinline__ uint32_t deposit_bits(uint32_t m, uint32_t mask) {
-  uint32_t r = 0;
-  for (uint32_t bit = 1; mask; bit <<= 1) {
-    uint32_t low = mask & (0u - mask);
-    if (m & bit) r |= low;
-    mask ^= low;
-  }
-  return r;
-}
-
 // 1. Grow the treelet at `root` (lbvh_plus_builder.cu:73-114): up to 6 times, expand the leaf
 //    with the largest area among those that are internal nodes (first such on ties).  Run by
 //    one lane; the lanes of a warp grow their own treelets side by side.
@@ -122,64 +129,139 @@ __device__ void treelet_grow(const Node* nodes, int32_t root, LaneTreelet& T) {
   T.n = cnt;
 }
 
+// The split p of s with the smallest cost among `count` from the (first+1)-th of its enumeration on (p =
+// the nonempty subsets of s without its lowest member, increasing); the first of equals; 0 where none is
+// below INF.  Unrolled, so that all cost loads are in flight together.
+template <int COUNT>
+__device__ __forceinline__ float scan_splits(const float* cost, uint32_t s, uint32_t first, uint32_t end, uint32_t& bp) {
+  const uint32_t delta = s & (s - 1u);
+  // the (first+1)-th nonempty subset of delta: the bits of first + 1 spread over delta's members
+  uint32_t p = 0, rest = delta;
+#pragma unroll
+  for (int i = 0; i < kTlMax - 1; ++i) {
+    const uint32_t low = rest & (0u - rest);
+    p |= ((first + 1u) >> i) & 1u ? low : 0u;
+    rest ^= low;
+  }
+  float v[COUNT];
+  uint32_t q[COUNT];
+#pragma unroll
+  for (int k = 0; k < COUNT; ++k) {
+    q[k] = p;
+    v[k] = first + (uint32_t)k < end ? __fadd_rn(cost[p], cost[s ^ p]) : kTlInf;
+    p = (p - delta) & delta;
+  }
+  float best = kTlInf;
+  bp = 0;
+#pragma unroll
+  for (int k = 0; k < COUNT; ++k)
+    if (v[k] < best) {
+      best = v[k];
+      bp = q[k];
+    }
+  return best;
+}
+
+// One size K of the DP: COUNT subsets from c_subsets[c_sub_off[K]], two per lane side by side.
+template <int K>
+__device__ __forceinline__ void warp_dp_size(LaneTreelet& T, float* cost, const float* area, uint32_t full) {
+  constexpr uint32_t kParts = (1u << (K - 1)) - 1u;
+  const uint32_t lane = threadIdx.x & 31, base = c_sub_off[K], count = c_sub_off[K + 1] - base;
+  uint32_t s[2], bp[2];
+  float best[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t e = lane + 32u * i;
+    s[i] = e < count ? c_subsets[base + e] : 0u;
+    if (s[i] > full) s[i] = 0;
+    best[i] = s[i] ? scan_splits<(int)kParts>(cost, s[i], 0, kParts, bp[i]) : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (s[i]) {
+      cost[s[i]] = __fadd_rn(best[i], area[s[i]]);  // (no split below INF: INF plus the area, and split 0)
+      T.part[s[i]] = (uint8_t)bp[i];
+    }
+  __syncwarp();
+}
+
+// A float's bits as an unsigned number of the same order (no NaN).
+__device__ __forceinline__ uint32_t ordered_bits(float v) {
+  const uint32_t u = __float_as_uint(v);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+
 // 2+3. Subset areas and the DP over subsets by size (:119-165), by the whole warp for one
-//    lane's treelet.  cost[s] = min over splits (cost[p] + cost[s^p]) + area[s], leaves cost 0;
+//    treelet.  cost[s] = min over splits (cost[p] + cost[s^p]) + area[s], leaves cost 0;
 //    the best split is the first minimum in the enumeration p = increasing nonempty subsets of
-//    s without its lowest member.  Sizes 2..5 take one lane per subset, size 6 four lanes and
-//    size 7 the whole warp, each lane scanning a contiguous run of that enumeration.
+//    s without its lowest member.  Sizes 3 to 5 take one lane per subset, size 6 four lanes and
+//    size 7 the whole warp.  A chain of five sizes: bound by latency, so each size's loads are issued
+//    together (one node of k_tl_narrow: see there).
 __device__ void treelet_dp(LaneTreelet& T, float* cost, float* area) {
-  const int lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31;
   const int n = T.n;
   const uint32_t full = (1u << n) - 1u;
-  for (uint32_t s = 1 + lane; s <= full; s += 32) {
-    Box b = box_empty();
+  // lane's subsets lane + 32 {0..3}: the members among leaves 0..4 once, then with leaves 5, 6, both
+  Box low = box_empty();
 #pragma unroll
-    for (int i = 0; i < kTlMax; ++i)
-      if ((s >> i) & 1u) b = box_union(b, leaf_box(T, i));
-    area[s] = box_area(b);
-    cost[s] = __popc(s) == 1 ? 0.0f : kTlInf;
+  for (int i = 0; i < 5; ++i)
+    if ((lane >> i) & 1u) low = box_union(low, leaf_box(T, i));
+  const Box b5 = leaf_box(T, 5), b6 = leaf_box(T, 6);
+#pragma unroll
+  for (uint32_t hi = 0; hi < 4; ++hi) {
+    const uint32_t s = lane + 32u * hi;
+    Box b = low;
+    if (hi & 1u) b = box_union(b, b5);
+    if (hi & 2u) b = box_union(b, b6);
+    if (s >= 1 && s <= full) {
+      const float a = box_area(b);
+      const int members = __popc(s);
+      area[s] = a;
+      // one member: 0; two: the only split costs 0 + 0
+      cost[s] = members == 1 ? 0.0f : members == 2 ? __fadd_rn(0.0f, a) : kTlInf;
+      if (members == 2) T.part[s] = (uint8_t)(s & (s - 1u));
+    }
   }
   __syncwarp();
-  for (int k = 2; k <= n; ++k) {
-    const uint32_t L = k <= 5 ? 1u : (k == 6 ? 4u : 32u);
-    const uint32_t base = c_sub_off[k], count = c_sub_off[k + 1] - base;
-    const uint32_t nparts = (1u << (k - 1)) - 1u;
-    const uint32_t chunk = (nparts + L - 1) / L;
-    for (uint32_t r0 = 0; r0 < count * L; r0 += 32) {
-      const uint32_t slot = r0 + (uint32_t)lane, e = slot / L, j = slot % L;
-      const uint32_t s = e < count ? c_subsets[base + e] : 0u;
-      const bool valid = e < count && s <= full;
-      float best = kTlInf;
-      uint32_t best_ord = 0xffffffffu, best_p = 0;
-      if (valid) {
-        const uint32_t delta = s & (s - 1u);
-        const uint32_t o0 = j * chunk, o1 = min(o0 + chunk, nparts);
-        uint32_t p = o0 < o1 ? deposit_bits(o0 + 1u, delta) : 0u;
-        for (uint32_t ord = o0; ord < o1; ++ord) {
-          const float c = __fadd_rn(cost[p], cost[s ^ p]);
-          if (c < best) { best = c; best_ord = ord; best_p = p; }
-          p = (p - delta) & delta;  // next subset of delta
-        }
-      }
-      for (uint32_t o = 1; o < L; o <<= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const uint32_t oo = __shfl_xor_sync(0xffffffffu, best_ord, o);
-        const uint32_t op = __shfl_xor_sync(0xffffffffu, best_p, o);
-        if (ob < best || (ob == best && oo < best_ord)) { best = ob; best_ord = oo; best_p = op; }
-      }
-      if (valid && j == 0) {
-        // the reference starts from INF with strict <, so an all-INF subset keeps INF / -1
-        cost[s] = __fadd_rn(best, area[s]);
-        T.part[s] = (uint8_t)(best_ord == 0xffffffffu ? 0xffu : best_p);
+  warp_dp_size<3>(T, cost, area, full);
+  if (n >= 4) warp_dp_size<4>(T, cost, area, full);
+  if (n >= 5) warp_dp_size<5>(T, cost, area, full);
+  if (n >= 6) {  // 7 subsets of 31 splits, four lanes each
+    const uint32_t e = lane >> 2, j = lane & 3u;
+    uint32_t s = e < 7 ? c_subsets[c_sub_off[6] + e] : 0u, bp = 0;
+    if (s > full) s = 0;
+    float best = s ? scan_splits<8>(cost, s, 8u * j, 31u, bp) : kTlInf;
+    uint32_t ord = best < kTlInf ? j : 4u;
+#pragma unroll
+    for (uint32_t o = 1; o < 4; o <<= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const uint32_t oo = __shfl_xor_sync(0xffffffffu, ord, o), op = __shfl_xor_sync(0xffffffffu, bp, o);
+      if (ob < best || (ob == best && oo < ord)) {
+        best = ob;
+        ord = oo;
+        bp = op;
       }
     }
+    if (s && j == 0) {
+      cost[s] = __fadd_rn(best, area[s]);
+      T.part[s] = (uint8_t)bp;
+    }
+    __syncwarp();
+  }
+  if (n == 7) {  // the full set's 63 splits, two per lane; only its split is asked for
+    uint32_t bp = 0;
+    const float best = scan_splits<2>(cost, 127u, 2u * lane, 63u, bp);
+    const uint32_t key = ordered_bits(best), least = __reduce_min_sync(0xffffffffu, key);
+    const uint32_t first = __ffs(__ballot_sync(0xffffffffu, key == least)) - 1;
+    bp = __shfl_sync(0xffffffffu, bp, first);
+    if (lane == 0) T.part[127] = (uint8_t)bp;
     __syncwarp();
   }
 }
 
 // 4. Reuse the treelet's internal ids (DFS from the root, right child popped first,
 //    :167-191) and rebuild it breadth-first from the partitions (:194-246).  One lane.
-__device__ void treelet_rebuild(Node* nodes, int32_t root, LaneTreelet& T) {
+__device__ void treelet_rebuild(Node* nodes, int32_t* parents, int32_t root, LaneTreelet& T) {
   const int n = T.n;
   if (n < 2) return;
   const uint32_t full = (1u << n) - 1u;
@@ -239,8 +321,8 @@ __device__ void treelet_rebuild(Node* nodes, int32_t root, LaneTreelet& T) {
     __stcg(p, b.lo);
     __stcg(p + 1, b.hi);
     __stcg(reinterpret_cast<int2*>(&nodes[cur].left), make_int2(li, ri));
-    __stcg(&nodes[li].aux0, cur);
-    __stcg(&nodes[ri].aux0, cur);
+    __stcg(parents + li, cur);
+    __stcg(parents + ri, cur);
   }
 }
 
@@ -248,10 +330,17 @@ __device__ void treelet_rebuild(Node* nodes, int32_t root, LaneTreelet& T) {
 // Level-synchronous pass.  Any children-before-parent order gives the same tree, and nodes of
 // equal height have disjoint subtrees (neither is an ancestor of the other), so each height
 // is one parallel step: every lane owns one treelet and does its refit, growth, DP and rebuild
-// alone, so the 32 lanes of a warp run the same 7-leaf work in step.  Heights come from a
-// climb that carries them in the rendezvous words; node ids are then grouped by height.
+// alone, so the 32 lanes of a warp run the same 7-leaf work in step.  Heights come from the emission
+// and, for a further pass, from the rebuilds of the one before; node ids are then grouped by height.
 // Trees higher than kTlMaxHeight (not reachable by a Karras tree: its depth is at most the
-// key bits plus 32) fall back to the climb-ordered kernel above.
+// key bits plus 32; many passes might) fall back to the climb-ordered kernel below for the rest.
+//
+// A pass is bound by its scattered 32-byte sectors, so what a node carries is laid out for it: the children's
+// areas lie beside their ids (a treelet grows through one sector per expansion instead of two nodes of two
+// sectors), tame boxes are not refitted or rewritten at the root, and there are no parent links.  10M
+// triangles, one pass, before -> with that: growth 1.60 -> 0.63 ms, heights by a climb over parent links
+// 0.31 ms -> none, DP and rebuild of heights 2, 3 and 4 on 0.35, 0.55 and 1.99 -> 0.21, 0.39 and 1.50 ms;
+// three passes 19.0 -> 12.1 ms, one pass at 200k 880 -> 542 us.
 // ---------------------------------------------------------------------------------------
 constexpr int kTlMaxHeight = 254;
 constexpr int kLvThreads = 32;  // one warp per block; its DP table is 16 KB of shared memory
@@ -259,23 +348,10 @@ constexpr int kLvThreads = 32;  // one warp per block; its DP table is 16 KB of 
 // A lane's treelet in registers (all indexing below is unrolled to constant indices).
 struct RegTreelet {
   Box b[kTlMax];
-  int32_t id[kTlMax], cl[kTlMax], cr[kTlMax];
-  float area[kTlMax];
-  int32_t en[kTlMax - 1], el[kTlMax - 1], er[kTlMax - 1];  // expansions: node and its children
+  int32_t id[kTlMax];
   int n;
 };
 
-__device__ __forceinline__ void reg_set(RegTreelet& T, int i, int32_t id, const Box& b, int2 ch) {
-#pragma unroll
-  for (int k = 0; k < kTlMax; ++k)
-    if (k == i) {
-      T.id[k] = id;
-      T.b[k] = b;
-      T.cl[k] = ch.x;
-      T.cr[k] = ch.y;
-      T.area[k] = box_area(b);
-    }
-}
 __device__ __forceinline__ int32_t reg_id(const RegTreelet& T, int i) {
   int32_t v = 0;
 #pragma unroll
@@ -291,93 +367,121 @@ __device__ __forceinline__ Box reg_union(const RegTreelet& T, uint32_t mask) {
   return b;
 }
 
-// Growth state without the leaf boxes (only their areas are compared).
+// Growth state: the leaves (ids and areas), the links of those that are inner nodes, and the expanded
+// nodes in order.  Expansion s replaces leaf `slot s` by the left child and appends the right child
+// as leaf s + 1; the slots, 3 bits each, say what the treelet looks like.
 struct GrowTreelet {
-  int32_t id[kTlMax], cl[kTlMax], cr[kTlMax];
+  int32_t id[kTlMax];
   float area[kTlMax];
-  int32_t en[kTlMax - 1], el[kTlMax - 1], er[kTlMax - 1];
+  Links k[kTlMax];
+  int32_t en[kTlMax - 1];
+  uint32_t slots;
   int n;
 };
-__device__ __forceinline__ void reg_set(GrowTreelet& T, int i, int32_t id, const Box& b, int2 ch) {
-#pragma unroll
-  for (int k = 0; k < kTlMax; ++k)
-    if (k == i) {
-      T.id[k] = id;
-      T.cl[k] = ch.x;
-      T.cr[k] = ch.y;
-      T.area[k] = box_area(b);
-    }
-}
 
-// Growth (lbvh_plus_builder.cu:73-114) with each leaf's children and area cached on entry.
-template <typename TL>
-__device__ __forceinline__ void reg_grow(const Node* nodes, int32_t root, const Box& rootbox, int2 rootch, TL& T) {
-  reg_set(T, 0, root, rootbox, rootch);
-  int cnt = 1;
+// Growth (lbvh_plus_builder.cu:73-114) from the root's links: the leaf with the largest area among the
+// inner ones is expanded, the first such on ties.
+__device__ __forceinline__ void reg_grow(const Node* nodes, int32_t first_leaf, int32_t root, const Links& rl,
+                                         GrowTreelet& T) {
 #pragma unroll
-  for (int step = 0; step < kTlMax - 1; ++step) {
-    int best = -1;
-    float max_area = -1.0f;
-    int32_t bl = 0, br = 0, bn = 0;
-#pragma unroll
-    for (int i = 0; i < kTlMax; ++i) {
-      if (i < cnt && !((uint32_t)T.cl[i] & kLeafBit) && T.area[i] > max_area) {
-        max_area = T.area[i];
-        best = i;
-        bl = T.cl[i];
-        br = T.cr[i];
-        bn = T.id[i];
-      }
-    }
-    if (best < 0) break;
-    T.en[step] = bn;
-    T.el[step] = bl;
-    T.er[step] = br;
-    const Box lb = ldcg_box(nodes, bl), rb = ldcg_box(nodes, br);
-    const int2 lc = ldcg_children(nodes, bl), rc = ldcg_children(nodes, br);
-    reg_set(T, best, bl, lb, lc);
-    reg_set(T, cnt, br, rb, rc);
-    ++cnt;
+  for (int i = 0; i < kTlMax; ++i) {
+    T.id[i] = first_leaf;
+    T.area[i] = 0.f;
+    T.k[i] = Links{0, 0, 0.f, 0.f};
   }
-  T.n = cnt;
-}
-
-// reg_grow after its first step, the root's expansion, whose loads the caller has made: leaves
-// (left, right) with their boxes and children, then the same steps from there.
-__device__ __forceinline__ void reg_grow_expanded(const Node* nodes, int32_t root, int2 rootch, const Box& lb,
-                                                  const Box& rb, int2 lc, int2 rc, GrowTreelet& T) {
-  reg_set(T, 0, rootch.x, lb, lc);
-  reg_set(T, 1, rootch.y, rb, rc);
+  T.id[0] = rl.l;
+  T.id[1] = rl.r;
+  T.area[0] = rl.al;
+  T.area[1] = rl.ar;
+  if (rl.l < first_leaf) T.k[0] = ldcg_links(nodes, rl.l);
+  if (rl.r < first_leaf) T.k[1] = ldcg_links(nodes, rl.r);
   T.en[0] = root;
-  T.el[0] = rootch.x;
-  T.er[0] = rootch.y;
-  int cnt = 2;
+  T.slots = 0;
+  T.n = 2;
 #pragma unroll
   for (int step = 1; step < kTlMax - 1; ++step) {
     int best = -1;
     float max_area = -1.0f;
-    int32_t bl = 0, br = 0, bn = 0;
+    Links x{0, 0, 0.f, 0.f};
+    int32_t xid = 0;
 #pragma unroll
-    for (int i = 0; i < kTlMax; ++i) {
-      if (i < cnt && !((uint32_t)T.cl[i] & kLeafBit) && T.area[i] > max_area) {
+    for (int i = 0; i <= step; ++i)
+      if (T.id[i] < first_leaf && T.area[i] > max_area) {
         max_area = T.area[i];
         best = i;
-        bl = T.cl[i];
-        br = T.cr[i];
-        bn = T.id[i];
+        x = T.k[i];
+        xid = T.id[i];
       }
-    }
     if (best < 0) break;
-    T.en[step] = bn;
-    T.el[step] = bl;
-    T.er[step] = br;
-    const Box lb2 = ldcg_box(nodes, bl), rb2 = ldcg_box(nodes, br);
-    const int2 lc2 = ldcg_children(nodes, bl), rc2 = ldcg_children(nodes, br);
-    reg_set(T, best, bl, lb2, lc2);
-    reg_set(T, cnt, br, rb2, rc2);
-    ++cnt;
+    T.en[step] = xid;
+    T.slots |= (uint32_t)best << (3 * step);
+    Links kl{0, 0, 0.f, 0.f};
+    if (x.l < first_leaf) kl = ldcg_links(nodes, x.l);
+    if (x.r < first_leaf) T.k[step + 1] = ldcg_links(nodes, x.r);
+    T.id[step + 1] = x.r;
+    T.area[step + 1] = x.ar;
+#pragma unroll
+    for (int i = 0; i <= step; ++i)
+      if (i == best) {
+        T.id[i] = x.l;
+        T.area[i] = x.al;
+        T.k[i] = kl;
+      }
+    T.n = step + 2;
   }
-  T.n = cnt;
+}
+
+// The order in which a rebuild reuses the treelet's inner ids (:167-191): depth first from the root, the
+// right child first.  Four bits each, the expansions' numbers.
+__device__ __forceinline__ uint32_t reuse_order(uint32_t slots, int m) {
+  uint32_t order = 0, stack = 0;  // stack: four bits per entry, the top lowest; 0 (the root) is never pushed
+  int s = 0;
+#pragma unroll
+  for (int k = 0; k < kTlMax - 1; ++k) {
+    if (k >= m) break;
+    order |= (uint32_t)s << (4 * k);
+    const uint32_t left = (slots >> (3 * s)) & 7u, right = (uint32_t)s + 1u;
+    int l = 0, r = 0;  // the first later expansion of either child
+#pragma unroll
+    for (int e = kTlMax - 2; e >= 1; --e) {
+      const uint32_t x = (slots >> (3 * e)) & 7u;
+      if (e > s && e < m && x == left) l = e;
+      if (e > s && e < m && x == right) r = e;
+    }
+    if (l) stack = stack << 4 | (uint32_t)l;
+    if (r) stack = stack << 4 | (uint32_t)r;
+    s = (int)(stack & 15u);
+    stack >>= 4;
+  }
+  return order;
+}
+
+// The root's links for its treelet, and whether it grows at all (not where its area is NaN).  Tame boxes
+// are final as they are; others are refitted (box and areas) from the children, as the reference does.
+__device__ __forceinline__ Links refit_root(Node* nodes, int32_t x, bool wild, bool& expand) {
+  Links k = ldcg_links(nodes, x);
+  expand = true;
+  if (wild) {
+    const Box lb = ldcg_box(nodes, k.l), rb = ldcg_box(nodes, k.r);
+    const Box box = box_union(lb, rb);
+    float4* p = reinterpret_cast<float4*>(nodes + x);
+    __stcg(p, box.lo);
+    __stcg(p + 1, box.hi);
+    k.al = box_area(lb);
+    k.ar = box_area(rb);
+    stcg_links(nodes, x, k);
+    expand = box_area(box) > -1.0f;
+  }
+  return k;
+}
+
+// A root whose treelet is not rebuilt by the DP (n = 1 or 2 leaves): two leaves change places, since the
+// DP's only split puts the second left.  Its height follows its children's.
+__device__ __forceinline__ void finish_short(Node* nodes, uint8_t* hgt, int32_t first_leaf, int32_t x, const Links& k,
+                                             bool two) {
+  if (two) stcg_links(nodes, x, Links{k.r, k.l, k.ar, k.al});
+  if (hgt)
+    __stcg(hgt + x, (uint8_t)min(1u + max(node_height(hgt, first_leaf, k.l), node_height(hgt, first_leaf, k.r)), 255u));
 }
 
 // Areas of the subsets s < 2^nv with two or more leaves into this lane's column A (stride 32):
@@ -436,113 +540,99 @@ __device__ __forceinline__ uint32_t best_split(const float* C, uint32_t mask) {
   return bp;
 }
 
-// Id reuse (:167-191): the treelet's internal nodes in DFS order from the root, right child
-// popped first, from the cached expansions.  Returns how many were found.
-template <typename TL>
-__device__ __forceinline__ int reg_avail(const Node* nodes, int32_t root, const TL& T, int* avail) {
-  const int n = T.n;
-  int n_avail = 0;
-  int stack[kTlMax + 8];
-  int top = 0;
-  stack[top++] = root;
-  while (top > 0) {
-    const int cur = stack[--top];
-    bool in_leaves = false;
+// The subsets of a rebuilt treelet, breadth-first (:194-246): byte j of masks is the j-th subset, of lefts
+// its left part; nibble j of lpos / rpos the place of that part in the queue (0: a single leaf).
+struct Splits {
+  unsigned long long masks, lefts;
+  uint32_t lpos, rpos;
+};
+// split(mask): the best split of a subset.  False where one has no finite split (NaN areas).
+template <typename Split>
+__device__ __forceinline__ bool reg_splits(int n, Split split, Splits& Q) {
+  Q.masks = (1u << n) - 1u;
+  Q.lefts = 0;
+  Q.lpos = Q.rpos = 0;
+  uint32_t qt = 1;
 #pragma unroll
-    for (int i = 0; i < kTlMax; ++i)
-      if (i < n && T.id[i] == cur) in_leaves = true;
-    if (!in_leaves && n_avail < kTlMax && top + 2 <= kTlMax + 8) {
-      avail[n_avail++] = cur;
-      int2 ch = make_int2(0, 0);
-      bool known = false;
-#pragma unroll
-      for (int e = 0; e < kTlMax - 1; ++e)
-        if (!known && e < n - 1 && T.en[e] == cur) {
-          ch = make_int2(T.el[e], T.er[e]);
-          known = true;
-        }
-      if (!known) ch = ldcg_children(nodes, cur);
-      stack[top++] = ch.x;
-      stack[top++] = ch.y;
+  for (int j = 0; j < kTlMax - 1; ++j) {
+    if (j >= n - 1) break;
+    const uint32_t mask = (uint32_t)(Q.masks >> (8 * j)) & 255u;
+    const uint32_t lm = split(mask), rm = mask ^ lm;
+    if (lm == 0 || rm == 0 || (lm & ~mask)) return false;
+    Q.lefts |= (unsigned long long)lm << (8 * j);
+    if (__popc(lm) > 1) {
+      Q.masks |= (unsigned long long)lm << (8 * qt);
+      Q.lpos |= qt++ << (4 * j);
+    }
+    if (__popc(rm) > 1) {
+      Q.masks |= (unsigned long long)rm << (8 * qt);
+      Q.rpos |= qt++ << (4 * j);
     }
   }
-  return n_avail;
+  return true;
 }
 
-// Rebuild (:194-246) breadth-first, handing out the reused ids in order: the j-th subset of the queue
-// gets the j-th id.  split(mask): the best split of a subset.  A subset with no finite split (NaN
-// areas) leaves the treelet unchanged.  The queues are bytes of 64-bit words, so nothing is indexed
-// through local memory.
-template <typename Split>
-__device__ __forceinline__ void reg_build(Node* nodes, const RegTreelet& T, Split split, const int* avail, int n_avail) {
-  const int n = T.n;
-  if (n_avail != n - 1) return;
-  unsigned long long masks = (1u << n) - 1u, lefts = 0;
-  int qt = 1;
+// Rebuild by one lane: the j-th subset of the queue gets the j-th reused id.  Children come later in the
+// queue than their parents, so the nodes are written from the last: a node's areas and height then have
+// its children's at hand.  root_box: the root's box is written too (a tame one is what it was).
+__device__ __forceinline__ void reg_build(Node* nodes, uint8_t* hgt, int32_t first_leaf, const RegTreelet& T,
+                                          const Splits& Q, const int* avail, bool root_box) {
+  float area[kTlMax], narea[kTlMax - 1];
+  uint32_t h[kTlMax], nh[kTlMax - 1];
 #pragma unroll
-  for (int j = 0; j < kTlMax - 1; ++j) {
-    if (j >= n - 1) break;
-    const uint32_t mask = (uint32_t)(masks >> (8 * j)) & 255u;
-    const uint32_t lm = split(mask), rm = mask ^ lm;
-    if (lm == 0 || rm == 0 || (lm & ~mask)) return;
-    lefts |= (unsigned long long)lm << (8 * j);
-    if (__popc(lm) > 1) masks |= (unsigned long long)lm << (8 * qt++);
-    if (__popc(rm) > 1) masks |= (unsigned long long)rm << (8 * qt++);
+  for (int i = 0; i < kTlMax; ++i) {
+    area[i] = box_area(T.b[i]);
+    h[i] = hgt && i < T.n ? node_height(hgt, first_leaf, T.id[i]) : 0u;
   }
-  int used = 1;
 #pragma unroll
-  for (int j = 0; j < kTlMax - 1; ++j) {
-    if (j >= n - 1) break;
-    const uint32_t mask = (uint32_t)(masks >> (8 * j)) & 255u, lm = (uint32_t)(lefts >> (8 * j)) & 255u;
-    const int cur = avail[j];
+  for (int j = kTlMax - 2; j >= 0; --j) {
+    narea[j] = 0.f;
+    nh[j] = 0;
+    if (j >= T.n - 1) continue;
+    const uint32_t mask = (uint32_t)(Q.masks >> (8 * j)) & 255u, lm = (uint32_t)(Q.lefts >> (8 * j)) & 255u;
     int child[2];
+    float ca[2];
+    uint32_t hm = 0;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       const uint32_t cm = s ? mask ^ lm : lm;
-      child[s] = reg_id(T, __ffs(cm) - 1);
-      if (__popc(cm) > 1) {
+      const int pos = (int)(((s ? Q.rpos : Q.lpos) >> (4 * j)) & 15u), leaf = __ffs(cm) - 1;
+      uint32_t ch = 0;
+      child[s] = 0;
+      ca[s] = 0.f;
 #pragma unroll
-        for (int k = 1; k < kTlMax - 1; ++k)
-          if (k == used) child[s] = avail[k];
-        used++;
-      }
+      for (int k = 0; k < kTlMax; ++k)
+        if (k == leaf) {
+          child[s] = T.id[k];
+          ca[s] = area[k];
+          ch = h[k];
+        }
+#pragma unroll
+      for (int k = 1; k < kTlMax - 1; ++k)
+        if (k > j && k == pos) {
+          child[s] = avail[k];
+          ca[s] = narea[k];
+          ch = nh[k];
+        }
+      hm = max(hm, ch);
     }
     const Box b = reg_union(T, mask);
-    float4* p = reinterpret_cast<float4*>(nodes + cur);
-    __stcg(p, b.lo);
-    __stcg(p + 1, b.hi);
-    __stcg(reinterpret_cast<int2*>(&nodes[cur].left), make_int2(child[0], child[1]));
-    __stcg(&nodes[child[0]].aux0, cur);
-    __stcg(&nodes[child[1]].aux0, cur);
-  }
-}
-
-// Heights: a climb from every leaf; the first child to reach a parent leaves its height in the
-// rendezvous word, the second computes the parent's.
-__global__ void __launch_bounds__(256) k_tl_heights(const Node* __restrict__ nodes, unsigned long long* __restrict__ slots,
-                                                    const uint32_t* epoch_word, uint32_t round, uint32_t n,
-                                                    uint8_t* __restrict__ hgt, uint32_t* __restrict__ flags) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned long long tag = (unsigned long long)(__ldcg(epoch_word) + 1u + round) << 32;
-  int32_t idx = (int32_t)(n - 1 + i);
-  uint32_t h = 0;
-  while (idx != 0) {
-    const int32_t parent = __ldcg(&nodes[idx].aux0);
-    const unsigned long long old = atomicExch(slots + parent, tag | h);
-    if ((old & 0xffffffff00000000ull) != tag) return;  // first child to arrive
-    h = 1u + max(h, (uint32_t)old);
-    if (h > (uint32_t)kTlMaxHeight) {
-      atomicOr(flags, 1u);
-      h = kTlMaxHeight + 1;
+    narea[j] = box_area(b);
+    nh[j] = hm + 1u;
+    if (j > 0 || root_box) {
+      float4* p = reinterpret_cast<float4*>(nodes + avail[j]);
+      __stcg(p, b.lo);
+      __stcg(p + 1, b.hi);
     }
-    hgt[parent] = (uint8_t)h;
-    idx = parent;
+    stcg_links(nodes, avail[j], Links{child[0], child[1], ca[0], ca[1]});
+    if (hgt) __stcg(hgt + avail[j], (uint8_t)min(nh[j], 255u));
   }
 }
 
 // Nodes per height (block histograms in shared memory, one global add per nonzero bin).
-__global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hgt, uint32_t m, uint32_t* __restrict__ cnt) {
+// A height past kTlMaxHeight hands this pass and the following ones to the fallback (flags[0]).
+__global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hgt, uint32_t m, uint32_t* __restrict__ cnt,
+                                                  uint32_t* __restrict__ flags) {
   __shared__ uint32_t s_cnt[256];
   s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -551,6 +641,7 @@ __global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hg
   __syncthreads();
   const uint32_t c = s_cnt[threadIdx.x];
   if (c) atomicAdd(cnt + threadIdx.x, c);
+  if (c && threadIdx.x > kTlMaxHeight) atomicOr(flags, 1u);
 }
 
 // off[h] = first list position of height h (exclusive scan of cnt over 256 heights), cursor
@@ -584,7 +675,7 @@ __global__ void __launch_bounds__(256) k_tl_offsets(const uint32_t* __restrict__
   __syncthreads();
   if (t == 0) {
     flags[1] = s_maxh;
-    flags[2] = 1;  // the first height processed
+    flags[2] = 4;  // the first height of the loop (heights 1 to 3 have launches of their own)
   }
 }
 
@@ -607,57 +698,63 @@ __global__ void __launch_bounds__(256) k_tl_scatter(const uint8_t* __restrict__ 
   }
 }
 
-// Per height, two kernels: k_tl_grow (latency-bound: many warps, few registers) refits each
-// node, grows its treelet and writes a descriptor; k_tl_dp (compute-bound) reloads the leaf
-// boxes, runs the DP and rebuilds.  Descriptors are structure-of-arrays, kTlDescWords words per
+// Per height, two kernels: k_tl_grow (latency-bound: many warps, few registers) grows each node's
+// treelet and writes a descriptor; k_tl_dp (compute-bound) loads the leaf boxes, runs the DP and
+// rebuilds.  Descriptors are structure-of-arrays, kTlDescWords words per
 // node at stride `stride` (>= the largest height's node count): [0] n | n_avail << 8,
 // [1..7] leaf ids, [8..13] reused internal ids in order.  ctl: [0] too high, [1] largest
-// height, [2] current height.
+// height, [2] current height.  at: the height, 0 for the current one.
 constexpr int kGrowThreads = 128;
 
-__global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(Node* __restrict__ nodes, const uint32_t* __restrict__ list,
-                                                          const uint32_t* __restrict__ off,
-                                                          const uint32_t* __restrict__ ctl, uint32_t* __restrict__ desc,
-                                                          uint32_t stride) {
+struct TlArgs {
+  Node* nodes;
+  uint8_t* hgt;  // heights, kept up to date where another pass follows (else NULL)
+  int32_t first_leaf;
+  const uint32_t* wild;
+  const uint32_t* off;
+  uint32_t* desc;
+  uint32_t stride;
+};
+
+__global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(TlArgs A, const uint32_t* __restrict__ list,
+                                                             const uint32_t* __restrict__ ctl, uint32_t at) {
   if (__ldcg(ctl) != 0u) return;  // too high: the fallback pass does the work
-  const uint32_t h = __ldcg(ctl + 2);
-  const uint32_t b = __ldcg(off + h), e = __ldcg(off + h + 1);
+  const uint32_t h = at ? at : __ldcg(ctl + 2);
+  const uint32_t b = __ldcg(A.off + h), e = __ldcg(A.off + h + 1);
+  const bool wild = __ldcg(A.wild) != 0u;
   for (uint32_t k = b + blockIdx.x * blockDim.x + threadIdx.x; k < e; k += gridDim.x * blockDim.x) {
     const int32_t x = (int32_t)__ldcg(list + k);
-    const int2 ch = ldcg_children(nodes, x);
-    // the children's boxes (the refit) and their own children (the root's expansion) together
-    const Box lb = ldcg_box(nodes, ch.x), rb = ldcg_box(nodes, ch.y);
-    const int2 lc = h == 1 ? make_int2(0, 0) : ldcg_children(nodes, ch.x);
-    const int2 rc = h == 1 ? make_int2(0, 0) : ldcg_children(nodes, ch.y);
-    const Box box = box_union(lb, rb);
-    float4* p = reinterpret_cast<float4*>(nodes + x);
-    __stcg(p, box.lo);
-    __stcg(p + 1, box.hi);
+    bool expand;
+    const Links rl = refit_root(A.nodes, x, wild, expand);
     const uint32_t q = k - b;
-    // growth expands the root first, unless its area is not above -1 (NaN): then n = 1
-    const bool expand = box_area(box) > -1.0f;
-    if (h == 1) {  // both children are BVH leaves: the two-leaf treelet below, without growing it
-      if (expand) __stcg(reinterpret_cast<int2*>(&nodes[x].left), make_int2(ch.y, ch.x));
-      desc[q] = 0u;
-      continue;
+    if (h == 1) {  // both children are BVH leaves
+      if (expand) stcg_links(A.nodes, x, Links{rl.r, rl.l, rl.ar, rl.al});
+      continue;  // (no DP is launched for height 1)
     }
     GrowTreelet T;
-    if (expand) reg_grow_expanded(nodes, x, ch, lb, rb, lc, rc, T);
-    else reg_grow(nodes, x, box, ch, T);
-    if (T.n == 2) {
-      // Two leaves (the root's children; both are BVH leaves): the DP's only split puts the
-      // second leaf left, so the rebuild swaps the children (box and parent links stay).
-      __stcg(reinterpret_cast<int2*>(&nodes[x].left), make_int2(T.id[1], T.id[0]));
-      desc[q] = 0u;  // nothing left for k_tl_dp
+    T.n = 1;
+    if (expand) reg_grow(A.nodes, A.first_leaf, x, rl, T);
+    if (T.n <= 2) {
+      finish_short(A.nodes, A.hgt, A.first_leaf, x, rl, T.n == 2);
+      A.desc[q] = 0u;  // nothing left for k_tl_dp
       continue;
     }
-    int avail[kTlMax];
-    const int na = T.n >= 2 ? reg_avail(nodes, x, T, avail) : 0;
-    desc[q] = (uint32_t)T.n | ((uint32_t)na << 8);
+    const int m = T.n - 1;
+    const uint32_t order = reuse_order(T.slots, m);
+    A.desc[q] = (uint32_t)T.n | ((uint32_t)m << 8);
 #pragma unroll
-    for (int i = 0; i < kTlMax; ++i) desc[(size_t)(1 + i) * stride + q] = (uint32_t)T.id[i];
+    for (int i = 0; i < kTlMax; ++i)
+      if (i < T.n) A.desc[(size_t)(1 + i) * A.stride + q] = (uint32_t)T.id[i];
 #pragma unroll
-    for (int i = 0; i < kTlMax - 1; ++i) desc[(size_t)(8 + i) * stride + q] = i < na ? (uint32_t)avail[i] : 0u;
+    for (int i = 0; i < kTlMax - 1; ++i) {
+      if (i >= m) break;
+      const int s = (int)((order >> (4 * i)) & 15u);
+      int32_t id = 0;
+#pragma unroll
+      for (int c = 0; c < kTlMax - 1; ++c)
+        if (c == s) id = T.en[c];
+      A.desc[(size_t)(8 + i) * A.stride + q] = (uint32_t)id;
+    }
   }
 }
 
@@ -666,16 +763,14 @@ __global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(Node* __restrict__ 
 // (stride 32), then the rebuild.  The warp runs the DP variant of its largest treelet, at most
 // NVMAX leaves.  Called by all 32 lanes together.
 template <int NVMAX>
-__device__ __forceinline__ void lane_dp(Node* nodes, const uint32_t* desc, uint32_t stride, uint32_t q, bool act,
-                                        float* C) {
-  const uint32_t w0 = act ? __ldcg(desc + q) : 0u;
+__device__ __forceinline__ void lane_dp(const TlArgs& A, bool wild, uint32_t q, bool act, float* C) {
+  const uint32_t w0 = act ? __ldcg(A.desc + q) : 0u;
   RegTreelet T;
   T.n = (int)(w0 & 255u);
-  const int na = (int)(w0 >> 8);
 #pragma unroll
   for (int i = 0; i < kTlMax; ++i) {
-    T.id[i] = i < NVMAX && i < T.n ? (int32_t)__ldcg(desc + (size_t)(1 + i) * stride + q) : 0;
-    T.b[i] = i < NVMAX && i < T.n ? ldcg_box(nodes, T.id[i]) : box_empty();
+    T.id[i] = i < NVMAX && i < T.n ? (int32_t)__ldcg(A.desc + (size_t)(1 + i) * A.stride + q) : 0;
+    T.b[i] = i < NVMAX && i < T.n ? ldcg_box(A.nodes, T.id[i]) : box_empty();
   }
   const int nv = (int)__reduce_max_sync(0xffffffffu, (uint32_t)T.n);
   if (nv < 2) return;
@@ -685,66 +780,31 @@ __device__ __forceinline__ void lane_dp(Node* nodes, const uint32_t* desc, uint3
   if (T.n >= 2) {
     int avail[kTlMax];
 #pragma unroll
-    for (int i = 0; i < kTlMax - 1; ++i) avail[i] = (int)__ldcg(desc + (size_t)(8 + i) * stride + q);
+    for (int i = 0; i < kTlMax - 1; ++i)
+      avail[i] = i < NVMAX - 1 && i < T.n - 1 ? (int)__ldcg(A.desc + (size_t)(8 + i) * A.stride + q) : 0;
     const uint32_t full = (1u << of) - 1u;
-    reg_build(nodes, T, [&](uint32_t mask) { return mask == full ? top : best_split(C, mask); }, avail, na);
+    Splits Q;
+    if (reg_splits(T.n, [&](uint32_t mask) { return mask == full ? top : best_split(C, mask); }, Q))
+      reg_build(A.nodes, A.hgt, A.first_leaf, T, Q, avail, wild);
+    else
+      finish_short(A.nodes, A.hgt, A.first_leaf, avail[0], ldcg_links(A.nodes, avail[0]), false);
   }
 }
 
 // NVMAX < kTlMax: a DP for treelets of at most NVMAX leaves (heights where no more fit: height 2
 // holds at most 4), compiled for fewer registers, so more warps share an SM.
 template <int NVMAX>
-__global__ void __launch_bounds__(kLvThreads) k_tl_dp(Node* __restrict__ nodes, const uint32_t* __restrict__ off,
-                                                      const uint32_t* __restrict__ ctl,
-                                                      const uint32_t* __restrict__ desc, uint32_t stride) {
-  // per-lane columns of 2^NVMAX areas, then costs (the narrow path below uses 768 words)
-  __shared__ float s_cost[std::max((1 << NVMAX) * 32, 1024)];
+__global__ void __launch_bounds__(kLvThreads) k_tl_dp(TlArgs A, const uint32_t* __restrict__ ctl, uint32_t at) {
+  __shared__ float s_cost[(1 << NVMAX) * 32];  // per-lane columns of 2^NVMAX areas, then costs
   if (__ldcg(ctl) != 0u) return;
-  const uint32_t h = __ldcg(ctl + 2);
-  const uint32_t b = __ldcg(off + h), e = __ldcg(off + h + 1);
+  const uint32_t h = at ? at : __ldcg(ctl + 2);
+  const uint32_t b = __ldcg(A.off + h), e = __ldcg(A.off + h + 1);
+  const bool wild = __ldcg(A.wild) != 0u;
   const int lane = threadIdx.x & 31;
-  if (e - b <= 8u * gridDim.x) {
-    // a narrow height: one treelet per warp with the warp-cooperative DP (shorter critical path)
-    LaneTreelet& S = *reinterpret_cast<LaneTreelet*>(s_cost);
-    float* cost = s_cost + 512;
-    float* area = s_cost + 640;
-    for (uint32_t k = b + blockIdx.x; k < e; k += gridDim.x) {
-      const uint32_t q = k - b;
-      const uint32_t w0 = __ldcg(desc + q);
-      const int n = (int)(w0 & 255u);
-      if (n < 2) continue;  // uniform over the warp
-      if (lane < kTlMax) {
-        const int32_t id = (int32_t)__ldcg(desc + (size_t)(1 + lane) * stride + q);
-        S.act[lane] = id;
-        const Box bx = lane < n ? ldcg_box(nodes, id) : box_empty();
-        S.box[0][lane] = bx.lo.x; S.box[1][lane] = bx.lo.y; S.box[2][lane] = bx.lo.z;
-        S.box[3][lane] = bx.hi.x; S.box[4][lane] = bx.hi.y; S.box[5][lane] = bx.hi.z;
-      }
-      if (lane == 0) S.n = n;
-      __syncwarp();
-      treelet_dp(S, cost, area);
-      if (lane == 0) {
-        RegTreelet T;
-        T.n = n;
-#pragma unroll
-        for (int i = 0; i < kTlMax; ++i) {
-          T.id[i] = S.act[i];
-          T.b[i] = leaf_box(S, i);
-        }
-        int avail[kTlMax];
-#pragma unroll
-        for (int i = 0; i < kTlMax - 1; ++i) avail[i] = (int)__ldcg(desc + (size_t)(8 + i) * stride + q);
-        reg_build(nodes, T, [&](uint32_t mask) { return (uint32_t)S.part[mask]; }, avail, (int)(w0 >> 8));
-      }
-      __syncwarp();
-    }
-    return;
-  }
-  float* C = s_cost + lane;
   // warp-uniform loop: the warp runs the DP variant of its largest treelet
   for (uint32_t kb = b + blockIdx.x * kLvThreads; kb < e; kb += gridDim.x * kLvThreads) {
     const uint32_t k = kb + lane;
-    lane_dp<NVMAX>(nodes, desc, stride, k - b, k < e, C);
+    lane_dp<NVMAX>(A, wild, k - b, k < e, s_cost + lane);
   }
 }
 
@@ -754,15 +814,13 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dp(Node* __restrict__ nodes, 
 // R rounds of 32 nodes, packs those of its class into a shared list (ballots) and runs them 32
 // at a time; R shrinks with the height's node count so that every block gets a chunk.
 template <int NV>
-__global__ void __launch_bounds__(kLvThreads) k_tl_dpc(Node* __restrict__ nodes, const uint32_t* __restrict__ off,
-                                                       const uint32_t* __restrict__ ctl,
-                                                       const uint32_t* __restrict__ desc, uint32_t stride) {
+__global__ void __launch_bounds__(kLvThreads) k_tl_dpc(TlArgs A, const uint32_t* __restrict__ ctl, uint32_t at) {
   constexpr int R = 8;
   __shared__ float s_cost[(1 << NV) * 32];
   __shared__ uint32_t s_list[32 * R];
   if (__ldcg(ctl) != 0u) return;
-  const uint32_t h = __ldcg(ctl + 2);
-  const uint32_t b = __ldcg(off + h), e = __ldcg(off + h + 1);
+  const uint32_t b = __ldcg(A.off + at), e = __ldcg(A.off + at + 1);
+  const bool wild = __ldcg(A.wild) != 0u;
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
   float* C = s_cost + lane;
@@ -771,7 +829,7 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dpc(Node* __restrict__ nodes,
     uint32_t cnt = 0;
     for (uint32_t r = 0; r < rounds; ++r) {
       const uint32_t k = chunk + r * 32u + (uint32_t)lane;
-      const int n = k < e ? (int)(__ldcg(desc + (k - b)) & 255u) : 0;
+      const int n = k < e ? (int)(__ldcg(A.desc + (k - b)) & 255u) : 0;
       const bool match = n >= 2 && (n <= 4 ? 4 : n) == NV;
       const uint32_t bal = __ballot_sync(0xffffffffu, match);
       if (match) s_list[cnt + __popc(bal & lt)] = k - b;
@@ -780,18 +838,19 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dpc(Node* __restrict__ nodes,
     __syncwarp();
     for (uint32_t i = 0; i < cnt; i += 32) {
       const bool act = i + (uint32_t)lane < cnt;
-      lane_dp<NV>(nodes, desc, stride, act ? s_list[i + lane] : 0u, act, C);
+      lane_dp<NV>(A, wild, act ? s_list[i + lane] : 0u, act, C);
     }
     __syncwarp();  // the list is refilled by the next chunk
   }
 }
 
-// The narrow heights in one cooperative launch.  Once a height has few nodes, its two launches
-// (growth, DP) cost mostly their latency; k_tl_narrow runs the remaining heights, from the current
-// one (ctl[2]) to the largest (ctl[1]), with a grid barrier between heights (nodes of one height
-// have disjoint subtrees, a height needs all lower ones done).  Per node, one warp: lane 0 refits
-// the node and grows its treelet (as k_tl_grow), the warp runs the cooperative DP and lane 0
-// rebuilds (as k_tl_dp's narrow path).  Same work and result as the per-height kernels.
+// The narrow heights in one cooperative launch.  Once a height has few nodes, its launches (growth, DP) cost
+// mostly their latency; k_tl_narrow runs the remaining heights, from the current one (ctl[2]) to the
+// largest (ctl[1]), with a grid barrier between heights (nodes of one height have disjoint subtrees, a
+// height needs all lower ones done).  Per node, one warp: lane 0 grows the treelet, seven lanes load the
+// leaf boxes, the warp runs the cooperative DP, all lanes follow the splits and each writes one of the
+// rebuilt nodes.  Same work and result as the per-height kernels.  A height is a chain of some ten L2
+// round trips and a barrier: about 8 us (17 us with a DP whose cost loads waited for one another).
 constexpr int kNarrowThreads = 256;
 
 struct NarrowWarp {
@@ -799,62 +858,109 @@ struct NarrowWarp {
   float cost[1 << kTlMax];
   float area[1 << kTlMax];
   int32_t avail[kTlMax];
-  int32_t na;
+  uint8_t h[kTlMax + 1];
 };
 
-__global__ void __launch_bounds__(kNarrowThreads) k_tl_narrow(Node* __restrict__ nodes, const uint32_t* __restrict__ list,
-                                                              const uint32_t* __restrict__ off, uint32_t* __restrict__ ctl,
+__global__ void __launch_bounds__(kNarrowThreads) k_tl_narrow(TlArgs A, const uint32_t* __restrict__ list,
+                                                              uint32_t* __restrict__ ctl,
                                                               uint32_t* __restrict__ status) {
   __shared__ NarrowWarp s_warp[kNarrowThreads / 32];
   __shared__ uint32_t s_ok;
   // every block reads the same words (nothing writes them in this kernel)
   if (__ldcg(ctl) != 0u) return;  // too high: the fallback pass does the work
   const uint32_t h0 = __ldcg(ctl + 2), h1 = __ldcg(ctl + 1);
+  const bool wild = __ldcg(A.wild) != 0u;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   NarrowWarp& W = s_warp[w];
   const uint32_t gw = blockIdx.x * (kNarrowThreads / 32) + (uint32_t)w, nw = gridDim.x * (kNarrowThreads / 32);
   uint32_t nbar = 0;
+  bool alone = false;
   for (uint32_t h = h0; h <= h1; ++h) {
-    const uint32_t b = __ldcg(off + h), e = __ldcg(off + h + 1);
-    for (uint32_t k = b + gw; k < e; k += nw) {
+    const uint32_t b = __ldcg(A.off + h), e = __ldcg(A.off + h + 1);
+    // A height has no more nodes than the one below it: from the first that one block's warps hold on,
+    // block 0 goes on alone, with block barriers.
+    alone = alone || e - b <= kNarrowThreads / 32;
+    if (alone && blockIdx.x != 0) return;
+    for (uint32_t k = b + gw; k < e; k += alone ? kNarrowThreads / 32 : nw) {
       if (lane == 0) {
         const int32_t x = (int32_t)__ldcg(list + k);
-        const int2 ch = ldcg_children(nodes, x);
-        const Box box = box_union(ldcg_box(nodes, ch.x), ldcg_box(nodes, ch.y));
-        float4* p = reinterpret_cast<float4*>(nodes + x);
-        __stcg(p, box.lo);
-        __stcg(p + 1, box.hi);
+        bool expand;
+        const Links rl = refit_root(A.nodes, x, wild, expand);
         GrowTreelet T;
-        reg_grow(nodes, x, box, ch, T);
-        W.S.n = T.n;
+        T.n = 1;
+        if (expand) reg_grow(A.nodes, A.first_leaf, x, rl, T);
+        if (T.n <= 2) {
+          finish_short(A.nodes, A.hgt, A.first_leaf, x, rl, T.n == 2);
+        } else {
+          const uint32_t order = reuse_order(T.slots, T.n - 1);
 #pragma unroll
-        for (int i = 0; i < kTlMax; ++i) W.S.act[i] = T.id[i];
-        W.na = T.n >= 2 ? reg_avail(nodes, x, T, W.avail) : 0;
+          for (int i = 0; i < kTlMax; ++i) W.S.act[i] = T.id[i];
+#pragma unroll
+          for (int i = 0; i < kTlMax - 1; ++i) W.S.exp_node[i] = T.en[i];
+#pragma unroll
+          for (int i = 0; i < kTlMax - 1; ++i)
+            if (i < T.n - 1) W.avail[i] = W.S.exp_node[(order >> (4 * i)) & 15u];
+        }
+        W.S.n = T.n;
       }
       __syncwarp();
       const int n = W.S.n;
-      if (n >= 2) {  // uniform over the warp
+      if (n > 2) {  // uniform over the warp
         if (lane < kTlMax) {
-          const Box bx = lane < n ? ldcg_box(nodes, W.S.act[lane]) : box_empty();
+          const Box bx = lane < n ? ldcg_box(A.nodes, W.S.act[lane]) : box_empty();
           W.S.box[0][lane] = bx.lo.x; W.S.box[1][lane] = bx.lo.y; W.S.box[2][lane] = bx.lo.z;
           W.S.box[3][lane] = bx.hi.x; W.S.box[4][lane] = bx.hi.y; W.S.box[5][lane] = bx.hi.z;
+          W.h[lane] = A.hgt && lane < n ? (uint8_t)node_height(A.hgt, A.first_leaf, W.S.act[lane]) : 0;
         }
         __syncwarp();
         treelet_dp(W.S, W.cost, W.area);
-        if (lane == 0) {
-          RegTreelet T;
-          T.n = n;
-#pragma unroll
-          for (int i = 0; i < kTlMax; ++i) {
-            T.id[i] = W.S.act[i];
-            T.b[i] = leaf_box(W.S, i);
+        Splits Q;
+        if (!reg_splits(n, [&](uint32_t mask) { return (uint32_t)W.S.part[mask]; }, Q)) {
+          if (lane == 0) finish_short(A.nodes, A.hgt, A.first_leaf, W.avail[0], ldcg_links(A.nodes, W.avail[0]), false);
+        } else {
+          // every lane walks the queue for the heights (last first); lane j keeps node j
+          uint32_t mine = 0;
+          unsigned long long hq = 0;  // byte j: node j's height
+          for (int j = n - 2; j >= 0; --j) {
+            const uint32_t mask = (uint32_t)(Q.masks >> (8 * j)) & 255u, lm = (uint32_t)(Q.lefts >> (8 * j)) & 255u;
+            const uint32_t lp = (Q.lpos >> (4 * j)) & 15u, rp = (Q.rpos >> (4 * j)) & 15u;
+            const uint32_t hl = lp ? (uint32_t)(hq >> (8 * lp)) & 255u : W.h[__ffs(lm) - 1];
+            const uint32_t hr = rp ? (uint32_t)(hq >> (8 * rp)) & 255u : W.h[__ffs(mask ^ lm) - 1];
+            const uint32_t nh = min(1u + max(hl, hr), 255u);
+            hq |= (unsigned long long)nh << (8 * j);
+            if (j == lane) mine = nh;
           }
-          reg_build(nodes, T, [&](uint32_t mask) { return (uint32_t)W.S.part[mask]; }, W.avail, W.na);
+          if (lane < n - 1) {
+            const uint32_t mask = (uint32_t)(Q.masks >> (8 * lane)) & 255u, lm = (uint32_t)(Q.lefts >> (8 * lane)) & 255u;
+            const uint32_t rm = mask ^ lm, lp = (Q.lpos >> (4 * lane)) & 15u, rp = (Q.rpos >> (4 * lane)) & 15u;
+            const int32_t cur = W.avail[lane];
+            const int li = __ffs(lm) - 1, ri = __ffs(rm) - 1;
+            Links out;
+            out.l = lp ? W.avail[lp] : W.S.act[li];
+            out.r = rp ? W.avail[rp] : W.S.act[ri];
+            out.al = lp ? W.area[lm] : box_area(leaf_box(W.S, li));
+            out.ar = rp ? W.area[rm] : box_area(leaf_box(W.S, ri));
+            Box bx = box_empty();
+            for (int i = 0; i < n; ++i)
+              if ((mask >> i) & 1u) bx = box_union(bx, leaf_box(W.S, i));
+            if (lane > 0 || wild) {
+              float4* p = reinterpret_cast<float4*>(A.nodes + cur);
+              __stcg(p, bx.lo);
+              __stcg(p + 1, bx.hi);
+            }
+            stcg_links(A.nodes, cur, out);
+            if (A.hgt) __stcg(A.hgt + cur, (uint8_t)mine);
+          }
         }
       }
       __syncwarp();
     }
-    if (h < h1 && !grid_sync(ctl + 4, ++nbar * gridDim.x, status, &s_ok)) return;
+    if (alone) {
+      __threadfence_block();
+      __syncthreads();
+    } else if (h < h1 && !grid_sync(ctl + 4, ++nbar * gridDim.x, status, &s_ok)) {
+      return;
+    }
   }
 }
 
@@ -872,9 +978,22 @@ __global__ void k_tl_step(uint32_t* __restrict__ ctl, const uint32_t* __restrict
   if constexpr (GRAPH) cudaGraphSetConditional(handle, go ? 1u : 0u);
 }
 
+// Parent links for the fallback; returns at once unless flags[0] is set.
+__global__ void __launch_bounds__(256) k_tl_parents(const Node* __restrict__ nodes, uint32_t m,
+                                                    int32_t* __restrict__ parents, const uint32_t* __restrict__ flags) {
+  if (__ldcg(flags) == 0u) return;
+  for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) {
+    const int2 ch = ldcg_children(nodes, (int32_t)x);
+    parents[ch.x] = (int32_t)x;
+    parents[ch.y] = (int32_t)x;
+  }
+}
+
 // The climb-ordered pass as a fallback for trees higher than kTlMaxHeight: persistent warps
-// take groups of 32 leaves.  Launched every pass; returns at once unless flags[0] is set.
-__global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ nodes, unsigned long long* __restrict__ slots,
+// take groups of 32 leaves.  Launched every pass; returns at once unless flags[0] is set, which it
+// stays for the following passes (this kernel keeps neither heights nor areas).
+__global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ nodes, int32_t* __restrict__ parents,
+                                                         unsigned long long* __restrict__ slots,
                                                          const uint32_t* epoch_word, uint32_t round, uint32_t n,
                                                          const uint32_t* __restrict__ flags) {
   __shared__ LaneTreelet S[64];
@@ -893,7 +1012,7 @@ __global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ node
         if (idx == 0) {
           active = false;
         } else {
-          int32_t parent = __ldcg(&nodes[idx].aux0);
+          int32_t parent = __ldcg(parents + idx);
           __threadfence();
           unsigned long long old = atomicExch(slots + parent, tag | 1u);
           if ((old & 0xffffffff00000000ull) != tag) {
@@ -919,7 +1038,7 @@ __global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ node
         treelet_dp(S[w * 32 + src], s_cost[w], s_area[w]);
       }
       __syncwarp();
-      if (work) treelet_rebuild(nodes, idx, mine);
+      if (work) treelet_rebuild(nodes, parents, idx, mine);
       __threadfence();
     }
   }
@@ -931,9 +1050,8 @@ static int g_dpc_grid[64][4] = {};  // resident blocks of k_tl_dpc<4..7> per dev
 static int g_narrow_grid[64] = {};  // resident blocks of k_tl_narrow per device (-1: no cooperative launch)
 
 // The loop over heights as a graph: WHILE(cond) { grow; dp; step }.
-static cudaError_t make_height_graph(Node* nodes, const uint32_t* list, const uint32_t* off, uint32_t* ctl,
-                                     uint32_t* desc, uint32_t stride, uint32_t grow_grid, uint32_t dp_grid,
-                                     uint32_t narrow, cudaGraphExec_t* out) {
+static cudaError_t make_height_graph(const TlArgs& A, const uint32_t* list, uint32_t* ctl, uint32_t grow_grid,
+                                     uint32_t dp_grid, uint32_t narrow, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaGraphCreate(&g, 0);
   if (e != cudaSuccess) return e;
@@ -953,9 +1071,9 @@ static cudaError_t make_height_graph(Node* nodes, const uint32_t* list, const ui
     if ((e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
         cudaSuccess)
       break;
-    k_tl_grow<<<grow_grid, kGrowThreads, 0, cs>>>(nodes, list, off, ctl, desc, stride);
-    k_tl_dp<kTlMax><<<dp_grid, kLvThreads, 0, cs>>>(nodes, off, ctl, desc, stride);
-    k_tl_step<true><<<1, 32, 0, cs>>>(ctl, off, narrow, handle);
+    k_tl_grow<<<grow_grid, kGrowThreads, 0, cs>>>(A, list, ctl, 0u);
+    k_tl_dp<kTlMax><<<dp_grid, kLvThreads, 0, cs>>>(A, ctl, 0u);
+    k_tl_step<true><<<1, 32, 0, cs>>>(ctl, A.off, narrow, handle);
     cudaGraph_t captured = nullptr;
     const cudaError_t e2 = cudaGetLastError();
     e = cudaStreamEndCapture(cs, &captured);
@@ -1001,12 +1119,11 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
   // heights of at most `narrow` nodes (two per warp of the cooperative grid) run in k_tl_narrow
   const uint32_t narrow =
       !host_loop && g_narrow_grid[dev] > 0 ? 2u * (uint32_t)g_narrow_grid[dev] * (kNarrowThreads / 32) : 0u;
-  // scratch: heights in the delta bytes (emission is done with them), the id list in the idle
-  // value buffer, descriptors in the triangle boxes (32 B per triangle; a height has at most
-  // n/2 nodes), counters / offsets / control words in the sort histogram words
-  uint8_t* hgt = ws.delta;
+  // scratch: the id list in the idle value buffer, descriptors in the triangle boxes (32 B per triangle; a
+  // height has at most n/2 nodes), the fallback's parent links in the idle key buffer, counters / offsets /
+  // control words in the sort histogram words
   uint32_t* list = ws.vals[fb ^ 1];
-  uint32_t* desc = reinterpret_cast<uint32_t*>(ws.boxes);
+  int32_t* parents = static_cast<int32_t*>(ws.keys[fb ^ 1]);
   const uint32_t stride = std::max<uint32_t>(n / 2, 1);
   uint32_t* cnt = ws.scratch + L.hist;       // 256
   uint32_t* off = cnt + 256;                 // 257
@@ -1014,45 +1131,58 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
   uint32_t* ctl = cursor + 256;              // [0] too high, [1] largest height, [2] current height
   static_assert(kTlCtlWord == 256 + 264 + 256, "control words of the treelet pass");
   static_assert(kTlCtlWord + 8 <= (size_t)kMaxPasses * 256, "treelet words fit the histogram area");
+  TlArgs A;
+  A.nodes = ws.nodes;
+  A.first_leaf = (int32_t)(n - 1);
+  A.wild = ws.scratch + L.wild;
+  A.off = off;
+  A.desc = reinterpret_cast<uint32_t*>(ws.boxes);
+  A.stride = stride;
   const uint32_t* epoch = ws.scratch + L.epoch;
   const uint32_t grow_grid = std::max<uint32_t>(1, std::min<uint32_t>(div_up(stride, kGrowThreads), sms * 16));
   if (host_loop && !ws.ploc_host && (e = cudaMallocHost(&ws.ploc_host, 64)) != cudaSuccess) return e;
-  const bool same = host_loop || ws.tl_exec && ws.tl_key_n == n && ws.tl_key_nodes == ws.nodes && ws.tl_key_list == list &&
-                    ws.tl_key_desc == desc && ws.tl_key_ctl == ctl;
-  if (!same) {
-    if (ws.tl_exec) cudaGraphExecDestroy(ws.tl_exec);
-    ws.tl_exec = nullptr;
-    if ((e = make_height_graph(ws.nodes, list, off, ctl, desc, stride, grow_grid, (uint32_t)g_dp_grid[dev], narrow,
-                               &ws.tl_exec)) != cudaSuccess)
-      return e;
+  const auto kept = [&](int round) { return round + 1 < rounds ? ws.heights : nullptr; };
+  // one loop graph per choice of keeping the heights: [1] for a pass that another follows
+  for (int keep = rounds > 1 ? 1 : 0; keep >= 0 && !host_loop; --keep) {
+    const bool same = ws.tl_exec[keep] && ws.tl_key_n == n && ws.tl_key_nodes == ws.nodes && ws.tl_key_list == list &&
+                      ws.tl_key_desc == A.desc && ws.tl_key_ctl == ctl;
+    if (same) continue;
+    for (cudaGraphExec_t& x : ws.tl_exec) {
+      if (x) cudaGraphExecDestroy(x);
+      x = nullptr;
+    }
+    for (int k = 0; k <= (rounds > 1 ? 1 : 0); ++k) {
+      A.hgt = k ? ws.heights : nullptr;
+      if ((e = make_height_graph(A, list, ctl, grow_grid, (uint32_t)g_dp_grid[dev], narrow, &ws.tl_exec[k])) != cudaSuccess)
+        return e;
+    }
     ws.tl_key_n = n;
     ws.tl_key_nodes = ws.nodes;
     ws.tl_key_list = list;
-    ws.tl_key_desc = desc;
+    ws.tl_key_desc = A.desc;
     ws.tl_key_ctl = ctl;
   }
   ws.tl_narrow = narrow != 0;
+  if ((e = cudaMemsetAsync(ctl, 0, 4, st)) != cudaSuccess) return e;
   for (int r = 0; r < rounds && r + 1 < 0x20; ++r) {
+    A.hgt = kept(r);
     if ((e = cudaMemsetAsync(cnt, 0, 256 * 4, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(ctl, 0, 8 * 4, st)) != cudaSuccess) return e;  // [4]: k_tl_narrow's barrier
-    k_tl_heights<<<div_up(n, 256), 256, 0, st>>>(ws.nodes, ws.slots, epoch, (uint32_t)r, n, hgt, ctl);
-    k_tl_count<<<std::max<uint32_t>(1, std::min<uint32_t>(div_up(n - 1, 256), sms * 8)), 256, 0, st>>>(hgt, n - 1, cnt);
+    if ((e = cudaMemsetAsync(ctl + 1, 0, 7 * 4, st)) != cudaSuccess) return e;  // [4]: k_tl_narrow's barrier
+    k_tl_count<<<std::max<uint32_t>(1, std::min<uint32_t>(div_up(n - 1, 256), sms * 8)), 256, 0, st>>>(ws.heights, n - 1,
+                                                                                                      cnt, ctl);
     k_tl_offsets<<<1, 256, 0, st>>>(cnt, n - 1, off, cursor, ctl);
-    k_tl_scatter<<<div_up(n - 1, 256), 256, 0, st>>>(hgt, n - 1, cursor, list);
+    k_tl_scatter<<<div_up(n - 1, 256), 256, 0, st>>>(ws.heights, n - 1, cursor, list);
     // heights 1 to 3 first: every height-1 treelet has two leaves and is finished by the growth
-    // kernel; height 2 holds at most 4 leaves and takes the smaller DP; height 3 mixes treelet
-    // sizes (mostly 4 and 5 leaves, few 7) and runs one DP per size class
-    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(ws.nodes, list, off, ctl, desc, stride);
-    k_tl_step<false><<<1, 32, 0, st>>>(ctl, off, 0u, cudaGraphConditionalHandle{});
-    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(ws.nodes, list, off, ctl, desc, stride);
-    k_tl_dp<4><<<g_dp4_grid[dev], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
-    k_tl_step<false><<<1, 32, 0, st>>>(ctl, off, 0u, cudaGraphConditionalHandle{});
-    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(ws.nodes, list, off, ctl, desc, stride);
-    k_tl_dpc<4><<<g_dpc_grid[dev][0], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
-    k_tl_dpc<5><<<g_dpc_grid[dev][1], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
-    k_tl_dpc<6><<<g_dpc_grid[dev][2], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
-    k_tl_dpc<7><<<g_dpc_grid[dev][3], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
-    k_tl_step<false><<<1, 32, 0, st>>>(ctl, off, 0u, cudaGraphConditionalHandle{});
+    // kernel (in the first pass by the emission); height 2 holds at most 4 leaves and takes the smaller
+    // DP; height 3 mixes treelet sizes (mostly 4 and 5 leaves, few 7) and runs one DP per size class
+    if (r > 0) k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 1u);
+    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 2u);
+    k_tl_dp<4><<<g_dp4_grid[dev], kLvThreads, 0, st>>>(A, ctl, 2u);
+    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 3u);
+    k_tl_dpc<4><<<g_dpc_grid[dev][0], kLvThreads, 0, st>>>(A, ctl, 3u);
+    k_tl_dpc<5><<<g_dpc_grid[dev][1], kLvThreads, 0, st>>>(A, ctl, 3u);
+    k_tl_dpc<6><<<g_dpc_grid[dev][2], kLvThreads, 0, st>>>(A, ctl, 3u);
+    k_tl_dpc<7><<<g_dpc_grid[dev][3], kLvThreads, 0, st>>>(A, ctl, 3u);
     if (host_loop) {
       // read the largest height (and the too-high flag) once, then one grow + dp per height
       if ((e = cudaMemcpyAsync(ws.ploc_host, ctl, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
@@ -1060,12 +1190,12 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
         return e;
       const uint32_t maxh = ws.ploc_host[0] ? 0u : ws.ploc_host[1];
       for (uint32_t h = 4; h <= maxh; ++h) {
-        k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(ws.nodes, list, off, ctl, desc, stride);
-        k_tl_dp<kTlMax><<<g_dp_grid[dev], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
+        k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 0u);
+        k_tl_dp<kTlMax><<<g_dp_grid[dev], kLvThreads, 0, st>>>(A, ctl, 0u);
         k_tl_step<false><<<1, 32, 0, st>>>(ctl, off, 0u, cudaGraphConditionalHandle{});
       }
     } else {
-      if ((e = cudaGraphLaunch(ws.tl_exec, st)) != cudaSuccess) return e;
+      if ((e = cudaGraphLaunch(ws.tl_exec[A.hgt ? 1 : 0], st)) != cudaSuccess) return e;
       if (narrow) {  // the remaining heights, from where the graph's loop stopped
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((uint32_t)g_narrow_grid[dev]);
@@ -1077,8 +1207,8 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         e = ws.no_cooperative ? cudaErrorNotSupported
-                              : cudaLaunchKernelEx(&cfg, k_tl_narrow, ws.nodes, (const uint32_t*)list,
-                                                   (const uint32_t*)off, ctl, ws.scratch + L.status);
+                              : cudaLaunchKernelEx(&cfg, k_tl_narrow, A, (const uint32_t*)list, ctl,
+                                                   ws.scratch + L.status);
         if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
           // no co-resident grid (a client limited to part of the GPU, or asked for): the
           // remaining heights as one grow + dp launch each, driven from the host
@@ -1090,8 +1220,8 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
             return e;
           if (!ws.ploc_host[0])
             for (uint32_t h = ws.ploc_host[2]; h <= ws.ploc_host[1]; ++h) {
-              k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(ws.nodes, list, off, ctl, desc, stride);
-              k_tl_dp<kTlMax><<<g_dp_grid[dev], kLvThreads, 0, st>>>(ws.nodes, off, ctl, desc, stride);
+              k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 0u);
+              k_tl_dp<kTlMax><<<g_dp_grid[dev], kLvThreads, 0, st>>>(A, ctl, 0u);
               k_tl_step<false><<<1, 32, 0, st>>>(ctl, off, 0u, cudaGraphConditionalHandle{});
             }
         } else if (e != cudaSuccess) {
@@ -1099,7 +1229,8 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
         }
       }
     }
-    k_treelet_fallback<<<sms * 8, 64, 0, st>>>(ws.nodes, ws.slots, epoch, (uint32_t)r, n, ctl);
+    k_tl_parents<<<sms * 8, 256, 0, st>>>(ws.nodes, n - 1, parents, ctl);
+    k_treelet_fallback<<<sms * 8, 64, 0, st>>>(ws.nodes, parents, ws.slots, epoch, (uint32_t)r, n, ctl);
   }
   return cudaGetLastError();
 }
