@@ -27,7 +27,7 @@ struct BatchGraph {
 struct TuneEntry {
   int32_t algo = -1, bucket = -1;
   int32_t sort_variant = 0;
-  uint32_t tail_pairs = 100000;
+  uint32_t tail_pairs = 25000;
   int32_t nn_bps = 3, mg_bps = 8;
   uint32_t grid_max = 0xffffffffu;  // PLOC: k_ploc_grid from this many live clusters (0: never)
 };

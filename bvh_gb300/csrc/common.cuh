@@ -206,8 +206,9 @@ __device__ __forceinline__ bool grid_sync(uint32_t* bar, uint32_t target, uint32
                                           uint32_t limit = kSpinLimit) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(bar, 1u);
+    // release: what this block wrote is visible before its arrival; acquire: what the others wrote is
+    // visible after the last arrival (a fence on each side of a relaxed add cost 0.4 us per barrier)
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     uint32_t ok = 1, spins = 0;
     while (ld_acquire(bar) < target) {
       if (++spins > limit) {
@@ -215,9 +216,8 @@ __device__ __forceinline__ bool grid_sync(uint32_t* bar, uint32_t target, uint32
         ok = 0;
         break;
       }
-      __nanosleep(32);
+      if (spins > 64) __nanosleep(32);
     }
-    __threadfence();
     *s_ok = ok;
   }
   __syncthreads();

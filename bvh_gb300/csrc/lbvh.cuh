@@ -17,7 +17,7 @@ struct Workspace {
   uint32_t cap_n = 0;        // triangles the buffers can hold
   int sort_variant = 0;      // onesweep variant (bvh_autotune)
   // PLOC launch shapes (bvh_autotune_build); none of them changes the tree
-  uint32_t ploc_tail_pairs = 100000;  // hand over to k_ploc_tail below this many pair areas (0: never)
+  uint32_t ploc_tail_pairs = 25000;   // hand over to k_ploc_tail below this many pair areas (0: never)
   uint32_t ploc_grid_max = 0xffffffffu;  // k_ploc_grid takes over at this many live clusters
                                          // (capped at what its grid holds; 0: never)
   int ploc_nn_bps = 3;                // neighbour-search blocks per SM

@@ -772,6 +772,85 @@ __global__ void k_ploc_step(PlocBufs B, cudaGraphConditionalHandle handle) {
 constexpr int kTailThreads = 1024;
 constexpr uint32_t kTailMax = 2048;
 
+// log2 of the lanes that share one cluster's search of 2r pairs when a block of kTailThreads searches for
+// cnt clusters: as many as the block has to spare, but no more than have four pairs each.
+__device__ __forceinline__ int search_lanes(uint32_t cnt, int r) {
+  int lg = 0;
+  while (lg < 5 && (cnt << (lg + 1)) <= (uint32_t)kTailThreads && (4 << lg) < 2 * r) ++lg;
+  return lg;
+}
+
+// The searches of the one-launch kernels compare halves of areas: doubling is exact, so the order is the
+// same, and a half below 2^127 is an area below infinity.
+constexpr float kHalfInf = 0x1p127f;
+__device__ __forceinline__ float pair_half(float4 xa, float4 xb, float4 ja, float4 jb) {
+  const float dx = __fsub_rn(fmaxf(xb.x, jb.x), fminf(xa.x, ja.x)), dy = __fsub_rn(fmaxf(xb.y, jb.y), fminf(xa.y, ja.y)),
+              dz = __fsub_rn(fmaxf(xb.z, jb.z), fminf(xa.z, ja.z));
+  return __fmaf_rn(dz, dx, __fmaf_rn(dx, dy, __fmul_rn(dy, dz)));
+}
+
+// The nearest of the clusters j0..j1 (staged boxes) to cluster x of that range: the smallest area, the smallest
+// j on ties, -1 where none is below infinity.  Alone (lg = 0), a thread scans both sides of x without
+// checks; otherwise lane g of 2^lg takes every 2^lg-th j, four at a time, so that a search is not one
+// chain of shared-memory loads, and the lanes' bests are compared.  Every lane of the warp takes part.
+__device__ __forceinline__ int32_t group_nearest(const float4* lo, const float4* hi, int x, int j0, int j1, int g,
+                                                 int lg) {
+  const float4 xa = lo[x], xb = hi[x];
+  float best = kHalfInf;
+  int32_t bj = -1;
+  if (lg == 0) {
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+      const int e = side ? j1 + 1 : x;
+      int j = side ? x + 1 : j0;
+#pragma unroll 1
+      for (; j + 4 <= e; j += 4) {
+        float d[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[q] = pair_half(xa, xb, lo[j + q], hi[j + q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (d[q] < best) {  // ascending j: the first of equal areas stays
+            best = d[q];
+            bj = j + q;
+          }
+      }
+      for (; j < e; ++j) {
+        const float d = pair_half(xa, xb, lo[j], hi[j]);
+        if (d < best) {
+          best = d;
+          bj = j;
+        }
+      }
+    }
+    return bj;
+  }
+  for (int j = j0 + g; j <= j1; j += 4 << lg) {
+    float d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = j + (q << lg);
+      d[q] = pair_half(xa, xb, lo[min(k, j1)], hi[min(k, j1)]);
+      if (k > j1 || k == x) d[q] = kHalfInf;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (d[q] < best) {
+        best = d[q];
+        bj = j + (q << lg);
+      }
+  }
+  for (int o = 0; o < lg; ++o) {
+    const float od = __shfl_xor_sync(0xffffffffu, best, 1 << o);
+    const int32_t oj = __shfl_xor_sync(0xffffffffu, bj, 1 << o);
+    if (od < best || (od == best && oj < bj)) {  // (two without a candidate both have j = -1)
+      best = od;
+      bj = oj;
+    }
+  }
+  return bj;
+}
+
 uint32_t ploc_tail_threshold(int radius, uint32_t pairs) {
   if (pairs == 0) return 0;
   const uint32_t t = pairs / (2u * (uint32_t)std::max(radius, 1));
@@ -807,31 +886,24 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_ploc_tail(PlocBufs B, int r
   unsigned long long sum = (unsigned long long)__ldcg(B.ctrl + 9) << 32 | __ldcg(B.ctrl + 8);
   int cur = 0;
   bool no_progress = false;
-  const float kInf = __int_as_float(0x7f800000);
   __syncthreads();
-  while (true) {
+  while (c > 32) {
     sum += c;
     ++it;
     const float4* lo = s_lo[cur];
     const float4* hi = s_hi[cur];
-    // neighbours: ascending j with a strict < keeps the smallest j of equal areas
-    for (uint32_t x = tid; x < c; x += kTailThreads) {
-      const float4 xa = lo[x], xb = hi[x];
-      const uint32_t j0 = x > (uint32_t)r ? x - (uint32_t)r : 0u, j1 = min(c - 1, x + (uint32_t)r);
-      float best = kInf;
-      int32_t bj = -1;
-      for (uint32_t j = j0; j <= j1; ++j) {
-        if (j == x) continue;
-        const float d = pair_area(xa, xb, lo[j], hi[j]);
-        if (d < best) {
-          best = d;
-          bj = (int32_t)j;
-        }
+    {
+      const int lg = search_lanes(c, r), g = tid & ((1 << lg) - 1);
+      for (uint32_t base = (uint32_t)(wid * 32) >> lg; base < c; base += (uint32_t)kTailThreads >> lg) {
+        const uint32_t x = base + (uint32_t)(lane >> lg);  // (a warp without clusters skips the search)
+        const int xi = (int)min(x, c - 1);
+        const int32_t j = group_nearest(lo, hi, xi, max(0, xi - r), min((int)c - 1, xi + r), g, lg);
+        if (x < c && g == 0) s_nbr[x] = j;
       }
-      s_nbr[x] = bj;
     }
     __syncthreads();
     // merge and survivor flags of this thread's clusters x = 2 tid, 2 tid + 1 (ascending)
+    const bool busy = 64u * (uint32_t)wid < c;  // the warp has clusters
     uint32_t mk = 0, vk = 0;
     bool m2[2], v2[2];
 #pragma unroll
@@ -849,27 +921,21 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_ploc_tail(PlocBufs B, int r
       mk += mm;
       vk += vv;
     }
-    // block exclusive scan of (merges, survivors), packed 16 + 16 bits (c <= 2048)
+    // block exclusive scan of (merges, survivors), packed 16 + 16 bits (c <= 2048); every busy warp adds
+    // up the totals before it
     uint32_t packed = mk << 16 | vk, x = packed;
+    if (busy) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
     }
     if (lane == 31) s_w[wid] = x;
     __syncthreads();
-    if (wid == 0) {
-      uint32_t t = s_w[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += y;
-      }
-      s_w[32 + lane] = t;  // inclusive warp totals
-    }
-    __syncthreads();
-    const uint32_t before = (wid ? s_w[32 + wid - 1] : 0u) + x - packed;
-    const uint32_t total = s_w[32 + 31];
+    const uint32_t wt = s_w[lane];
+    const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < wid ? wt : 0u) + x - packed;
     uint32_t mpos = before >> 16, vpos = before & 0xffffu;
     const int nb = cur ^ 1;
 #pragma unroll
@@ -909,6 +975,68 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_ploc_tail(PlocBufs B, int r
     if (c >= prev || it >= cap) {  // no mutual pair anywhere, or the cap
       no_progress = true;
       break;
+    }
+  }
+  // The last 32 clusters: one warp, a cluster per lane, flags and positions from ballots, no barriers.
+  if (wid == 0 && !no_progress) {
+    const uint32_t lt = (1u << lane) - 1u;
+    while (c > 1) {
+      sum += c;
+      ++it;
+      const float4* lo = s_lo[cur];
+      const float4* hi = s_hi[cur];
+      const int x = min(lane, (int)c - 1);
+      float4 a = lo[x], b = hi[x];
+      float best = kHalfInf;
+      int32_t nbr = -1;
+      for (int j = 0; j < (int)c; j += 4) {
+        float d[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int k = min(j + q, (int)c - 1), away = j + q - x;
+          d[q] = pair_half(a, b, lo[k], hi[k]);
+          if (j + q >= (int)c || away == 0 || away > r || away < -r) d[q] = kHalfInf;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (d[q] < best) {
+            best = d[q];
+            nbr = j + q;
+          }
+      }
+      const bool in = lane < (int)c;
+      const int32_t back = __shfl_sync(0xffffffffu, nbr, nbr < 0 ? lane : nbr);
+      const bool mutual = in && nbr >= 0 && back == lane;
+      const uint32_t merges = __ballot_sync(0xffffffffu, mutual && lane < nbr);
+      const uint32_t lives = __ballot_sync(0xffffffffu, in && !(mutual && nbr < lane));
+      int32_t nid = s_id[cur][x];
+      if ((merges >> lane) & 1u) {
+        const float4 ja = lo[nbr], jb = hi[nbr];
+        a = make_float4(fminf(a.x, ja.x), fminf(a.y, ja.y), fminf(a.z, ja.z), 0.f);
+        b = make_float4(fmaxf(b.x, jb.x), fmaxf(b.y, jb.y), fmaxf(b.z, jb.z), 0.f);
+        const int32_t id_new = (int32_t)(next + __popc(merges & lt));
+        float4* np = reinterpret_cast<float4*>(B.nodes + id_new);
+        np[0] = a;
+        np[1] = b;
+        reinterpret_cast<int4*>(np + 2)[0] = make_int4(nid, s_id[cur][nbr], 0, 0);
+        if (nid == 0) B.ctrl[13] = (uint32_t)id_new;
+        nid = id_new;
+      }
+      if ((lives >> lane) & 1u) {
+        const uint32_t p = __popc(lives & lt);
+        s_lo[cur ^ 1][p] = a;
+        s_hi[cur ^ 1][p] = b;
+        s_id[cur ^ 1][p] = nid;
+      }
+      __syncwarp();
+      next += __popc(merges);
+      cur ^= 1;
+      const uint32_t prev = c;
+      c = __popc(lives);
+      if (c > 1 && (c >= prev || it >= cap)) {
+        no_progress = true;
+        break;
+      }
     }
   }
   if (tid == 0) {
@@ -979,7 +1107,8 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
   int32_t* s_id = reinterpret_cast<int32_t*>(gsm + 2 * kGridWin);
   int32_t* s_nbr = s_id + kGridWin;  // neighbours of [h0, h1)
   unsigned long long* s_w = reinterpret_cast<unsigned long long*>(s_nbr + kGridNbr);
-  __shared__ uint32_t s_ok;
+  __shared__ uint32_t s_ok, s_asked;
+  __shared__ uint32_t s_ask[2 * kGridMaxR];  // clusters outside the chunk whose neighbour is asked for
   const uint32_t G = gridDim.x, b = blockIdx.x;
   const int tid = threadIdx.x;
   if (b == 0 && tid == 0) B.ctrl[18] = 1;  // (no block reads it)
@@ -996,7 +1125,6 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
   unsigned long long* totals = reinterpret_cast<unsigned long long*>(B.flags);  // one per block
   uint32_t nbar = 0;
   bool no_progress = false, ok = true;
-  const float kInf = __int_as_float(0x7f800000);
   while (true) {
     const Box* cin = par ? B.cbox[1] : B.cbox[0];
     const int32_t* idin = par ? B.cid[1] : B.cid[0];
@@ -1013,23 +1141,32 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
       s_id[x - w0] = __ldcg(idin + x);
     }
     __syncthreads();
-    // neighbours of the chunk and r clusters either side: ascending j with a strict < keeps the
-    // smallest j of equal areas
-    for (uint32_t x = h0 + tid; x < h1; x += kGridThreads) {
-      const float4 xa = s_lo[x - w0], xb = s_hi[x - w0];
-      const uint32_t j0 = x > (uint32_t)r ? x - (uint32_t)r : 0u, j1 = min(c - 1, x + (uint32_t)r);
-      float best = kInf;
-      int32_t bj = -1;
-      for (uint32_t j = j0; j <= j1; ++j) {
-        if (j == x) continue;
-        const float d = pair_area(xa, xb, s_lo[j - w0], s_hi[j - w0]);
-        if (d < best) {
-          best = d;
-          bj = (int32_t)j;
-        }
+    // Neighbours of the chunk's clusters, then of those outside it (within r) that some of them point to: a
+    // mutual pair may cross the chunk's ends.  They are few, where all 2r of them were as many as the
+    // chunk itself.
+    const auto search = [&](uint32_t cnt, const auto& cluster) {
+      static_assert(kGridThreads == kTailThreads, "search_lanes");
+      const int lg = search_lanes(cnt, r), g = tid & ((1 << lg) - 1);
+      for (uint32_t base = (uint32_t)((tid >> 5) * 32) >> lg; base < cnt; base += (uint32_t)kGridThreads >> lg) {
+        const uint32_t k = base + (uint32_t)((tid & 31) >> lg);
+        const uint32_t x = cluster(min(k, cnt - 1));
+        const uint32_t j0 = x > (uint32_t)r ? x - (uint32_t)r : 0u, j1 = min(c - 1, x + (uint32_t)r);
+        const int32_t j = group_nearest(s_lo, s_hi, (int)(x - w0), (int)(j0 - w0), (int)(j1 - w0), g, lg);
+        if (k < cnt && g == 0) s_nbr[x - h0] = j < 0 ? -1 : j + (int32_t)w0;
       }
-      s_nbr[x - h0] = bj;
+    };
+    if (tid == 0) s_asked = 0;
+    for (uint32_t x = h0 + tid; x < h1; x += kGridThreads)
+      if (x < x0 || x >= x1) s_nbr[x - h0] = -2;  // not asked for
+    search(x1 - x0, [&](uint32_t k) { return x0 + k; });
+    __syncthreads();
+    for (uint32_t x = x0 + tid; x < x1; x += kGridThreads) {
+      const int32_t j = s_nbr[x - h0];
+      if (j >= 0 && ((uint32_t)j < x0 || (uint32_t)j >= x1) && atomicCAS(&s_nbr[(uint32_t)j - h0], -2, -3) == -2)
+        s_ask[atomicAdd(&s_asked, 1u)] = (uint32_t)j;
     }
+    __syncthreads();
+    search(s_asked, [&](uint32_t k) { return s_ask[k]; });
     __syncthreads();
     // merge / survivor flags of this thread's clusters x0 + kGridPer tid + q (ascending); a
     // neighbour j lies within r of x, so both j and its neighbour are in s_nbr
@@ -1041,7 +1178,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
       const uint32_t x = x0 + (uint32_t)kGridPer * (uint32_t)tid + (uint32_t)q;
       m2[q] = v2[q] = false;
       nj[q] = -1;
-      if (x < x1) {
+      if (x < x1) {  // (a chunk may be empty)
         const int32_t j = s_nbr[x - h0];
         const int32_t back = j >= 0 ? s_nbr[(uint32_t)j - h0] : -1;
         const bool mutual = j >= 0 && back == (int32_t)x;
@@ -1056,14 +1193,26 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
     const unsigned long long before = grid_block_scan((unsigned long long)mk << 32 | vk, s_w, &btot);
     if (tid == 0) __stcg(totals + b, btot);
     if (!(ok = grid_sync(bar, ++nbar * G, B.status, &s_ok))) break;
-    // this block's offset and the totals over all blocks
-    unsigned long long mine = 0;
-    for (uint32_t k = (uint32_t)tid; k < G; k += kGridThreads) mine += k < b ? __ldcg(totals + k) : 0ull;
-    unsigned long long all = 0;
-    for (uint32_t k = (uint32_t)tid; k < G; k += kGridThreads) all += __ldcg(totals + k);
-    unsigned long long offs_b, grand_b;  // the block sums of `mine` and `all`
-    grid_block_scan(mine, s_w, &offs_b);
-    grid_block_scan(all, s_w, &grand_b);
+    // this block's offset and the totals over all blocks, added up by one warp
+    if (tid < 32) {
+      unsigned long long mine = 0, all = 0;
+      for (uint32_t k = (uint32_t)tid; k < G; k += 32) {
+        const unsigned long long t = __ldcg(totals + k);
+        all += t;
+        if (k < b) mine += t;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        mine += __shfl_xor_sync(0xffffffffu, mine, o);
+        all += __shfl_xor_sync(0xffffffffu, all, o);
+      }
+      if (tid == 0) {
+        s_w[0] = mine;
+        s_w[1] = all;
+      }
+    }
+    __syncthreads();
+    const unsigned long long offs_b = s_w[0], grand_b = s_w[1];
     uint32_t mpos = (uint32_t)(offs_b >> 32) + (uint32_t)(before >> 32);
     uint32_t vpos = (uint32_t)offs_b + (uint32_t)before;
     const uint32_t M = (uint32_t)(grand_b >> 32), V = (uint32_t)grand_b;
@@ -1261,7 +1410,7 @@ cudaError_t workspace_reserve_ploc(Workspace& ws, uint32_t n) {
   // (smaller tiles in late iterations: at most one partial tile's worth more; never more tiles
   // than the grid, so desc_words holds their totals)
   size_t flag_words = (size_t)div_up(cap, kPlocTile) * (kPlocThreads / 32) * kPlocRounds +
-                      (kPlocThreads / 32) * kPlocRounds;
+                      (kPlocThreads / 32) * kPlocRounds + kGridMaxBlocks;  // (k_ploc_grid: one total per block)
   if ((e = cudaMalloc(&ws.nbr, (size_t)cap * 4 + desc_words * 8 + flag_words * 8 + 64)) != cudaSuccess) return e;
   ws.ploc_cap = cap;
   return cudaSuccess;
@@ -1401,12 +1550,12 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
   const uint32_t cap = max_iter > 0 ? (uint32_t)max_iter : n;
   const uint32_t tail = ploc_tail_threshold(radius, ws.ploc_tail_pairs);
   // k_ploc_grid: from grid_at live clusters down to the tail hand-over (its per-block totals
-  // live in the ballot words, which hold them from 65,536 triangles on)
+  // live in the ballot words)
   const uint32_t grid_blocks = ploc_grid_blocks();
   uint32_t grid_at = 0;
-  if (grid_blocks && radius <= kGridMaxR && n >= 65536)
+  if (grid_blocks && radius <= kGridMaxR)
     grid_at = std::min<uint32_t>(ws.ploc_grid_max, grid_blocks * kGridPerBlock);
-  if (grid_at <= tail) grid_at = 0;
+  if (grid_at <= tail || n <= tail) grid_at = 0;
   const bool loop = n > 1 && n > std::max(tail, grid_at);  // else the one-launch kernels do every iteration
   const PlocShape sh = ploc_shape(ws);
   if (host_loop && !ws.ploc_host && (e = cudaMallocHost(&ws.ploc_host, 64)) != cudaSuccess) return e;
