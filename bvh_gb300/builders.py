@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import abc
 import ctypes
+import sys
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -64,6 +65,38 @@ class TriangleMesh:
         return v.min(0), v.max(0)
 
 
+class _HostArrays:
+    """Memory for the arrays that builds return.  The pages of a new 100 MB array cost three times what
+    copying a tree into it does, so memory that nobody refers to any more (every array made from it is
+    gone) serves the next result.  At most `keep` idle pieces stay, none more than twice as large as asked for."""
+
+    def __init__(self, keep: int = 2):
+        self._keep = keep
+        self._pieces: list = []
+
+    def take(self, dtype, count: int) -> np.ndarray:
+        """An array of `count` items, uninitialised."""
+        dtype = np.dtype(dtype)
+        need = count * dtype.itemsize
+        if need < 1 << 20:
+            return np.empty(count, dtype)
+        idle, busy, found = [], [], None
+        pieces, self._pieces = self._pieces, []
+        while pieces:
+            piece = pieces.pop()
+            # the only references left: this name and getrefcount's argument (a view refers to its piece)
+            if sys.getrefcount(piece) > 2:
+                busy.append(piece)
+            elif found is None and need <= piece.size <= 2 * need:
+                found = piece
+            else:
+                idle.append(piece)
+        if found is None:
+            found = np.empty(need, np.uint8)
+        self._pieces = (idle[: self._keep] + busy)[:: -1] + [found]
+        return found[:need].view(dtype)
+
+
 class Context:
     """A library context on one CUDA device (owns the workspace and the last tree)."""
 
@@ -73,8 +106,10 @@ class Context:
         C.check(self.lib.bvh_ctx_create(ctypes.byref(h), int(device)), "bvh_ctx_create")
         self.handle = h
         self.device = device
+        self._host = _HostArrays()
 
     def close(self):
+        self._host = _HostArrays()
         if self.handle:
             self.lib.bvh_ctx_destroy(self.handle)
             self.handle = None
@@ -181,8 +216,8 @@ class Context:
         n = mesh.size()
         arrs = mesh.arrays()
         m = C.mesh_struct([a.ctypes.data for a in arrs], n)
-        nodes = np.zeros(max(2 * n - 1, 0), C.NODE_DTYPE)
-        idx = np.zeros(n, np.uint32)
+        nodes = self._host.take(C.NODE_DTYPE, max(2 * n - 1, 0))
+        idx = self._host.take(np.uint32, n)
         nn = ctypes.c_uint32(0)
         C.check(self.lib.bvh_build_host(self.handle, ctypes.byref(m), ctypes.byref(params), ctypes.c_void_p(stream),
                                         nodes.ctypes.data if n else None, idx.ctypes.data if n else None,
@@ -190,8 +225,8 @@ class Context:
         return nodes[: nn.value], idx
 
     def download(self, tree: C.Tree, stream: int = 0):
-        nodes = np.zeros(tree.n_nodes, C.NODE_DTYPE)
-        idx = np.zeros(tree.n_prims, np.uint32)
+        nodes = self._host.take(C.NODE_DTYPE, tree.n_nodes)
+        idx = self._host.take(np.uint32, tree.n_prims)
         if tree.n_nodes:
             C.check(self.lib.bvh_tree_download(self.handle, ctypes.byref(tree), ctypes.c_void_p(stream),
                                                nodes.ctypes.data, idx.ctypes.data), "bvh_tree_download")

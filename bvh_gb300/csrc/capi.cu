@@ -9,6 +9,7 @@
 
 #include "../../include/bvh_gb300.h"
 #include "lbvh.cuh"
+#include "prefault.h"
 #include "trace.cuh"
 
 using namespace bvhgb;
@@ -387,6 +388,10 @@ extern "C" bvh_status bvh_build_host(bvh_ctx* ctx, const bvh_mesh_soa* mesh, con
     if (e != cudaSuccess) return from_cuda(e);
     ws.mesh_cap = n;
   }
+  // the output pages become present while the mesh goes up and the build runs
+  void* const out_ptr[2] = {host_indices, host_nodes};
+  const size_t out_bytes[2] = {(size_t)n * 4, (2 * (size_t)n - 1) * sizeof(bvh_node)};
+  Prefault pages(out_ptr, out_bytes, 2);
   const size_t stride = ((size_t)ws.mesh_cap + 3) & ~size_t(3);
   const float* src[9] = {mesh->v0x, mesh->v0y, mesh->v0z, mesh->v1x, mesh->v1y, mesh->v1z,
                          mesh->v2x, mesh->v2y, mesh->v2z};
@@ -418,6 +423,7 @@ extern "C" bvh_status bvh_build_host(bvh_ctx* ctx, const bvh_mesh_soa* mesh, con
   bvh_status s = build_impl(ctx, &dm, params, st, &tree);
   ws.indices_ready = ws.leaves_ready = nullptr;
   if (s != BVH_OK) return s;
+  pages.finish();
   if (early) {
     cudaStream_t dl = ctx->dl_stream;
     cudaError_t e = cudaStreamWaitEvent(dl, ctx->ev_sorted, 0);  // sort (and run fix-up) done

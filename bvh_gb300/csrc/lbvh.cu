@@ -486,13 +486,13 @@ void sort_variant_describe(int v, int* ipt, int* window, int* minb) {
 }
 
 // Kernel attributes set once per device, outside any stream capture.
-cudaError_t prepare_kernels() {
+cudaError_t prepare_kernels(bool small) {
   for (int v = 0; v < kNumVariants; ++v) {
     const SortVariant& sv = variant(v);
     cudaError_t e = cudaFuncSetAttribute(sv.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sv.smem);
     if (e != cudaSuccess) return e;
   }
-  return prepare_small();
+  return small ? prepare_small() : cudaSuccess;
 }
 
 // `passes` stable 8-bit passes over the 32-bit keys in ws.keys[0] (values: the original index).

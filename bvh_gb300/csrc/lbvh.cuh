@@ -79,6 +79,7 @@ struct Workspace {
   // build's own kernel has written it
   uint32_t* report = nullptr;
   bool reported = false;
+  uint32_t small_ready = 0;  // one-block kernels whose attributes are set, by variant
 };
 
 // First epoch value; every build adds kEpochStride (emission uses E, treelet round r uses E+1+r).
@@ -178,7 +179,9 @@ cudaError_t wait_selftest(uint32_t limit, uint32_t* status_out);
 cudaError_t grid_wait_selftest(uint32_t limit, uint32_t* status_out);
 
 // Kernel attributes (dynamic shared memory limits), set once per device before any capture.
-cudaError_t prepare_kernels();
+// small: those of the one-block builds too (14 kernels to load, 0.2 ms), which a workspace otherwise sets
+// when it first needs each.
+cudaError_t prepare_kernels(bool small = false);
 
 // Count one build that bumps the epoch; before the build that would reuse an old epoch, clear the
 // rendezvous slots on `st`.  Not counted while `st` is being captured: each launch of the graph

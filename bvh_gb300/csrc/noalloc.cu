@@ -53,7 +53,7 @@ cudaError_t static_scratch(int device, unsigned char** out) {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(g_mutex);
   if (!g_prepared[device]) {
-    e = prepare_kernels();
+    e = prepare_kernels(true);
     if (e != cudaSuccess) return e;
     g_prepared[device] = true;
   }
@@ -105,6 +105,7 @@ extern "C" bvh_status bvh_build_lbvh_static(const bvh_mesh_soa* mesh, int32_t mo
     g_epoch_builds[device] = ws.epoch_builds + 1;
   }
   ws.sort_variant = default_sort_variant(n);
+  ws.small_ready = ~0u;  // set with the others, once per device
   cudaError_t e = lbvh_build(ws, m, n, morton_bits, 0, reinterpret_cast<cudaStream_t>(stream), nullptr, &out_idx);
   if (e != cudaSuccess) return BVH_ERR_DEVICE;
   return out_idx == indices ? BVH_OK : BVH_ERR_DEVICE;

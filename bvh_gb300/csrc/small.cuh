@@ -277,6 +277,11 @@ static cudaError_t small_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int
   if (e != cudaSuccess) return e;
   size_t smem = 0;
   const void* fn = small_kernel(bits, mode, n, &smem);
+  const uint32_t bit = 1u << ((mode * 3 + (bits == 60) + 2 * (bits == 63)) * 2 + (n > (uint32_t)kSmallThreads));
+  if (!(ws.small_ready & bit)) {
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    ws.small_ready |= bit;
+  }
   MeshPtrs mp = m;
   ScratchLayout Lc = L;
   void* args[] = {&mp, &n, &ws.vals[0], &ws.boxes, &ws.nodes, &ws.scratch, &Lc, &host, &ws.heights};

@@ -98,3 +98,22 @@ def test_host_builder(gpu, oracle_lib):
         b.build(m)
         assert _equal(oracle_lib, (b.getNodes(), b.getIndices()), oracle_lib.lbvh(m.arrays(), 63))
         assert b.getLastBuildTimeMS() > 0
+
+
+@pytest.mark.parametrize("n,bits", [(1000, 30), (2000, 63)])
+def test_first_build_captured(gpu, oracle_lib, n, bits):
+    """A context whose first build of its kind is recorded into a graph."""
+    c = Context(0)
+    m = meshgen.clustered(n, seed=n)
+    _, ptrs = to_device(gpu, m.arrays())
+    p = c.params(C.ALGO_LBVH, morton_bits=bits)
+    c.reserve(n)
+    gpu.cuda.synchronize()
+    g = gpu.cuda.CUDAGraph()
+    with gpu.cuda.graph(g):
+        tree = c.build_device(ptrs, n, p, stream(gpu))
+    g.replay()
+    gpu.cuda.synchronize()
+    assert _equal(oracle_lib, c.download(tree, stream(gpu)), oracle_lib.lbvh(m.arrays(), bits))
+    del g
+    c.close()
