@@ -247,114 +247,258 @@ __device__ __forceinline__ void nn_tiles(const PlocBufs& B, int r, uint32_t c, c
   }
 }
 
-// The large iterations take a second form of the same search (ploc_builder.cu:173-209), which
-// moves about half the shared-memory bytes: thread t owns kNcP consecutive clusters x0 .. x0 + 3, so each window box
-// it loads serves all four (r + 3 loads for 4r pairs instead of 4r), and the backward candidates
-// a thread produces for one later cluster are reduced to one (area, index) entry before they go
-// through the shared-memory table.  Both searches pick the smallest (area, index) pair in each
-// direction, so they give the same neighbours.  The first H = ceil(r / kNcP) threads of a tile hold
-// the r clusters before it: they only feed backward candidates.  Window box w is stored at
-// w ^ ((w >> 3) & 3), which puts the 16-byte boxes that 8 lanes read -- every fourth box, or 8
-// consecutive ones -- in distinct bank groups.
-constexpr int kNcP = 4;      // consecutive clusters per thread
-constexpr int kNcQ = 4;      // thread distances per table round
-constexpr int kNcMaxR = 128;  // larger radii keep the strided form (a halo of 32 threads at 128)
-__host__ __device__ constexpr int nc_swz(int w) { return w ^ ((w >> 3) & 3); }
-// boxes staged: the halo, the tile, r past it, + kNcP read past the last pair; rounded to 8
-__host__ __device__ constexpr int nc_span(int r) { return (kPlocThreads * kNcP + r + kNcP + 7) & ~7; }
-static size_t nc_smem(int r) {
-  const int h = (r + kNcP - 1) / kNcP;
-  return 2 * 16 * (size_t)nc_span(r) + 8 * (size_t)kNcQ * kNcP * (kPlocThreads + h);
+// Searches that keep no areas compare halves: doubling is exact, so the order is the same, and a half below
+// 2^127 is an area below infinity.
+constexpr float kHalfInf = 0x1p127f;
+__device__ __forceinline__ float pair_half(float4 xa, float4 xb, float4 ja, float4 jb) {
+  const float dx = __fsub_rn(fmaxf(xb.x, jb.x), fminf(xa.x, ja.x)), dy = __fsub_rn(fmaxf(xb.y, jb.y), fminf(xa.y, ja.y)),
+              dz = __fsub_rn(fmaxf(xb.z, jb.z), fminf(xa.z, ja.z));
+  return __fmaf_rn(dz, dx, __fmaf_rn(dx, dy, __fmul_rn(dy, dz)));
 }
 
-template <bool SEG, bool CHECK>
-__device__ __forceinline__ void nc_pairs(int r, int c, int x0, int o, const float4 (&a)[kNcP], const float4 (&b)[kNcP],
-                                         float4 jl, float4 jh, float (&fd)[kNcP], int (&fj)[kNcP], float& pa,
-                                         int& ps) {
+// The large iterations take a second form of the same search (ploc_builder.cu:173-209): thread t owns kNcP
+// consecutive clusters x0 .. x0 + 3, so each window box it loads serves all four (r + 3 loads for 4r pairs),
+// and the backward candidates it produces for one later cluster are reduced to one before they go
+// through the shared-memory table, a distance q of threads at a time.  The first h = ceil(r / kNcP)
+// threads of a tile hold the r clusters before it: they only feed backward candidates.  One box in nine
+// of the window's storage is unused, which puts the 16-byte boxes that 8 lanes read -- every fourth
+// box, or 8 consecutive ones -- in distinct bank groups at constant offsets from a thread's first.
+// What bounds it is instructions (the six min/max of a pair on the half-rate pipe, three blocks per SM
+// by registers), and what it loads waits on L1, whose lines loads in flight need and the window takes:
+// pairs past the last distances' ends only are checked against r, areas are halves, and the table
+// holds one distance.  First iteration on 10M: r = 25
+// 319 -> 275 us, r = 100 (nc_tile_min) 1,071 -> 826.
+// Two pairs per packed add or multiply took longer than two single ones (its operands are moved into place).
+constexpr int kNcP = 4;      // consecutive clusters per thread
+constexpr int kNcMaxR = 128;  // larger radii keep the strided form (a halo of 32 threads at 128)
+// From here on nc_tile_min: settling indexes at the end costs as much as 30 radii of keeping them (4M, whole loop:
+// r = 10 1,674 against 1,566 us, 25 2,363 / 2,325, 32 2,595 / 2,629, 64 3,818 / 4,045).
+constexpr int kNcMinR = 32;
+__host__ __device__ constexpr int nc_at(int w) { return w + (w >> 3); }
+// boxes staged: the halo, the tile, r past it, + kNcP read past the last pair; rounded to 8
+__host__ __device__ constexpr int nc_span(int r) { return nc_at((kPlocThreads * kNcP + r + kNcP + 7) & ~7); }
+// per thread, the table holds a distance's four (area, index) twice, or its four areas once
+__host__ __device__ constexpr int nc_table(int r) { return (r < kNcMinR ? 4 : 1) * (kPlocThreads + (r + kNcP - 1) / kNcP); }
+static size_t nc_smem(int r) { return 16 * (2 * (size_t)nc_span(r) + nc_table(r)); }
+
+template <bool SEG>
+__device__ __forceinline__ float nc_half(float4 xa, float4 xb, float4 ja, float4 jb) {
+  if (SEG && __float_as_int(xa.w) != __float_as_int(ja.w)) return kHalfInf;  // (two meshes: no area)
+  return pair_half(xa, xb, ja, jb);
+}
+
+// The thread's clusters against box j = x0 + o (those with m < o <= m + r): fd, fj and the smallest of the four,
+// with its index.
+template <bool SEG, bool CHECK, bool EDGE>
+__device__ __forceinline__ float2 nc_four(int r, int c, int x0, int o, const float4 (&a)[kNcP],
+                                          const float4 (&b)[kNcP], float4 jl, float4 jh, float (&fd)[kNcP],
+                                          int (&fj)[kNcP]) {
+  static_assert(kNcP == 4, "two halves");
+  float t[2];
+  int i[2];
 #pragma unroll
-  for (int m = 0; m < kNcP; ++m) {
-    if (m < o && o - m <= r) {
-      float d = pair_d<SEG>(a[m], b[m], jl, jh);
-      if (CHECK && !(x0 + m >= 0 && x0 + o < c)) d = __int_as_float(0x7f800000);
-      if (d < fd[m]) {  // increasing o: the first of equal areas stays
-        fd[m] = d;
-        fj[m] = x0 + o;
-      }
-      if (d < pa) {  // increasing m: the smaller index stays
-        pa = d;
-        ps = x0 + m;
+  for (int k = 0; k < 2; ++k) {
+    t[k] = kHalfInf;
+    i[k] = 2 * k;
+    if (EDGE && (o <= 2 * k || o - 2 * k - 1 > r)) continue;  // (the same for every thread)
+    float d[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int m = 2 * k + e;
+      d[e] = nc_half<SEG>(a[m], b[m], jl, jh);
+      if (EDGE && (o <= m || o - m > r)) d[e] = kHalfInf;
+      if (CHECK && !(x0 + m >= 0 && x0 + o < c)) d[e] = kHalfInf;
+      if (d[e] < fd[m]) {  // increasing o: the first of equal areas stays
+        fd[m] = d[e];
+        fj[m] = o;
       }
     }
+    t[k] = fminf(d[0], d[1]);  // (NaN only where both are)
+    if (t[k] != d[0]) i[k] = 2 * k + 1;
+  }
+  const float m = fminf(t[0], t[1]);
+  return make_float2(m, __int_as_float(x0 + (m == t[0] ? i[0] : i[1])));
+}
+
+// Group q, the clusters of thread t + q, whose table entry is col.
+template <bool SEG, bool CHECK, bool EDGE>
+__device__ __forceinline__ void nc_group(int r, int c, int x0, int q, const float4 (&a)[kNcP], const float4 (&b)[kNcP],
+                                         const float4* s_lo, const float4* s_hi, float4* col, int tw,
+                                         float (&fd)[kNcP], int (&fj)[kNcP]) {
+  const int w = nc_at(kNcP * ((int)threadIdx.x + q));  // (four boxes from a multiple of four on are adjacent)
+  const float4* lo = s_lo + w;
+  const float4* hi = s_hi + w;
+#pragma unroll
+  for (int mp = 0; mp < kNcP; mp += 2) {
+    const float2 e = nc_four<SEG, CHECK, EDGE>(r, c, x0, kNcP * q + mp, a, b, lo[mp], hi[mp], fd, fj);
+    const float2 f = nc_four<SEG, CHECK, EDGE>(r, c, x0, kNcP * q + mp + 1, a, b, lo[mp + 1], hi[mp + 1], fd, fj);
+    col[mp / 2 * tw] = make_float4(e.x, e.y, f.x, f.y);
   }
 }
 
 template <bool SEG, bool CHECK>
 __device__ __forceinline__ void nc_tile(const PlocBufs& B, int r, int c, int lo, int h, const float4* s_lo,
-                                        const float4* s_hi, float2* sT) {
-  constexpr int P = kNcP, Q = kNcQ;
+                                        const float4* s_hi, float4* sT) {
+  constexpr int P = kNcP;
   const int t = threadIdx.x, tw = kPlocThreads + h;
   const int x0 = lo + P * t;
-  const float kInf = __int_as_float(0x7f800000);
   float4 a[P], b[P];
   float fd[P], ed[P];
-  int fj[P], ej[P];
+  int fj[P], ej[P];  // fj: relative to x0
 #pragma unroll
   for (int m = 0; m < P; ++m) {
-    a[m] = s_lo[nc_swz(P * t + m)];
-    b[m] = s_hi[nc_swz(P * t + m)];
-    fd[m] = ed[m] = kInf;
-    fj[m] = ej[m] = -1;
+    a[m] = s_lo[nc_at(P * t) + m];
+    b[m] = s_hi[nc_at(P * t) + m];
+    fd[m] = ed[m] = kHalfInf;
+    fj[m] = 0;
+    ej[m] = -1;
   }
   // pairs among the thread's own clusters
 #pragma unroll
   for (int o = 1; o < P; ++o) {
-    float pa = kInf;
-    int ps = -1;
-    nc_pairs<SEG, CHECK>(r, c, x0, o, a, b, a[o], b[o], fd, fj, pa, ps);
-    if (pa < ed[o] || (pa == ed[o] && ps < ej[o])) {
-      ed[o] = pa;
-      ej[o] = ps;
+    const float2 e = nc_four<SEG, CHECK, true>(r, c, x0, o, a, b, a[o], b[o], fd, fj);
+    if (e.x < kHalfInf) {
+      ed[o] = e.x;
+      ej[o] = __float_as_int(e.y);
     }
   }
-  // pairs with the clusters of the threads q = 1 .. h further on, Q distances per table round
-  for (int q0 = 1; q0 <= h; q0 += Q) {
-    const int qn = min(Q, h - q0 + 1);
-    for (int s = 0; s < qn; ++s) {
-      const int q = q0 + s;
-#pragma unroll
-      for (int mp = 0; mp < P; ++mp) {
-        const int o = P * q + mp;
-        const int w = nc_swz(P * t + o);
-        float pa = kInf;
-        int ps = -1;
-        nc_pairs<SEG, CHECK>(r, c, x0, o, a, b, s_lo[w], s_hi[w], fd, fj, pa, ps);
-        sT[(s * P + mp) * tw + t + q] = make_float2(pa, __int_as_float(ps));
-      }
-    }
+  // pairs with the clusters of the threads q = 1 .. h further on; every pair up to distance qf is within r
+  const int qf = r >= P - 1 ? (r - (P - 1)) / P : 0;
+  for (int q = 1, buf = 0; q <= h; ++q, buf ^= P / 2 * tw) {
+    if (q <= qf) nc_group<SEG, CHECK, false>(r, c, x0, q, a, b, s_lo, s_hi, sT + buf + t + q, tw, fd, fj);
+    else nc_group<SEG, CHECK, true>(r, c, x0, q, a, b, s_lo, s_hi, sT + buf + t + q, tw, fd, fj);
     __syncthreads();
-    for (int s = 0; s < qn; ++s) {
 #pragma unroll
-      for (int mp = 0; mp < P; ++mp) {
-        const float2 e = sT[(s * P + mp) * tw + t];
-        const int es = __float_as_int(e.y);
-        if (e.x < ed[mp] || (e.x == ed[mp] && es < ej[mp])) {  // the smaller index wins ties
-          ed[mp] = e.x;
-          ej[mp] = es;
-        }
+    for (int mp = 0; mp < P; mp += 2) {
+      const float4 e = sT[buf + mp / 2 * tw + t];
+      if (e.x <= ed[mp]) {  // a larger distance has the smaller indices: it wins ties
+        ed[mp] = e.x;
+        ej[mp] = __float_as_int(e.y);
+      }
+      if (e.z <= ed[mp + 1]) {
+        ed[mp + 1] = e.z;
+        ej[mp + 1] = __float_as_int(e.w);
       }
     }
-    __syncthreads();  // the table is refilled by the next round
   }
   if (t >= h) {
 #pragma unroll
     for (int m = 0; m < P; ++m) {
       const int x = x0 + m;
-      if (x < c) B.nbr[x] = (ej[m] >= 0 && ed[m] <= fd[m]) ? ej[m] : fj[m];  // earlier index wins ties
+      // the earlier index wins ties
+      if (x < c) B.nbr[x] = ed[m] < kHalfInf && ed[m] <= fd[m] ? ej[m] : fd[m] < kHalfInf ? x0 + fj[m] : -1;
     }
   }
 }
 
-template <bool SEG>
+// The thread's four clusters against box j = x0 + o: d[m], kHalfInf where not m < o <= m + r.
+template <bool SEG, bool CHECK, bool EDGE>
+__device__ __forceinline__ void nc_areas(int r, int c, int x0, int o, const float4 (&a)[kNcP], const float4 (&b)[kNcP],
+                                        float4 jl, float4 jh, float (&d)[kNcP]) {
+#pragma unroll
+  for (int m = 0; m < kNcP; ++m) {
+    d[m] = kHalfInf;
+    if (EDGE && (o <= m || o - m > r)) continue;  // (the same for every thread)
+    d[m] = nc_half<SEG>(a[m], b[m], jl, jh);
+    if (CHECK && !(x0 + m >= 0 && x0 + o < c)) d[m] = kHalfInf;
+  }
+}
+template <bool SEG, bool CHECK, bool EDGE>
+__device__ __forceinline__ void nc_group_min(int r, int c, int x0, int q, const float4 (&a)[kNcP], const float4 (&b)[kNcP],
+                                         const float4* s_lo, const float4* s_hi, float4* col, float (&fm)[kNcP]) {
+  static_assert(kNcP == 4, "one float4 of the table");
+  const int w = nc_at(kNcP * ((int)threadIdx.x + q));
+  const float4* lo = s_lo + w;
+  const float4* hi = s_hi + w;
+  float e[kNcP];
+#pragma unroll
+  for (int mp = 0; mp < kNcP; ++mp) {
+    float d[kNcP];
+    nc_areas<SEG, CHECK, EDGE>(r, c, x0, kNcP * q + mp, a, b, lo[mp], hi[mp], d);
+#pragma unroll
+    for (int m = 0; m < kNcP; ++m) fm[m] = mp == 0 ? d[m] : fminf(fm[m], d[m]);
+    e[mp] = fminf(fminf(d[0], d[1]), fminf(d[2], d[3]));
+  }
+  *col = make_float4(e[0], e[1], e[2], e[3]);
+}
+
+// The form of radii from kNcMinR on keeps only smallest areas, with the group q of four clusters -- thread t + q's
+// or t - q's -- that they were seen in, and settles the index at the end, once per cluster: the winning
+// group's four areas are computed again (the same bits) and the first that equals the minimum is the
+// neighbour.
+template <bool SEG, bool CHECK>
+__device__ __forceinline__ void nc_tile_min(const PlocBufs& B, int r, int c, int lo, int h, const float4* s_lo,
+                                        const float4* s_hi, float4* sT) {
+  constexpr int P = kNcP;
+  const int t = threadIdx.x;
+  const int x0 = lo + P * t;
+  float4 a[P], b[P];
+  float fd[P], ed[P];
+  uint32_t fe[P];  // the groups of fd (low half) and ed
+#pragma unroll
+  for (int m = 0; m < P; ++m) {
+    a[m] = s_lo[nc_at(P * t) + m];
+    b[m] = s_hi[nc_at(P * t) + m];
+    fd[m] = ed[m] = kHalfInf;
+    fe[m] = 0;
+  }
+  // group 0, the thread's own clusters
+#pragma unroll
+  for (int o = 1; o < P; ++o) {
+    float d[P];
+    nc_areas<SEG, CHECK, true>(r, c, x0, o, a, b, a[o], b[o], d);
+#pragma unroll
+    for (int m = 0; m < P; ++m)
+      if (m < o) {
+        fd[m] = fminf(fd[m], d[m]);
+        ed[o] = fminf(ed[o], d[m]);
+      }
+  }
+  // groups 1 .. h; every pair of groups up to qf is within r
+  const int qf = r >= P - 1 ? (r - (P - 1)) / P : 0;
+  for (int q = 1; q <= h; ++q) {
+    float fm[P];
+    if (q <= qf) nc_group_min<SEG, CHECK, false>(r, c, x0, q, a, b, s_lo, s_hi, sT + t + q, fm);
+    else nc_group_min<SEG, CHECK, true>(r, c, x0, q, a, b, s_lo, s_hi, sT + t + q, fm);
+#pragma unroll
+    for (int m = 0; m < P; ++m)
+      if (fm[m] < fd[m]) {  // increasing distance: the first of equal areas stays
+        fd[m] = fm[m];
+        fe[m] = __byte_perm(fe[m], q, 0x3254);
+      }
+    __syncthreads();
+    const float4 e4 = sT[t];
+    const float e[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+    for (int mp = 0; mp < P; ++mp)
+      if (e[mp] <= ed[mp]) {  // a larger distance has the smaller indices: it wins ties
+        ed[mp] = e[mp];
+        fe[mp] = __byte_perm(fe[mp], q, 0x5410);
+      }
+    __syncthreads();  // the table is refilled by the next distance
+  }
+  if (t < h) return;
+#pragma unroll
+  for (int m = 0; m < P; ++m) {
+    const int x = x0 + m;
+    if (x >= c) break;
+    const bool back = ed[m] <= fd[m];  // the earlier index wins ties
+    const float best = back ? ed[m] : fd[m];
+    int nb = -1;
+    if (best < kHalfInf) {
+      const int g = back ? t - (int)(fe[m] >> 16) : t + (int)(fe[m] & 0xffffu), y0 = lo + P * g;
+      const int lim0 = back ? max(x - r, 0) : x + 1, lim1 = back ? x - 1 : min(x + r, c - 1);
+      const float4* gl = s_lo + nc_at(P * g);
+      const float4* gh = s_hi + nc_at(P * g);
+#pragma unroll
+      for (int mp = P - 1; mp >= 0; --mp)  // descending: the smallest index stays
+        if (nc_half<SEG>(gl[mp], gh[mp], a[m], b[m]) == best && y0 + mp >= lim0 && y0 + mp <= lim1) nb = y0 + mp;
+    }
+    B.nbr[x] = nb;
+  }
+}
+
+template <bool SEG, bool MIN>
 __device__ __forceinline__ void nn_tiles_consec(const PlocBufs& B, int r, uint32_t c, const Box* __restrict__ cbox,
                                                 float4* sw) {
   const int h = (r + kNcP - 1) / kNcP;            // halo threads = the largest thread distance of a pair
@@ -362,7 +506,7 @@ __device__ __forceinline__ void nn_tiles_consec(const PlocBufs& B, int r, uint32
   const int span = kPlocThreads * kNcP + r;       // boxes staged: the halo, the tile, r past it
   float4* s_lo = sw;
   float4* s_hi = sw + nc_span(r);
-  float2* sT = reinterpret_cast<float2*>(s_hi + nc_span(r));  // [kNcQ][kNcP][threads + h]
+  float4* sT = s_hi + nc_span(r);
   const int t = threadIdx.x;
   for (uint32_t tb = blockIdx.x * (uint32_t)out; tb < c; tb += gridDim.x * (uint32_t)out) {
     const int lo = (int)tb - kNcP * h;  // window position 0; may be negative
@@ -371,18 +515,24 @@ __device__ __forceinline__ void nn_tiles_consec(const PlocBufs& B, int r, uint32
       const int j = lo + k;
       if (j >= 0 && j < (int)c) {
         const float4* bp = reinterpret_cast<const float4*>(cbox + j);
-        s_lo[nc_swz(k)] = __ldcg(bp);
-        s_hi[nc_swz(k)] = __ldcg(bp + 1);
+        s_lo[nc_at(k)] = __ldcg(bp);
+        s_hi[nc_at(k)] = __ldcg(bp + 1);
       }
     }
     __syncthreads();
-    if (lo >= 0 && lo + span <= (int)c) nc_tile<SEG, false>(B, r, (int)c, lo, h, s_lo, s_hi, sT);
-    else nc_tile<SEG, true>(B, r, (int)c, lo, h, s_lo, s_hi, sT);
+    const bool inside = lo >= 0 && lo + span <= (int)c;
+    if constexpr (MIN) {
+      if (inside) nc_tile_min<SEG, false>(B, r, (int)c, lo, h, s_lo, s_hi, sT);
+      else nc_tile_min<SEG, true>(B, r, (int)c, lo, h, s_lo, s_hi, sT);
+    } else {
+      if (inside) nc_tile<SEG, false>(B, r, (int)c, lo, h, s_lo, s_hi, sT);
+      else nc_tile<SEG, true>(B, r, (int)c, lo, h, s_lo, s_hi, sT);
+    }
   }
 }
 
-template <bool SEG>
-__global__ void __launch_bounds__(kPlocThreads) k_ploc_nn(PlocBufs B, int r) {
+template <bool SEG, bool MIN>  // (MIN: r >= kNcMinR; both forms in one kernel cost each 2%)
+__global__ void __launch_bounds__(kPlocThreads, 3) k_ploc_nn(PlocBufs B, int r) {
   extern __shared__ float4 sw[];
   const uint32_t c = __ldcg(B.ctrl + 0);
   const Box* __restrict__ cbox = (__ldcg(B.ctrl + 3) & 1u) ? B.cbox[1] : B.cbox[0];  // no stack copy of B
@@ -390,7 +540,7 @@ __global__ void __launch_bounds__(kPlocThreads) k_ploc_nn(PlocBufs B, int r) {
   // one tile's latency: smaller tiles (2 or 1 clusters per thread) then spread it over more
   // blocks.  The result does not depend on the tiling.
   const uint32_t g = gridDim.x * (uint32_t)kPlocThreads;
-  if (c > 2u * g && r <= kNcMaxR) nn_tiles_consec<SEG>(B, r, c, cbox, sw);
+  if (c > 2u * g && r <= kNcMaxR) nn_tiles_consec<SEG, MIN>(B, r, c, cbox, sw);
   else if (c > 2u * g) nn_tiles<kNnPer, SEG>(B, r, c, cbox, sw);
   else if (c > g) nn_tiles<2, SEG>(B, r, c, cbox, sw);
   else nn_tiles<1, SEG>(B, r, c, cbox, sw);
@@ -778,15 +928,6 @@ __device__ __forceinline__ int search_lanes(uint32_t cnt, int r) {
   int lg = 0;
   while (lg < 5 && (cnt << (lg + 1)) <= (uint32_t)kTailThreads && (4 << lg) < 2 * r) ++lg;
   return lg;
-}
-
-// The searches of the one-launch kernels compare halves of areas: doubling is exact, so the order is the
-// same, and a half below 2^127 is an area below infinity.
-constexpr float kHalfInf = 0x1p127f;
-__device__ __forceinline__ float pair_half(float4 xa, float4 xb, float4 ja, float4 jb) {
-  const float dx = __fsub_rn(fmaxf(xb.x, jb.x), fminf(xa.x, ja.x)), dy = __fsub_rn(fmaxf(xb.y, jb.y), fminf(xa.y, ja.y)),
-              dz = __fsub_rn(fmaxf(xb.z, jb.z), fminf(xa.z, ja.z));
-  return __fmaf_rn(dz, dx, __fmaf_rn(dx, dy, __fmul_rn(dy, dz)));
 }
 
 // The nearest of the clusters j0..j1 (staged boxes) to cluster x of that range: the smallest area, the smallest
@@ -1417,7 +1558,8 @@ cudaError_t workspace_reserve_ploc(Workspace& ws, uint32_t n) {
 }
 
 static size_t nn_smem(int radius) {
-  const size_t strided = 32 * (kNnTile + 2 * (size_t)radius) + 4 * (size_t)kNnKc * kNnTile;
+  const size_t tile = radius <= kNcMaxR ? 2 * kPlocThreads : kNnTile;  // the largest strided tile that is taken
+  const size_t strided = 32 * (tile + 2 * (size_t)radius) + 4 * (size_t)kNnKc * tile;
   return radius <= kNcMaxR ? std::max(strided, nc_smem(radius)) : strided;
 }
 
@@ -1443,7 +1585,8 @@ template <bool SEG, bool GRAPH>
 static void enqueue_iteration(const PlocBufs& B, const PlocSeg& S, uint32_t n, int radius, const PlocShape& sh,
                               cudaStream_t st, cudaGraphConditionalHandle handle) {
   const uint32_t mg_grid = mg_grid_for(n, sh);
-  k_ploc_nn<SEG><<<nn_grid_for(n, sh), kPlocThreads, nn_smem(radius), st>>>(B, radius);
+  const auto nn = radius < kNcMinR ? k_ploc_nn<SEG, false> : k_ploc_nn<SEG, true>;
+  nn<<<nn_grid_for(n, sh), kPlocThreads, nn_smem(radius), st>>>(B, radius);
   k_ploc_count<<<mg_grid, kPlocThreads, 0, st>>>(B);
   if constexpr (SEG) k_ploc_seg<<<std::max<uint32_t>(1, std::min<uint32_t>(div_up(S.count, 256), 152 * 4)), 256, 0,
                                   st>>>(B, S, mg_grid);
@@ -1506,7 +1649,8 @@ static PlocBufs ploc_bufs(Workspace& ws, const ScratchLayout& L) {
 template <bool SEG>
 static cudaError_t set_nn_smem(int radius) {
   if (nn_smem(radius) <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(k_ploc_nn<SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nn_smem(radius));
+  const auto nn = radius < kNcMinR ? k_ploc_nn<SEG, false> : k_ploc_nn<SEG, true>;
+  return cudaFuncSetAttribute(nn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nn_smem(radius));
 }
 
 static cudaError_t set_tail_smem() {
