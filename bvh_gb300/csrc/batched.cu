@@ -286,8 +286,10 @@ cudaError_t batched_build(Workspace& ws, const MeshPtrs& m, uint32_t n, const ui
                         ws.vals[fb], ws.boxes, ws.nodes, n, seg, d_indices, frontier, fcount, kEmitMaxSteps,
                         reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps), nullptr)) != cudaSuccess)
     return e;
-  return launch_after(k_emit_climb<SegBatch, false>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st, ws.delta,
-                      ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount, nullptr);
+  // launched plainly, as the per-mesh kernels: with 29M triangles emission takes 1,357 us, started early 1,434
+  k_emit_climb<SegBatch, false><<<std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st>>>(
+      ws.delta, ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount, nullptr, ws.scratch + L.status);
+  return cudaGetLastError();
 }
 
 }  // namespace bvhgb

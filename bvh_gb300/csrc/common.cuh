@@ -32,7 +32,7 @@ constexpr uint32_t kLeafBit = 0x80000000u;
 // Device status word bits (set by kernels, read by the host after a build).
 enum : uint32_t {
   kStatusSortTimeout = 1u << 0,     // onesweep look-back spin gave up
-  kStatusClimbTimeout = 1u << 1,    // reserved: bounded waits in bottom-up passes
+  kStatusClimbTimeout = 1u << 1,    // a node announced by its writer did not arrive (k_emit_climb)
   kStatusNoProgress = 1u << 2,      // PLOC iteration merged nothing
   kStatusBadInput = 1u << 3,        // index outside its buffer was seen and skipped
   kStatusGridTimeout = 1u << 4,     // a grid-wide barrier of a cooperative kernel gave up

@@ -48,9 +48,12 @@ struct SegBatch {
   }
 };
 
-// In-tile climbs stop after this many levels and continue in k_emit_climb (k_emit's max_steps):
-// the longest chain of a block no longer holds its 512 threads.
+// In-tile climbs stop after this many levels and continue in k_emit_climb (k_emit's max_steps): the longest
+// chain of a block no longer holds its 512 threads.  Fewer levels leave more to k_emit_climb, which pays
+// while its chains' latency is what a build waits for (100,000 triangles: 4 levels 59.3 us, 5 59.7, 8 63.9; 1M
+// 155 / 154 / 160; 3M 5 345, 8 342; 10M 1,152 / 1,096 / 1,029).
 constexpr uint32_t kEmitMaxSteps = 8;
+inline uint32_t emit_max_steps(uint32_t n) { return n < 2000000u ? 5u : kEmitMaxSteps; }
 constexpr uint32_t kEmitTile = 512;  // sorted positions (threads) per k_emit block
 
 __device__ __forceinline__ void store_node(Node* nodes, uint32_t idx, const Box& b, int32_t l, int32_t r, int32_t aux0) {
@@ -76,9 +79,9 @@ __device__ __forceinline__ uint32_t atom_or_acq_rel_cta(uint32_t* p, uint32_t v)
   return old;
 }
 
-__device__ __forceinline__ unsigned long long atom_exch_acq_rel(unsigned long long* p, unsigned long long v) {
+__device__ __forceinline__ unsigned long long atom_exch_relaxed(unsigned long long* p, unsigned long long v) {
   unsigned long long old;
-  asm volatile("atom.acq_rel.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
+  asm volatile("atom.relaxed.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
   return old;
 }
 
@@ -118,6 +121,24 @@ struct Climb {
   uint32_t h;
   bool internal;
 };
+
+// 16 bytes read or written as one (b128 accesses are single-copy atomic).
+__device__ __forceinline__ float4 ld_relaxed16(const float4* p) {
+  unsigned long long x, y;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(x), "=l"(y)
+               : "l"(p)
+               : "memory");
+  return make_float4(__uint_as_float((uint32_t)x), __uint_as_float((uint32_t)(x >> 32)), __uint_as_float((uint32_t)y),
+                     __uint_as_float((uint32_t)(y >> 32)));
+}
+__device__ __forceinline__ void st_relaxed16(float4* p, float4 v) {
+  const unsigned long long x = (unsigned long long)__float_as_uint(v.y) << 32 | __float_as_uint(v.x),
+                           y = (unsigned long long)__float_as_uint(v.w) << 32 | __float_as_uint(v.z);
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+               "l"(x), "l"(y)
+               : "memory");
+}
 
 // PLUS: what the treelet passes read of a node besides its box -- the children's areas beside their ids
 // (one 16-byte load when a treelet grows through the node) and its height.
@@ -321,18 +342,74 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   if (nf > 1) frontier[s_base + slot_in_block + 1] = fr1;
 }
 
-// Climb from every frontier node (a finished node whose parent needs a sibling built by
-// another block) through the rendezvous words; the second child to arrive completes the parent.
+__device__ __forceinline__ void clear_padding(Node* nodes, uint32_t idx) {
+  __stcg(&nodes[idx].lo.w, 0.f);
+  __stcg(&nodes[idx].hi.w, 0.f);
+}
+constexpr uint32_t kClimbSpins = 1u << 22;  // re-reads of a node whose writer has announced it
+
+// The node c, a left child (LEFT) or a right one, and its sibling, announced by `old`, become their parent; dfar
+// becomes the delta byte past the sibling's far end.  slo, shi: the sibling's corners as read last, if it is
+// the internal node `sib`.  False where they did not arrive.  (One body per side: with selects in place of
+// branches, the loads wait for each other.)
+template <bool PLUS, bool LEFT>
+__device__ __forceinline__ bool climb_join(Climb& c, uint32_t& dfar, unsigned long long old, uint32_t sib, float4 slo,
+                                           float4 shi, uint32_t here, uint32_t g, uint32_t off, uint32_t cnt,
+                                           uint32_t nb, uint32_t n, uint32_t epoch, const uint8_t* __restrict__ D,
+                                           Node* nodes, const uint8_t* hgt) {
+  const uint32_t other = (uint32_t)old;
+  if (here) clear_padding(nodes, nb + (uint32_t)c.my);
+  if (LEFT) c.l = other;
+  else c.f = other;
+  if ((old >> 32) & 1u) {
+    const float4* sp = reinterpret_cast<const float4*>(nodes + nb + sib);
+    for (uint32_t spins = 0;
+         __float_as_uint(slo.w) != epoch || __float_as_uint(shi.w) >> 16 != ((epoch >> 6) & 0xffffu); ++spins) {
+      if (spins >= kClimbSpins) return false;
+      slo = ld_relaxed16(sp);
+      shi = ld_relaxed16(sp + 1);
+    }
+    clear_padding(nodes, nb + sib);
+    const uint32_t w = __float_as_uint(shi.w);
+    dfar = (w >> 8) & 0xffu;
+    Box sb;
+    sb.lo = make_float4(slo.x, slo.y, slo.z, 0.f);
+    sb.hi = make_float4(shi.x, shi.y, shi.z, 0.f);
+    climb_merge<PLUS>(c, LEFT, (int32_t)sib, sb, w & 0xffu);
+    return true;
+  }
+  const bool leaf = other == g + off + (LEFT ? 1u : 0u);
+  if (leaf) sib = LEFT ? cnt + g : cnt - 1 + g;
+  if (LEFT) dfar = other + 1 >= n ? 0u : __ldg(D + other);
+  else dfar = other == 0 ? 0u : __ldg(D + other - 1);
+  const uint32_t hs = PLUS && !leaf ? __ldcg(hgt + nb + sib) : 0u;
+  climb_merge<PLUS>(c, LEFT, (int32_t)sib, load_node_box(nodes, nb + sib), hs);
+  return true;
+}
+
+// Climb from every frontier node (a finished node whose parent needs a sibling built by another block)
+// through the rendezvous words; the second child to arrive completes the parent.
+//
+// What bounds it is the chain of one round trip after another, a dozen or more levels from the tiles to
+// the root.  A node is therefore its own message: while its parent is missing, the padding of its two
+// corners (each written and read as 16 bytes at once) holds the build's epoch and, beside it, the delta
+// byte past its far end and its height.  No fence orders the node's stores before its announcement: the
+// sibling, which reads the node while its own announcement is under way, sees by the epoch whether it has
+// it, and otherwise reads again.  Both paddings are 0 again once the parent is complete.  A rendezvous word is
+// (epoch | written in this kernel) << 32 | far end; a node written by k_emit (bit 0 clear) carries
+// no epoch and needs none.
+// With a fence before the exchange, and the sibling's box and delta byte read after it, emission took 43 us of
+// 100,000 triangles (30 now), 98 of 1M (77), 523 of 10M (496), 1,400 of 29M in 1,024 meshes (1,357).
 template <typename Seg, bool PLUS>
 __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ D, Node* __restrict__ nodes,
                                                     unsigned long long* __restrict__ slots,
                                                     const uint32_t* epoch_word, uint32_t n, Seg seg,
                                                     const uint2* __restrict__ frontier,
                                                     const uint32_t* __restrict__ frontier_count,
-                                                    uint8_t* __restrict__ hgt) {
+                                                    uint8_t* __restrict__ hgt, uint32_t* __restrict__ status) {
   after_previous();
   const uint32_t count = __ldcg(frontier_count);
-  const unsigned long long tag = (unsigned long long)__ldcg(epoch_word) << 32;
+  const uint32_t epoch = __ldcg(epoch_word);  // (a multiple of kEpochStride)
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
     const uint2 fl = __ldcg(frontier + e);
     Climb c;
@@ -340,41 +417,48 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
     c.l = fl.y;
     uint32_t off, cnt, nb;
     seg.get(c.f, off, cnt, nb);
-    int dl = c.f == 0 ? -1 : (int)__ldg(D + c.f - 1) - 1;
-    int dr = c.l + 1 >= n ? -1 : (int)__ldg(D + c.l) - 1;
+    // delta bytes beside the node's ends (0 at the ends of the mesh)
+    uint32_t dl = c.f == 0 ? 0u : __ldg(D + c.f - 1), dr = c.l + 1 >= n ? 0u : __ldg(D + c.l);
     bool is_left = dr > dl;
-    uint32_t gamma = is_left ? c.l : c.f - 1;
     c.my = c.f == c.l ? (int32_t)(cnt - 1 + (c.f - off)) : (int32_t)((is_left ? c.l : c.f) - off);
     c.box = load_node_box(nodes, nb + (uint32_t)c.my);
     c.h = PLUS && c.f != c.l ? __ldcg(hgt + nb + (uint32_t)c.my) : 0u;
+    uint32_t here = 0;  // 1: the node was written in this kernel
     while (true) {
-      const uint32_t far = is_left ? c.f : c.l;
-      const unsigned long long old = atom_exch_acq_rel(slots + gamma, tag | far);
-      if ((old & 0xffffffff00000000ull) != tag) break;  // first child to arrive
-      const uint32_t other = (uint32_t)old;
-      const int32_t g = (int32_t)(gamma - off);
-      int32_t sib;
-      if (is_left) {
-        sib = (other == gamma + 1) ? (int32_t)cnt + g : g + 1;
-        const uint32_t hs = PLUS && other != gamma + 1 ? __ldcg(hgt + nb + (uint32_t)sib) : 0u;
-        c.l = other;
-        climb_merge<PLUS>(c, true, sib, load_node_box(nodes, nb + (uint32_t)sib), hs);
-      } else {
-        sib = (other == gamma) ? (int32_t)cnt - 1 + g : g;
-        const uint32_t hs = PLUS && other != gamma ? __ldcg(hgt + nb + (uint32_t)sib) : 0u;
-        c.f = other;
-        climb_merge<PLUS>(c, false, sib, load_node_box(nodes, nb + (uint32_t)sib), hs);
+      const uint32_t gamma = is_left ? c.l : c.f - 1, g = gamma - off;
+      // the sibling, if it is an internal node: a right child is named by its first position, a left by its last
+      uint32_t sib = is_left ? g + 1 : g;
+      const float4* sp = reinterpret_cast<const float4*>(nodes + nb + sib);
+      float4 slo = make_float4(0.f, 0.f, 0.f, 0.f), shi = slo;
+      if (here) {
+        slo = ld_relaxed16(sp);
+        shi = ld_relaxed16(sp + 1);
       }
-      dl = c.f == 0 ? -1 : (int)__ldg(D + c.f - 1) - 1;
-      dr = c.l + 1 >= n ? -1 : (int)__ldg(D + c.l) - 1;
-      if (dl < 0 && dr < 0) {
+      const unsigned long long old =
+          atom_exch_relaxed(slots + gamma, (unsigned long long)(epoch | here) << 32 | (is_left ? c.f : c.l));
+      if ((uint32_t)(old >> 33) != epoch >> 1) break;  // first child to arrive
+      const bool ok =
+          is_left ? climb_join<PLUS, true>(c, dr, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, D, nodes, hgt)
+                  : climb_join<PLUS, false>(c, dl, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, D, nodes, hgt);
+      if (!ok) {
+        atomicOr(status, kStatusClimbTimeout);
+        break;
+      }
+      if (dl == 0 && dr == 0) {
         write_internal<PLUS>(nodes, hgt, nb, 0, c);
         break;
       }
       is_left = dr > dl;
-      gamma = is_left ? c.l : c.f - 1;
       c.my = (int32_t)((is_left ? c.l : c.f) - off);
-      write_internal<PLUS>(nodes, hgt, nb, c.my, c);
+      here = 1;
+      // (each corner, with its padding, may be read while it is written)
+      float4* np = reinterpret_cast<float4*>(nodes + nb + (uint32_t)c.my);
+      st_relaxed16(np, make_float4(c.box.lo.x, c.box.lo.y, c.box.lo.z, __uint_as_float(epoch)));
+      st_relaxed16(np + 1, make_float4(c.box.hi.x, c.box.hi.y, c.box.hi.z,
+                                       __uint_as_float((epoch >> 6) << 16 | (is_left ? dl : dr) << 8 | min(c.h, 255u))));
+      __stcg(reinterpret_cast<int4*>(np + 2), PLUS ? make_int4(c.lc, c.rc, __float_as_int(c.al), __float_as_int(c.ar))
+                                                   : make_int4(c.lc, c.rc, -1, 0));
+      if (PLUS) __stcg(hgt + nb + (uint32_t)c.my, (uint8_t)min(c.h, 255u));
     }
   }
 }

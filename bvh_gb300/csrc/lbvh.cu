@@ -781,11 +781,11 @@ static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchL
   unsigned long long* stamps = reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps);
   cudaError_t e = launch_after(k_emit<SegSingle, PLUS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
                                ws.delta, keys, ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier,
-                               fcount, kEmitMaxSteps, stamps, ws.heights);
+                               fcount, emit_max_steps(n), stamps, ws.heights);
   if (e != cudaSuccess) return e;
   if (ws.leaves_ready && !PLUS) cudaEventRecord(ws.leaves_ready, st);
   return launch_after(k_emit_climb<SegSingle, PLUS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
-                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount, ws.heights);
+                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount, ws.heights, ws.scratch + L.status);
 }
 
 bool one_block_build(uint32_t n) { return n <= kSmallMax; }

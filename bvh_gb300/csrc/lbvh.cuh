@@ -26,7 +26,7 @@ struct Workspace {
   uint32_t* vals[2] = {nullptr, nullptr};
   Box* boxes = nullptr;      // per-triangle AABB in input order
   Node* nodes = nullptr;     // 2n-1 output nodes
-  unsigned long long* slots = nullptr;  // n-1 rendezvous words (epoch << 32 | endpoint)
+  unsigned long long* slots = nullptr;  // n-1 rendezvous words (epoch | flag) << 32 | endpoint
   uint32_t* scratch = nullptr;          // histograms, look-back descriptors, counters
   uint8_t* delta = nullptr;             // n-1 adjacent common-prefix lengths (+1)
   uint8_t* heights = nullptr;           // LBVH+: n-1 inner nodes' heights (at most 255)
