@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(256) k_seg_bounds(MeshPtrs m, int vec4, const 
 // Keys mesh << 30 | code30 are written split: hkeys = key >> shift0 (the passes sort these 32
 // bits) and, when shift0 > 0, lows = the rest, in input order.
 // Bound by memory, 36 bytes read and 40 written a triangle: with four triangles per thread (float4 loads, one
-// 16-byte store of keys and of low bits) 29M triangles take 442 us (5.0 TB/s), one per thread took 647.
+// 16-byte store of keys and of low bits, boxes 32 bytes at a time) 29M triangles take 370 us (6.0 TB/s), one per
+// thread took 647.
 __global__ void __launch_bounds__(256) k_seg_morton(MeshPtrs m, int vec4, const SegItem* __restrict__ items, uint32_t n_items,
                                                     const float* __restrict__ mbox, int passes, int shift0,
                                                     uint32_t* __restrict__ hkeys, uint32_t* __restrict__ lows,
@@ -180,7 +181,6 @@ __global__ void __launch_bounds__(256) k_seg_morton(MeshPtrs m, int vec4, const 
 #pragma unroll
       for (int k = 0; k < 9; ++k) a[k] = __ldcs(reinterpret_cast<const float4*>(m.v[k]) + q);
       uint32_t hk[4], lw[4];
-      float4* bp = reinterpret_cast<float4*>(boxes + 4 * (size_t)q);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         float x[9];
@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(256) k_seg_morton(MeshPtrs m, int vec4, const 
         const unsigned long long key = code(x, box);
         hk[e] = (uint32_t)(key >> shift0);
         lw[e] = (uint32_t)key & low_mask;
-        bp[2 * e] = box.lo;
-        bp[2 * e + 1] = box.hi;
+        st_box(boxes + 4 * (size_t)q + e, box);
       }
       reinterpret_cast<uint4*>(hkeys)[q] = make_uint4(hk[0], hk[1], hk[2], hk[3]);
       if (shift0) reinterpret_cast<uint4*>(lows)[q] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
@@ -205,9 +204,7 @@ __global__ void __launch_bounds__(256) k_seg_morton(MeshPtrs m, int vec4, const 
       const unsigned long long key = code(x, box);
       hkeys[i] = (uint32_t)(key >> shift0);
       if (shift0) lows[i] = (uint32_t)key & low_mask;
-      float4* bp = reinterpret_cast<float4*>(boxes + i);
-      bp[0] = box.lo;
-      bp[1] = box.hi;
+      st_box(boxes + i, box);
     }
   }
   __syncthreads();

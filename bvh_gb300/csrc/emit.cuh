@@ -228,9 +228,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     const uint32_t prim_g = __ldcg(vals + i);
     const uint32_t prim = prim_g - off;  // original index within the mesh
     if (out_idx) out_idx[i] = prim;
-    const float4* bp = reinterpret_cast<const float4*>(tri_boxes + prim_g);
-    c.box.lo = __ldg(bp);
-    c.box.hi = __ldg(bp + 1);
+    c.box = ld_box_cg(tri_boxes + prim_g);
     c.my = (int32_t)(cnt - 1) + (int32_t)(i - off);
     store_node(nodes, nb + (uint32_t)c.my, c.box, (int32_t)(prim | kLeafBit), -1, -1);
     if (cnt == 1) active = false;  // a one-triangle mesh: the leaf is the root

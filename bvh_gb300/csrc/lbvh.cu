@@ -245,11 +245,9 @@ __global__ void __launch_bounds__(256) k_morton(MeshPtrs m, uint32_t n, int vec4
       if constexpr (sizeof(K) == 8)
         reinterpret_cast<uint4*>(lows)[q] = make_uint4((uint32_t)(c[0] & kLowMask), (uint32_t)(c[1] & kLowMask),
                                                        (uint32_t)(c[2] & kLowMask), (uint32_t)(c[3] & kLowMask));
-      float4* bp = reinterpret_cast<float4*>(boxes + 4 * (size_t)q);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        bp[2 * e] = b[e].lo;
-        bp[2 * e + 1] = b[e].hi;
+        st_box(boxes + 4 * (size_t)q + e, b[e]);
         if (PLUS) wild |= !tame_box(b[e]);
 #pragma unroll
         for (int p2 = 0; p2 < P; ++p2) atomicAdd(&s_hist[p2][(uint32_t)(c[e] >> (S0 + 8 * p2)) & 255u], 1u);

@@ -80,14 +80,12 @@ __global__ void k_ploc_init(const uint32_t* __restrict__ sidx, const Box* __rest
   }
   if (i >= n) return;
   uint32_t prim = __ldg(sidx + i);
-  const float4* bp = reinterpret_cast<const float4*>(tri_boxes + prim);
-  float4 lo = __ldg(bp), hi = __ldg(bp + 1);
-  reinterpret_cast<float4*>(B.cbox[0] + i)[0] = lo;
-  reinterpret_cast<float4*>(B.cbox[0] + i)[1] = hi;
+  const Box box = ld_box_cg(tri_boxes + prim);
+  st_box(B.cbox[0] + i, box);
   B.cid[0][i] = (int32_t)i;
   float4* np = reinterpret_cast<float4*>(B.nodes + i);
-  np[0] = lo;
-  np[1] = hi;
+  np[0] = box.lo;
+  np[1] = box.hi;
   reinterpret_cast<int4*>(np + 2)[0] = make_int4((int32_t)(prim | kLeafBit), -1, 0, 0);
 }
 
@@ -136,9 +134,9 @@ __device__ __forceinline__ void nn_tiles(const PlocBufs& B, int r, uint32_t c, c
     for (int k = t; k < span; k += kPlocThreads) {
       const int j = lo + k;
       if (j >= 0 && j < (int)c) {
-        const float4* bp = reinterpret_cast<const float4*>(cbox + j);
-        s_lo[k] = __ldcg(bp);
-        s_hi[k] = __ldcg(bp + 1);
+        const Box box = ld_box_cg(cbox + j);
+        s_lo[k] = box.lo;
+        s_hi[k] = box.hi;
       }
     }
     __syncthreads();
@@ -514,9 +512,9 @@ __device__ __forceinline__ void nn_tiles_consec(const PlocBufs& B, int r, uint32
     for (int k = t; k < span; k += kPlocThreads) {
       const int j = lo + k;
       if (j >= 0 && j < (int)c) {
-        const float4* bp = reinterpret_cast<const float4*>(cbox + j);
-        s_lo[nc_at(k)] = __ldcg(bp);
-        s_hi[nc_at(k)] = __ldcg(bp + 1);
+        const Box box = ld_box_cg(cbox + j);
+        s_lo[nc_at(k)] = box.lo;
+        s_hi[nc_at(k)] = box.hi;
       }
     }
     __syncthreads();
@@ -736,15 +734,15 @@ __device__ __forceinline__ void scatter_tiles(const PlocBufs& B, uint32_t c, uin
         lo[g] = hi[g] = jlo[g] = jhi[g] = make_float4(0.f, 0.f, 0.f, 0.f);
         id[g] = jid[g] = 0;
         if (m || v) {
-          const float4* ip = reinterpret_cast<const float4*>(cin + i);
-          lo[g] = __ldcg(ip);
-          hi[g] = __ldcg(ip + 1);
+          const Box x = ld_box_cg(cin + i);
+          lo[g] = x.lo;
+          hi[g] = x.hi;
           id[g] = __ldcg(idin + i);
         }
         if (m) {
-          const float4* jp = reinterpret_cast<const float4*>(cin + nj[r]);
-          jlo[g] = __ldcg(jp);
-          jhi[g] = __ldcg(jp + 1);
+          const Box y = ld_box_cg(cin + nj[r]);
+          jlo[g] = y.lo;
+          jhi[g] = y.hi;
           jid[g] = __ldcg(idin + nj[r]);
         }
       }
@@ -782,9 +780,7 @@ __device__ __forceinline__ void scatter_tiles(const PlocBufs& B, uint32_t c, uin
         }
         if (v) {
           const uint32_t o = vpos + __popc(vb[r] & lt);
-          float4* op = reinterpret_cast<float4*>(cout + o);
-          op[0] = a;
-          op[1] = b;
+          st_box(cout + o, Box{a, b});
           idout[o] = nid;
         }
         mpos += __popc(mb[r]);
@@ -891,11 +887,10 @@ __global__ void __launch_bounds__(256) k_ploc_init_seg(const uint32_t* __restric
     if (w.begin == off && threadIdx.x == 0) S.seg[w.mesh] = off;
     for (uint32_t p = w.begin + threadIdx.x; p < w.end; p += blockDim.x) {
       const uint32_t prim = __ldg(sidx + p);
-      const float4* bp = reinterpret_cast<const float4*>(tri_boxes + prim);
-      const float4 lo = __ldg(bp), hi = __ldg(bp + 1);
-      float4* cb = reinterpret_cast<float4*>(B.cbox[0] + p);
-      cb[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float((int)w.mesh));
-      cb[1] = hi;
+      Box box = ld_box_cg(tri_boxes + prim);
+      const float4 lo = box.lo, hi = box.hi;
+      box.lo.w = __int_as_float((int)w.mesh);
+      st_box(B.cbox[0] + p, box);
       B.cid[0][p] = (int32_t)(p - off);
       float4* np = reinterpret_cast<float4*>(B.nodes + base + (p - off));
       np[0] = make_float4(lo.x, lo.y, lo.z, 0.f);
@@ -1276,9 +1271,9 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
     const uint32_t h0 = x0 > (uint32_t)r ? x0 - (uint32_t)r : 0u, h1 = min(c, x1 + (uint32_t)r);
     const uint32_t w0 = h0 > (uint32_t)r ? h0 - (uint32_t)r : 0u, w1 = min(c, h1 + (uint32_t)r);
     for (uint32_t x = w0 + tid; x < w1; x += kGridThreads) {
-      const float4* bp = reinterpret_cast<const float4*>(cin + x);
-      s_lo[x - w0] = __ldcg(bp);
-      s_hi[x - w0] = __ldcg(bp + 1);
+      const Box box = ld_box_cg(cin + x);
+      s_lo[x - w0] = box.lo;
+      s_hi[x - w0] = box.hi;
       s_id[x - w0] = __ldcg(idin + x);
     }
     __syncthreads();
@@ -1378,9 +1373,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_ploc_grid(PlocBufs B, int r
         ++mpos;
       }
       if (v2[q]) {
-        float4* op = reinterpret_cast<float4*>(cout + vpos);
-        op[0] = a;
-        op[1] = bb;
+        st_box(cout + vpos, Box{a, bb});
         idout[vpos] = nid;
         ++vpos;
       }
