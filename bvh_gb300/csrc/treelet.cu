@@ -758,6 +758,16 @@ __global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(TlArgs A, const uin
   }
 }
 
+// A box through L1, whose line serves the second half: for kernels that write no box that they read (the treelets
+// of a height are disjoint).
+__device__ __forceinline__ Box ldca_box(const Node* nodes, int32_t idx) {
+  const float4* p = reinterpret_cast<const float4*>(nodes + idx);
+  Box b;
+  b.lo = __ldca(p);
+  b.hi = __ldca(p + 1);
+  return b;
+}
+
 // One lane's treelet q of the current height (act: a real one): leaf ids and boxes from its
 // descriptor and the nodes, subset areas and the DP in this lane's shared-memory column C
 // (stride 32), then the rebuild.  The warp runs the DP variant of its largest treelet, at most
@@ -770,7 +780,7 @@ __device__ __forceinline__ void lane_dp(const TlArgs& A, bool wild, uint32_t q, 
 #pragma unroll
   for (int i = 0; i < kTlMax; ++i) {
     T.id[i] = i < NVMAX && i < T.n ? (int32_t)__ldcg(A.desc + (size_t)(1 + i) * A.stride + q) : 0;
-    T.b[i] = i < NVMAX && i < T.n ? ldcg_box(A.nodes, T.id[i]) : box_empty();
+    T.b[i] = i < NVMAX && i < T.n ? ldca_box(A.nodes, T.id[i]) : box_empty();
   }
   const int nv = (int)__reduce_max_sync(0xffffffffu, (uint32_t)T.n);
   if (nv < 2) return;
@@ -1097,6 +1107,11 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   if (!g_dp_grid[dev]) {
     int per_sm = 0;
+    // Seven blocks of shared memory per SM in place of eight leave L1 the lines that the boxes' loads need while
+    // in flight: one pass over 10M 2,888 us with the default (72% of the memory shared), 2,822 with 58%, 2,716
+    // with the boxes read through L1; twelve blocks in fewer registers took 3,350, all memory shared 3,339.
+    if ((e = cudaFuncSetAttribute(k_tl_dp<kTlMax>, cudaFuncAttributePreferredSharedMemoryCarveout, 58)) != cudaSuccess)
+      return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tl_dp<kTlMax>, kLvThreads, 0)) != cudaSuccess)
       return e;
     g_dp_grid[dev] = std::max(1, per_sm * sms);
