@@ -316,7 +316,7 @@ extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {
   } else if (ctx->last_algo == BVH_ALGO_LBVH_PLUS) {
     ctx->last.tree_height = (int32_t)ctx->h_status[5];
     // LBVH kernels, then per treelet pass: counts, offsets, grouping, the fallback's links and check;
-    // heights 1 (growth, from the second pass on), 2 (growth, DP) and 3 (growth, four DPs by size
+    // heights 1 (growth, from the second pass on), 2 (growth, DP) and 3 (growth, one DP or four by size
     // class); then growth + DP + step per height of the loop (the graph runs at least
     // one), and k_tl_narrow for the rest (the last pass's heights stand for every pass)
     const uint32_t* c = ctx->h_status + 4;  // [0] too high, [1] largest height, [2] first height left
@@ -326,7 +326,7 @@ extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {
     // the LBVH (one kernel for a small mesh) and the final report
     const int32_t lbvh = one_block_build(ctx->last_n) ? 1 + 1 : 2 + 4 + (ctx->last_bits != 30 ? 2 : 0) + 2 + 1;
     ctx->last.kernel_launches =
-        ctx->last_n > 1 ? lbvh - 1 + ctx->last_rounds * (5 + 8 + 3 * loop_h + (ctx->ws.tl_narrow ? 1 : 0)) : lbvh;
+        ctx->last_n > 1 ? lbvh - 1 + ctx->last_rounds * (5 + 4 + ctx->ws.tl_dp3 + 3 * loop_h + (ctx->ws.tl_narrow ? 1 : 0)) : lbvh;
   }
   return check_status_word(ctx);
 }

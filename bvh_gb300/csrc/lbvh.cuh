@@ -46,6 +46,7 @@ struct Workspace {
   const void* tl_key_desc = nullptr;
   const void* tl_key_ctl = nullptr;
   bool tl_narrow = false;               // the last treelet pass launched k_tl_narrow
+  int tl_dp3 = 0;                       // its launches of the DP at height 3
   bool no_cooperative = false;          // run no cooperative kernel (their host-driven fallbacks)
   uint32_t ploc_key_n = 0;
   int ploc_key_r = 0;
@@ -145,6 +146,13 @@ inline cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t bl
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_plain(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
+                                A... args) {
+  kernel<<<grid, block, smem, st>>>(static_cast<P>(args)...);
+  return cudaGetLastError();
 }
 
 // The end of a build: writes its status word, `words` control words from scratch + first and the stage

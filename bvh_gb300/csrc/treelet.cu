@@ -633,6 +633,7 @@ __device__ __forceinline__ void reg_build(Node* nodes, uint8_t* hgt, int32_t fir
 // A height past kTlMaxHeight hands this pass and the following ones to the fallback (flags[0]).
 __global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hgt, uint32_t m, uint32_t* __restrict__ cnt,
                                                   uint32_t* __restrict__ flags) {
+  after_previous();
   __shared__ uint32_t s_cnt[256];
   s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -650,6 +651,7 @@ __global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hg
 __global__ void __launch_bounds__(256) k_tl_offsets(const uint32_t* __restrict__ cnt, uint32_t m,
                                                     uint32_t* __restrict__ off, uint32_t* __restrict__ cursor,
                                                     uint32_t* __restrict__ flags) {
+  after_previous();
   __shared__ uint32_t s_w[8];
   __shared__ uint32_t s_maxh;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -682,6 +684,7 @@ __global__ void __launch_bounds__(256) k_tl_offsets(const uint32_t* __restrict__
 // Internal node ids grouped by height (order within a height is irrelevant).
 __global__ void __launch_bounds__(256) k_tl_scatter(const uint8_t* __restrict__ hgt, uint32_t m,
                                                     uint32_t* __restrict__ cursor, uint32_t* __restrict__ list) {
+  after_previous();
   __shared__ uint32_t s_cnt[256], s_base[256];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   s_cnt[threadIdx.x] = 0;
@@ -718,6 +721,7 @@ struct TlArgs {
 
 __global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(TlArgs A, const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ ctl, uint32_t at) {
+  after_previous();
   if (__ldcg(ctl) != 0u) return;  // too high: the fallback pass does the work
   const uint32_t h = at ? at : __ldcg(ctl + 2);
   const uint32_t b = __ldcg(A.off + h), e = __ldcg(A.off + h + 1);
@@ -805,6 +809,7 @@ __device__ __forceinline__ void lane_dp(const TlArgs& A, bool wild, uint32_t q, 
 // holds at most 4), compiled for fewer registers, so more warps share an SM.
 template <int NVMAX>
 __global__ void __launch_bounds__(kLvThreads) k_tl_dp(TlArgs A, const uint32_t* __restrict__ ctl, uint32_t at) {
+  after_previous();
   __shared__ float s_cost[(1 << NVMAX) * 32];  // per-lane columns of 2^NVMAX areas, then costs
   if (__ldcg(ctl) != 0u) return;
   const uint32_t h = at ? at : __ldcg(ctl + 2);
@@ -825,6 +830,7 @@ __global__ void __launch_bounds__(kLvThreads) k_tl_dp(TlArgs A, const uint32_t* 
 // at a time; R shrinks with the height's node count so that every block gets a chunk.
 template <int NV>
 __global__ void __launch_bounds__(kLvThreads) k_tl_dpc(TlArgs A, const uint32_t* __restrict__ ctl, uint32_t at) {
+  after_previous();
   constexpr int R = 8;
   __shared__ float s_cost[(1 << NV) * 32];
   __shared__ uint32_t s_list[32 * R];
@@ -991,6 +997,7 @@ __global__ void k_tl_step(uint32_t* __restrict__ ctl, const uint32_t* __restrict
 // Parent links for the fallback; returns at once unless flags[0] is set.
 __global__ void __launch_bounds__(256) k_tl_parents(const Node* __restrict__ nodes, uint32_t m,
                                                     int32_t* __restrict__ parents, const uint32_t* __restrict__ flags) {
+  after_previous();
   if (__ldcg(flags) == 0u) return;
   for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) {
     const int2 ch = ldcg_children(nodes, (int32_t)x);
@@ -1006,6 +1013,7 @@ __global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ node
                                                          unsigned long long* __restrict__ slots,
                                                          const uint32_t* epoch_word, uint32_t round, uint32_t n,
                                                          const uint32_t* __restrict__ flags) {
+  after_previous();
   __shared__ LaneTreelet S[64];
   __shared__ float s_cost[2][1 << kTlMax], s_area[2][1 << kTlMax];
   if (__ldcg(flags) == 0u) return;
@@ -1178,26 +1186,46 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
     ws.tl_key_ctl = ctl;
   }
   ws.tl_narrow = narrow != 0;
-  if ((e = cudaMemsetAsync(ctl, 0, 4, st)) != cudaSuccess) return e;
   for (int r = 0; r < rounds && r + 1 < 0x20; ++r) {
     A.hgt = kept(r);
-    if ((e = cudaMemsetAsync(cnt, 0, 256 * 4, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(ctl + 1, 0, 7 * 4, st)) != cudaSuccess) return e;  // [4]: k_tl_narrow's barrier
+    if (r == 0) {  // the counts, the offsets and the control words ([0] stays for all passes)
+      if ((e = cudaMemsetAsync(cnt, 0, (kTlCtlWord + 8) * 4, st)) != cudaSuccess) return e;
+    } else {
+      if ((e = cudaMemsetAsync(cnt, 0, 256 * 4, st)) != cudaSuccess) return e;
+      if ((e = cudaMemsetAsync(ctl + 1, 0, 7 * 4, st)) != cudaSuccess) return e;  // [4]: k_tl_narrow's barrier
+    }
     k_tl_count<<<std::max<uint32_t>(1, std::min<uint32_t>(div_up(n - 1, 256), sms * 8)), 256, 0, st>>>(ws.heights, n - 1,
                                                                                                       cnt, ctl);
-    k_tl_offsets<<<1, 256, 0, st>>>(cnt, n - 1, off, cursor, ctl);
-    k_tl_scatter<<<div_up(n - 1, 256), 256, 0, st>>>(ws.heights, n - 1, cursor, list);
+    const uint32_t* clist = list;
+    const uint32_t* cctl = ctl;
+    // early starts save each launch's latency; the grids of large builds take room that the one before still
+    // has use for (one pass: 200,000 triangles 411 us against 427, 1M 747 / 770, 10M 3,817 / 3,806)
+    const auto launch = [&](auto kernel, uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, auto... args) {
+      return n < 2000000u ? launch_after(kernel, grid, block, smem, s, args...)
+                          : launch_plain(kernel, grid, block, smem, s, args...);
+    };
+    e = launch(k_tl_offsets, 1, 256, 0, st, cnt, n - 1, off, cursor, ctl);
+    if (e == cudaSuccess) e = launch(k_tl_scatter, div_up(n - 1, 256), 256, 0, st, ws.heights, n - 1, cursor, list);
     // heights 1 to 3 first: every height-1 treelet has two leaves and is finished by the growth
     // kernel (in the first pass by the emission); height 2 holds at most 4 leaves and takes the smaller
-    // DP; height 3 mixes treelet sizes (mostly 4 and 5 leaves, few 7) and runs one DP per size class
-    if (r > 0) k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 1u);
-    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 2u);
-    k_tl_dp<4><<<g_dp4_grid[dev], kLvThreads, 0, st>>>(A, ctl, 2u);
-    k_tl_grow<<<grow_grid, kGrowThreads, 0, st>>>(A, list, ctl, 3u);
-    k_tl_dpc<4><<<g_dpc_grid[dev][0], kLvThreads, 0, st>>>(A, ctl, 3u);
-    k_tl_dpc<5><<<g_dpc_grid[dev][1], kLvThreads, 0, st>>>(A, ctl, 3u);
-    k_tl_dpc<6><<<g_dpc_grid[dev][2], kLvThreads, 0, st>>>(A, ctl, 3u);
-    k_tl_dpc<7><<<g_dpc_grid[dev][3], kLvThreads, 0, st>>>(A, ctl, 3u);
+    // DP; height 3 mixes treelet sizes (mostly 4 and 5 leaves, few 7) and runs one DP per size class, where
+    // there are more of them than one round of the general DP's blocks holds (200,000 triangles: four
+    // launches 47 us, one of the general DP 19)
+    if (e == cudaSuccess && r > 0) e = launch(k_tl_grow, grow_grid, kGrowThreads, 0, st, A, clist, cctl, 1u);
+    if (e == cudaSuccess) e = launch(k_tl_grow, grow_grid, kGrowThreads, 0, st, A, clist, cctl, 2u);
+    if (e == cudaSuccess) e = launch(k_tl_dp<4>, g_dp4_grid[dev], kLvThreads, 0, st, A, cctl, 2u);
+    if (e == cudaSuccess) e = launch(k_tl_grow, grow_grid, kGrowThreads, 0, st, A, clist, cctl, 3u);
+    if (e != cudaSuccess) return e;
+    ws.tl_dp3 = n / 8 <= (uint32_t)g_dp_grid[dev] * kLvThreads ? 1 : 4;
+    if (ws.tl_dp3 == 1) {
+      e = launch(k_tl_dp<kTlMax>, g_dp_grid[dev], kLvThreads, 0, st, A, cctl, 3u);
+    } else {
+      e = launch(k_tl_dpc<4>, g_dpc_grid[dev][0], kLvThreads, 0, st, A, cctl, 3u);
+      if (e == cudaSuccess) e = launch(k_tl_dpc<5>, g_dpc_grid[dev][1], kLvThreads, 0, st, A, cctl, 3u);
+      if (e == cudaSuccess) e = launch(k_tl_dpc<6>, g_dpc_grid[dev][2], kLvThreads, 0, st, A, cctl, 3u);
+      if (e == cudaSuccess) e = launch(k_tl_dpc<7>, g_dpc_grid[dev][3], kLvThreads, 0, st, A, cctl, 3u);
+    }
+    if (e != cudaSuccess) return e;
     if (host_loop) {
       // read the largest height (and the too-high flag) once, then one grow + dp per height
       if ((e = cudaMemcpyAsync(ws.ploc_host, ctl, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
@@ -1244,8 +1272,10 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
         }
       }
     }
-    k_tl_parents<<<sms * 8, 256, 0, st>>>(ws.nodes, n - 1, parents, ctl);
-    k_treelet_fallback<<<sms * 8, 64, 0, st>>>(ws.nodes, parents, ws.slots, epoch, (uint32_t)r, n, ctl);
+    e = launch(k_tl_parents, sms * 8, 256, 0, st, ws.nodes, n - 1, parents, cctl);
+    if (e == cudaSuccess)
+      e = launch(k_treelet_fallback, sms * 8, 64, 0, st, ws.nodes, parents, ws.slots, epoch, (uint32_t)r, n, cctl);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
