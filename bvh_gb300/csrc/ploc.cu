@@ -60,6 +60,7 @@ struct PlocSeg {
 __global__ void k_ploc_init(const uint32_t* __restrict__ sidx, const Box* __restrict__ tri_boxes, PlocBufs B, uint32_t n,
                             uint32_t cap, uint32_t tail, uint32_t grid_at,
                             unsigned long long* __restrict__ stamps) {
+  after_previous();
   stage_stamp(stamps, 3);
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
@@ -995,6 +996,7 @@ uint32_t ploc_tail_threshold(int radius, uint32_t pairs) {
 static size_t tail_smem() { return (size_t)kTailMax * (4 * 16 + 3 * 4) + 2 * 32 * 4; }
 
 __global__ void __launch_bounds__(kTailThreads, 1) k_ploc_tail(PlocBufs B, int r) {
+  after_previous();
   extern __shared__ float4 tsm[];
   float4* s_lo[2] = {tsm, tsm + 2 * kTailMax};
   float4* s_hi[2] = {tsm + kTailMax, tsm + 3 * kTailMax};
@@ -1447,6 +1449,7 @@ cudaError_t grid_wait_selftest(uint32_t limit, uint32_t* status_out) {
 // node 0 (a leaf) has one, recorded by the merge that made it (ctrl[13]), so three nodes change:
 // 0, R and that parent.  Without a recorded parent every node is checked (one block).
 __global__ void k_ploc_root(Node* __restrict__ nodes, uint32_t total, const uint32_t* __restrict__ ctrl) {
+  after_previous();
   if (__ldcg(ctrl + 0) != 1 || total < 2) return;
   const uint32_t R = total - 1;
   auto fix = [&](int32_t c) -> int32_t {
@@ -1714,8 +1717,9 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
   uint32_t* sidx = nullptr;
   if ((e = prefix_sort30(ws, m, n, st, &sidx)) != cudaSuccess) return e;
   *out_indices = sidx;
-  k_ploc_init<<<div_up(n, 256), 256, 0, st>>>(sidx, ws.boxes, B, n, cap, tail, grid_at,
-                                              reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps));
+  if ((e = launch_after(k_ploc_init, div_up(n, 256), 256, 0, st, sidx, ws.boxes, B, n, cap, tail, grid_at,
+                        reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps))) != cudaSuccess)
+    return e;
   if (evs && evs->use) {
     cudaEventRecord(evs->ev[4], st);
     evs->split = true;
@@ -1766,8 +1770,8 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
         return e;
       }
     }
-    if (tail) k_ploc_tail<<<1, kTailThreads, tail_smem(), st>>>(B, radius);
-    k_ploc_root<<<1, 256, 0, st>>>(ws.nodes, 2 * n - 1, B.ctrl);
+    if (tail && (e = launch_after(k_ploc_tail, 1, kTailThreads, tail_smem(), st, B, radius)) != cudaSuccess) return e;
+    if ((e = launch_after(k_ploc_root, 1, 256, 0, st, ws.nodes, 2 * n - 1, B.ctrl)) != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
