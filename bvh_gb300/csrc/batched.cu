@@ -256,7 +256,7 @@ cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_
       (e = sort_fix_runs_split(hkeys, ws.vals[fb], lows, n, shift0,
                                reinterpret_cast<unsigned long long*>(ws.keys[fb ^ 1]), run_scratch, ws.vals[fb ^ 1],
                                reinterpret_cast<uint32_t*>(ws.delta), ws.scratch + L.counters + kLongRunCounter,
-                               nullptr, st)) != cudaSuccess)
+                               nullptr, st, ws.alone)) != cudaSuccess)
     return e;
   out->fb = fb;
   out->shift0 = shift0;
@@ -273,13 +273,13 @@ cudaError_t batched_build(Workspace& ws, const MeshPtrs& m, uint32_t n, const ui
   ScratchLayout L = scratch_layout(ws.cap_n);
   const int fb = bs.fb;
   const uint32_t* hkeys = reinterpret_cast<const uint32_t*>(ws.keys[fb]);
-  if ((e = launch_after(k_delta_seg_split, div_up(n, 256), 256, 0, st, hkeys, ws.vals[fb], bs.lows, d_offsets, bs.shift0,
+  if ((e = launch_after(ws.alone, k_delta_seg_split, div_up(n, 256), 256, 0, st, hkeys, ws.vals[fb], bs.lows, d_offsets, bs.shift0,
                         ws.delta, n)) != cudaSuccess)
     return e;
   uint32_t* fcount = ws.scratch + L.counters + kFrontierCounter;
   uint2* frontier = reinterpret_cast<uint2*>(ws.keys[fb ^ 1]);  // the sort's other key buffer
   const SegBatch seg{hkeys, d_offsets, 30 - bs.shift0};
-  if ((e = launch_after(k_emit<SegBatch, false, kEmitTile>, div_up(n, kEmitTile), kEmitTile, 0, st, ws.delta, nullptr,
+  if ((e = launch_after(ws.alone, k_emit<SegBatch, false, kEmitTile>, div_up(n, kEmitTile), kEmitTile, 0, st, ws.delta, nullptr,
                         ws.vals[fb], ws.boxes, ws.nodes, n, seg, d_indices, frontier, fcount, kEmitMaxSteps,
                         reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps), nullptr)) != cudaSuccess)
     return e;

@@ -357,13 +357,13 @@ __global__ void __launch_bounds__(kFixThreads) k_fixrun_split_long(const uint32_
 
 cudaError_t sort_fix_runs_split(const uint32_t* hkeys, uint32_t* vals, const uint32_t* lows, uint32_t n, int lbits,
                                 unsigned long long* scratch_a, unsigned long long* scratch_b, uint32_t* tvals,
-                                uint32_t* long_list, uint32_t* long_count, uint8_t* D, cudaStream_t st) {
+                                uint32_t* long_list, uint32_t* long_count, uint8_t* D, cudaStream_t st, bool early) {
   if (n < 2) return cudaSuccess;
   const uint32_t grid = div_up(div_up(n, 4u), 256u);
-  cudaError_t e = launch_after(D ? k_fixrun_split_short<true> : k_fixrun_split_short<false>, grid, 256, 0, st, hkeys, vals,
+  cudaError_t e = launch_after(early, D ? k_fixrun_split_short<true> : k_fixrun_split_short<false>, grid, 256, 0, st, hkeys, vals,
                                lows, n, lbits, D, long_list, long_count);
   if (e != cudaSuccess) return e;
-  return launch_after(D ? k_fixrun_split_long<true> : k_fixrun_split_long<false>, 152, kFixThreads, 0, st, hkeys, vals,
+  return launch_after(early, D ? k_fixrun_split_long<true> : k_fixrun_split_long<false>, 152, kFixThreads, 0, st, hkeys, vals,
                       lows, n, lbits, scratch_a, scratch_b, tvals, D, long_list, long_count);
 }
 

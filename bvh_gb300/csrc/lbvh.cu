@@ -519,7 +519,7 @@ static cudaError_t run_sort(Workspace& ws, uint32_t n, int passes, cudaStream_t 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ws.alone ? 1 : 0;
     cudaError_t e = cudaLaunchKernelExC(&cfg, sv.fn, args);
     if (e != cudaSuccess) return e;
     cur ^= 1;
@@ -639,7 +639,7 @@ __global__ void k_finish(const uint32_t* __restrict__ scratch, size_t status, si
 cudaError_t finish_build(const Workspace& ws, size_t first, int words, cudaStream_t st) {
   if (ws.reported) return cudaSuccess;
   const ScratchLayout L = scratch_layout(ws.cap_n);
-  return launch_after(k_finish, 1, 32, 0, st, ws.scratch, L.status, first, words, L.stamps, ws.report);
+  return launch_after(ws.alone, k_finish, 1, 32, 0, st, ws.scratch, L.status, first, words, L.stamps, ws.report);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -742,7 +742,7 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(div_up(work, 256), 152 * 8));
   // (the bounds partials and the last block's arrival count grow with the grid: no idle blocks)
   k_bounds<<<std::min<uint32_t>(grid, kBoundsBlocks), 256, 0, st>>>(m, n, vec4, ws.scratch, Lz);
-  if ((et = launch_after(plus ? k_morton<BITS, K, true> : k_morton<BITS, K, false>, grid, 256, 0, st, m, n, vec4, reinterpret_cast<uint32_t*>(ws.keys[0]), lows,
+  if ((et = launch_after(ws.alone, plus ? k_morton<BITS, K, true> : k_morton<BITS, K, false>, grid, 256, 0, st, m, n, vec4, reinterpret_cast<uint32_t*>(ws.keys[0]), lows,
                          ws.boxes, ws.scratch, L)) != cudaSuccess)
     return et;
   // 4 passes sort the 32-bit keys: the whole 30-bit code, or the high 32 bits of a 60/63-bit
@@ -754,7 +754,7 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
     e = sort_fix_runs_split(reinterpret_cast<const uint32_t*>(ws.keys[fb]), ws.vals[fb], lows, n, BITS - 32,
                             reinterpret_cast<unsigned long long*>(ws.keys[fb ^ 1]), split_run_scratch(ws, n),
                             ws.vals[fb ^ 1], split_long_list(ws, n), ws.scratch + L.counters + kLongRunCounter,
-                            ws.delta, st);
+                            ws.delta, st, ws.alone);
   }
   if (e == cudaSuccess && ws.indices_ready) e = cudaEventRecord(ws.indices_ready, st);
   return e;
@@ -777,12 +777,12 @@ static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchL
   uint2* frontier = reinterpret_cast<uint2*>(ws.keys[fb ^ 1]);  // the sort's other key buffer, 8 B per position
   // delta bytes: computed by k_emit from the 30-bit keys, written by the run fix-up for 60/63 bits
   unsigned long long* stamps = reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps);
-  cudaError_t e = launch_after(k_emit<SegSingle, PLUS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
+  cudaError_t e = launch_after(ws.alone, k_emit<SegSingle, PLUS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
                                ws.delta, keys, ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier,
                                fcount, emit_max_steps(n), stamps, ws.heights);
   if (e != cudaSuccess) return e;
   if (ws.leaves_ready && !PLUS) cudaEventRecord(ws.leaves_ready, st);
-  return launch_after(k_emit_climb<SegSingle, PLUS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
+  return launch_after(ws.alone, k_emit_climb<SegSingle, PLUS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
                       ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount, ws.heights, ws.scratch + L.status);
 }
 
@@ -801,7 +801,7 @@ cudaError_t lbvh_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int bits, i
   rec(evs, 0, st);
   int fb = 0;
   const bool plus = treelet_rounds > 0 && n >= 2;
-  if (n <= kSmallMax) {
+  if (n <= kSmallMax && ws.alone) {
     e = small_build(ws, m, n, bits, plus ? kSmallLbvhPlus : kSmallLbvh, st, L, plus ? nullptr : ws.report);
     ws.reported = e == cudaSuccess && ws.report && !plus;
   } else if (bits == 30) {

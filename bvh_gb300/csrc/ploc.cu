@@ -1717,7 +1717,7 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
   uint32_t* sidx = nullptr;
   if ((e = prefix_sort30(ws, m, n, st, &sidx)) != cudaSuccess) return e;
   *out_indices = sidx;
-  if ((e = launch_after(k_ploc_init, div_up(n, 256), 256, 0, st, sidx, ws.boxes, B, n, cap, tail, grid_at,
+  if ((e = launch_after(ws.alone, k_ploc_init, div_up(n, 256), 256, 0, st, sidx, ws.boxes, B, n, cap, tail, grid_at,
                         reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps))) != cudaSuccess)
     return e;
   if (evs && evs->use) {
@@ -1770,8 +1770,8 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
         return e;
       }
     }
-    if (tail && (e = launch_after(k_ploc_tail, 1, kTailThreads, tail_smem(), st, B, radius)) != cudaSuccess) return e;
-    if ((e = launch_after(k_ploc_root, 1, 256, 0, st, ws.nodes, 2 * n - 1, B.ctrl)) != cudaSuccess) return e;
+    if (tail && (e = launch_after(ws.alone, k_ploc_tail, 1, kTailThreads, tail_smem(), st, B, radius)) != cudaSuccess) return e;
+    if ((e = launch_after(ws.alone, k_ploc_root, 1, 256, 0, st, ws.nodes, 2 * n - 1, B.ctrl)) != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }

@@ -53,7 +53,7 @@ struct Pending {
 uint64_t ws_bytes(uint64_t cap) {
   if (!cap) return 0;
   cap = std::max<uint64_t>(cap, 1024);
-  return cap * (8 * 2 + 4 * 2 + sizeof(Box) + 2 * sizeof(Node) + 8 + 1) + 16 + scratch_layout((uint32_t)cap).total * 4;
+  return cap * (8 * 2 + 4 * 2 + sizeof(Box) + 2 * sizeof(Node) + 8 + 1 + 1) + 32 + scratch_layout((uint32_t)cap).total * 4;
 }
 
 struct Slot {
@@ -230,6 +230,7 @@ static cudaError_t launch_one(bvh_server* sv, Slot& s) {
   }
   uint32_t* idx = nullptr;
   s.ws.sort_variant = default_sort_variant(n);
+  s.ws.alone = false;
   if ((e = lbvh_build(s.ws, m, n, sv->cfg.morton_bits, 0, s.stream, nullptr, &idx)) != cudaSuccess) return e;
   float* ht = reinterpret_cast<float*>(s.hits);
   int32_t* hi = reinterpret_cast<int32_t*>(s.hits);
@@ -348,6 +349,7 @@ static cudaError_t launch_batch(bvh_server* sv, Slot& s) {
   for (int k = 0; k < 9; ++k) mp.v[k] = s.mesh + s.tri_cap * k;
   StageEvents none;
   s.ws.sort_variant = default_sort_variant(n);
+  s.ws.alone = false;
   if ((e = batched_build(s.ws, mp, n, s.d_meta + ML.offsets, count,
                          reinterpret_cast<const SegItem*>(s.d_meta + ML.items), n_items, s.mbox, s.indices, s.stream,
                          &none)) != cudaSuccess)

@@ -1,7 +1,7 @@
 // treelet.cu -- LBVH+ treelet restructuring passes.
 //
 // Reference: kRefitAndOptimize(doOptimize=true) with optimizeTreeletSerial,
-// src/cuda/lbvh_plus_builder.cu:71-247 and :341-366.  One pass climbs from every leaf; the
+// src/cuda/lbvh_plus_builder.cu:71-247 and :341-366.  There one pass climbs from every leaf; the
 // second child to arrive at a node refits its box and restructures the treelet rooted there
 // (up to 7 treelet leaves, grown by expanding the largest-area internal leaf; subset DP with
 // cost = min split + area; internal node ids reused in DFS order).
@@ -10,8 +10,10 @@
 // second child arrives, so the result is independent of scheduling and equal to any
 // children-before-parent order (the oracle uses post-order).
 //
-// Every warp keeps looping while any lane still climbs.  Lanes that reached a node grow and
-// rebuild their own treelets in parallel; the subset DP of each is done by all 32 lanes.
+// The pass goes height by height (a node's height is known from the emission or from the last rebuild): growth
+// writes a descriptor per treelet, the DP kernels read it, one lane per treelet; narrow heights take one
+// warp per treelet in one cooperative launch.  Trees higher than 254 take the climb-ordered fallback, whose
+// warps keep looping while any lane still climbs and do each treelet's DP with all 32 lanes.
 #include <algorithm>
 
 #include "emit.cuh"
@@ -1201,8 +1203,7 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
     // early starts save each launch's latency; the grids of large builds take room that the one before still
     // has use for (one pass: 200,000 triangles 411 us against 427, 1M 747 / 770, 10M 3,817 / 3,806)
     const auto launch = [&](auto kernel, uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, auto... args) {
-      return n < 2000000u ? launch_after(kernel, grid, block, smem, s, args...)
-                          : launch_plain(kernel, grid, block, smem, s, args...);
+      return launch_after(ws.alone && n < 2000000u, kernel, grid, block, smem, s, args...);
     };
     e = launch(k_tl_offsets, 1, 256, 0, st, cnt, n - 1, off, cursor, ctl);
     if (e == cudaSuccess) e = launch(k_tl_scatter, div_up(n - 1, 256), 256, 0, st, ws.heights, n - 1, cursor, list);
