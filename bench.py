@@ -152,7 +152,7 @@ def kernels_per_build(algo: str, bits: int, rounds: int = 0, ploc_iterations: in
     """Launches of this library's kernels in one build: bounds, Morton, 4 onesweep passes, the run
     fix-up of 60/63-bit codes (short runs, listed long runs; it writes the delta bytes too),
     emission (which computes the delta bytes of 30-bit codes) + frontier climb;
-    per treelet pass five (heights, counts, offsets, grouping by height, the fallback check) plus
+    per treelet pass five (counts, offsets, grouping by height, the fallback's links and check) plus
     growth, DP and loop control per tree level; PLOC adds cluster init, 4 per clustering iteration
     launched one kernel per phase (neighbours, tile counts + scan, merge + compaction, loop
     control) and the root fix
@@ -187,7 +187,7 @@ STAGE_KERNELS = {
     "morton_boxes_hist": "k_morton",
     "onesweep_sort": "k_onesweep x4 (+ k_fixrun_split_short/_long for 60/63-bit codes)",
     "emit_refit": "k_emit (with the delta bytes of 30-bit codes) + k_emit_climb",
-    "treelet_or_ploc_loop": "LBVH+: k_tl_heights, k_tl_count, k_tl_offsets, k_tl_scatter, then k_tl_grow +"
+    "treelet_or_ploc_loop": "LBVH+: k_tl_count, k_tl_offsets, k_tl_scatter, then k_tl_grow +"
                             " k_tl_dp per tree height; PLOC: k_ploc_nn, k_ploc_count, k_ploc_scatter, k_ploc_step"
                             " per iteration + k_ploc_root",
 }
@@ -197,8 +197,8 @@ STAGE_KERNELS = {
 # the stage's traffic grows with the triangle count, so a launch over n triangles moves about
 # n times this.  Keyed by (algorithm, Morton bits, stage).
 MEASURED_TRAFFIC_PER_TRI = {
-    ("lbvh", 63, "emit_refit"): (191.6, "one ncu capture of k_emit + k_emit_climb on 4M triangles of the same "
-                                        "distribution: 766 MB / 4M triangles, scaled by the triangle count"),
+    ("lbvh", 63, "emit_refit"): (193.8, "one ncu capture of k_emit + k_emit_climb on 4M triangles of the same "
+                                        "distribution: 775 MB / 4M triangles, scaled by the triangle count"),
 }
 
 

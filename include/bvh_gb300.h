@@ -60,7 +60,7 @@ typedef struct bvh_node {
   float max_x, max_y, max_z, pad1;
   int32_t left;  /* child index, or (primitive | 0x80000000) for a leaf */
   int32_t right; /* child index, or -1 for a leaf */
-  int32_t aux0;  /* implementation detail (parent index while building); ignore */
+  int32_t aux0;  /* implementation detail (LBVH+: a child's area); ignore */
   int32_t aux1;
 } bvh_node;
 
