@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import abc
 import ctypes
-import sys
+import weakref
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -65,14 +65,50 @@ class TriangleMesh:
         return v.min(0), v.max(0)
 
 
+class _Lease:
+    """What an array handed out by _HostArrays refers to: numpy keeps it as the array's base, so it is gone when
+    the last array, view or buffer of that memory is."""
+
+    __slots__ = ("__array_interface__", "__weakref__")
+
+    def __init__(self, piece: np.ndarray, size: int):
+        self.__array_interface__ = dict(piece.__array_interface__, shape=(size,))
+
+
 class _HostArrays:
     """Memory for the arrays that builds return.  The pages of a new 100 MB array cost three times what
     copying a tree into it does, so memory that nobody refers to any more (every array made from it is
-    gone) serves the next result.  At most `keep` idle pieces stay, none more than twice as large as asked for."""
+    gone) serves the next result.  At most `keep` idle pieces stay, none more than twice as large as asked for.
+
+    A piece is in `_pieces` only while it is idle; the finalizer of its lease puts it back, on whatever thread
+    drops the last reference (append and pop of a list are atomic)."""
 
     def __init__(self, keep: int = 2):
         self._keep = keep
         self._pieces: list = []
+
+    @staticmethod
+    def _give_back(pieces: list, keep: int, piece: np.ndarray):
+        pieces.append(piece)
+        while len(pieces) > keep:  # the oldest goes
+            try:
+                pieces.pop(0)
+            except IndexError:  # another thread took the rest
+                return
+
+    def _idle(self, need: int) -> Optional[np.ndarray]:
+        others, found = [], None
+        while found is None:
+            try:
+                piece = self._pieces.pop()
+            except IndexError:
+                break
+            if need <= piece.size <= 2 * need:
+                found = piece
+            else:
+                others.append(piece)
+        self._pieces.extend(reversed(others))
+        return found
 
     def take(self, dtype, count: int) -> np.ndarray:
         """An array of `count` items, uninitialised."""
@@ -80,21 +116,12 @@ class _HostArrays:
         need = count * dtype.itemsize
         if need < 1 << 20:
             return np.empty(count, dtype)
-        idle, busy, found = [], [], None
-        pieces, self._pieces = self._pieces, []
-        while pieces:
-            piece = pieces.pop()
-            # the only references left: this name and getrefcount's argument (a view refers to its piece)
-            if sys.getrefcount(piece) > 2:
-                busy.append(piece)
-            elif found is None and need <= piece.size <= 2 * need:
-                found = piece
-            else:
-                idle.append(piece)
-        if found is None:
-            found = np.empty(need, np.uint8)
-        self._pieces = (idle[: self._keep] + busy)[:: -1] + [found]
-        return found[:need].view(dtype)
+        piece = self._idle(need)
+        if piece is None:
+            piece = np.empty(need, np.uint8)
+        lease = _Lease(piece, need)
+        weakref.finalize(lease, self._give_back, self._pieces, self._keep, piece).atexit = False
+        return np.asarray(lease).view(dtype)
 
 
 class Context:
