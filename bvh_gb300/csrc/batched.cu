@@ -219,7 +219,8 @@ __global__ void __launch_bounds__(256) k_seg_morton(MeshPtrs m, int vec4, const 
 // (mesh, code30, index) order is in ws.vals[*fb] (global triangle indices) and ws.keys[*fb]
 // holds the high 32 bits of the keys.
 cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_t count, const SegItem* d_items,
-                           uint32_t n_items, float* d_mbox, cudaStream_t st, StageEvents* evs, BatchedSort* out) {
+                           uint32_t n_items, float* d_mbox, uint32_t* d_indices, cudaStream_t st, StageEvents* evs,
+                           BatchedSort* out) {
   cudaError_t e = workspace_reserve(ws, n, st);
   if (e != cudaSuccess) return e;
   ScratchLayout L = scratch_layout(ws.cap_n);
@@ -233,10 +234,8 @@ cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_
   const int passes = kbits > 32 ? 4 : (kbits + 7) / 8;
   L.zero_end = L.desc + (size_t)passes * div_up(std::max<uint32_t>(n, 1),
                                                  (uint32_t)sort_variant_tile(ws.sort_variant)) * 256;
-  // the low key bits live at the start of the node buffer until the delta pass has read them
-  uint32_t* lows = reinterpret_cast<uint32_t*>(ws.nodes);
-  unsigned long long* run_scratch = reinterpret_cast<unsigned long long*>(
-      reinterpret_cast<unsigned char*>(ws.nodes) + (((size_t)n * 4 + 15) & ~(size_t)15));
+  // the low key bits live in the output indices, which are written after the delta pass has read them
+  uint32_t* lows = d_indices;
   if (evs && evs->use) cudaEventRecord(evs->ev[0], st);
   if ((e = epoch_tick(ws, st)) != cudaSuccess) return e;
   k_seg_init<<<152 * 4, 256, 0, st>>>(d_mbox, count, ws.scratch, L);
@@ -254,7 +253,7 @@ cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_
   const uint32_t* hkeys = reinterpret_cast<const uint32_t*>(ws.keys[fb]);
   if (shift0 > 0 &&
       (e = sort_fix_runs_split(hkeys, ws.vals[fb], lows, n, shift0,
-                               reinterpret_cast<unsigned long long*>(ws.keys[fb ^ 1]), run_scratch, ws.vals[fb ^ 1],
+                               reinterpret_cast<unsigned long long*>(ws.keys[fb ^ 1]), ws.slots, ws.vals[fb ^ 1],
                                reinterpret_cast<uint32_t*>(ws.delta), ws.scratch + L.counters + kLongRunCounter,
                                nullptr, st, ws.alone)) != cudaSuccess)
     return e;
@@ -268,7 +267,7 @@ cudaError_t batched_build(Workspace& ws, const MeshPtrs& m, uint32_t n, const ui
                           const SegItem* d_items, uint32_t n_items, float* d_mbox, uint32_t* d_indices,
                           cudaStream_t st, StageEvents* evs) {
   BatchedSort bs;
-  cudaError_t e = batched_prefix(ws, m, n, count, d_items, n_items, d_mbox, st, evs, &bs);
+  cudaError_t e = batched_prefix(ws, m, n, count, d_items, n_items, d_mbox, d_indices, st, evs, &bs);
   if (e != cudaSuccess) return e;
   ScratchLayout L = scratch_layout(ws.cap_n);
   const int fb = bs.fb;

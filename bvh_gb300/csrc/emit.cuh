@@ -18,6 +18,7 @@
 // child's its first, the root is 0.  Segments (batched meshes) number their nodes from their
 // own base and see delta = -1 across their boundaries.
 #pragma once
+#include "climb_message.h"
 #include "common.cuh"
 
 namespace bvhgb {
@@ -187,11 +188,19 @@ __device__ __forceinline__ void climb_merge(Climb& c, bool is_left, int32_t sib_
   }
 }
 
+__device__ __forceinline__ void clear_padding(Node* nodes, uint32_t idx) {
+  __stcg(&nodes[idx].lo.w, 0.f);
+  __stcg(&nodes[idx].hi.w, 0.f);
+}
+
 // T sorted positions per block, one thread each (a larger block leaves fewer nodes whose sibling
 // lies in another block to the frontier pass).
 // KEYS30: the tile's delta bytes are computed here from the sorted 30-bit keys (the delta_nt
 // rule, as k_delta) and written to D for k_emit_climb; otherwise they are read from D.
-template <typename Seg, bool PLUS, uint32_t T = 256, bool KEYS30 = false>
+// CLEAR: the node memory is a caller's and may hold anything; the padding of the nodes that no climb in the
+// tile writes is cleared, since k_emit_climb reads it (100,000 triangles 0.4 us; 10M 24, 29M in 1,024 meshes
+// 104, which is why a workspace's memory is cleared when it is allocated and kept so).
+template <typename Seg, bool PLUS, uint32_t T = 256, bool KEYS30 = false, bool CLEAR = false>
 __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, const uint32_t* __restrict__ keys30,
                                             const uint32_t* __restrict__ vals,
                                             const Box* __restrict__ tri_boxes, Node* __restrict__ nodes,
@@ -209,10 +218,12 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   __shared__ float4 s_lo[2][T];
   __shared__ float4 s_hi[2][T];
   __shared__ uint8_t s_h[2][PLUS ? T : 1];  // the child's height
+  __shared__ uint8_t s_written[CLEAR ? T : 1];  // the inner node of position bbase + k was written here
   const uint32_t tid = threadIdx.x;
   const uint32_t i = blockIdx.x * T + tid;
   const uint32_t bbase = blockIdx.x * T;  // sorted position of thread 0
   s_flag[tid] = 0;
+  if (CLEAR) s_written[tid] = 0;
   after_previous();
   stage_stamp(stamps, 3);
   bool active = i < n;
@@ -282,6 +293,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     const uint32_t gamma = is_left ? c.l : c.f - 1;
     const bool pending = c.internal;  // complete; its id is known now: a left child is named by its last index
     if (pending) c.my = (int32_t)((is_left ? c.l : c.f) - off);
+    if (CLEAR && pending) s_written[(is_left ? c.l : c.f) - bbase] = 1;  // (below, on either way)
     // sibling starts outside the block, or the climb has gone max_steps levels: the node
     // continues in k_emit_climb, so that one long chain does not hold the block
     if (step >= max_steps || (is_left ? gamma + 1 >= bbase + T : gamma < bbase)) {
@@ -313,6 +325,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     c.internal = true;
   }
   __syncthreads();
+  if (CLEAR && i < n && i - off + 1 < cnt && !s_written[tid]) clear_padding(nodes, nb + (i - off));
   // ---- finished nodes whose parent needs a sibling built elsewhere continue in k_emit_climb:
   // those stopped at the block edge and those whose in-block sibling never completed ----
   uint2 fr0 = make_uint2(c.f, c.l), fr1 = make_uint2(0u, 0u);
@@ -340,10 +353,6 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
   if (nf > 1) frontier[s_base + slot_in_block + 1] = fr1;
 }
 
-__device__ __forceinline__ void clear_padding(Node* nodes, uint32_t idx) {
-  __stcg(&nodes[idx].lo.w, 0.f);
-  __stcg(&nodes[idx].hi.w, 0.f);
-}
 constexpr uint32_t kClimbSpins = 1u << 22;  // re-reads of a node whose writer has announced it
 
 // The node c, a left child (LEFT) or a right one, and its sibling, announced by `old`, become their parent; dfar
@@ -353,27 +362,26 @@ constexpr uint32_t kClimbSpins = 1u << 22;  // re-reads of a node whose writer h
 template <bool PLUS, bool LEFT>
 __device__ __forceinline__ bool climb_join(Climb& c, uint32_t& dfar, unsigned long long old, uint32_t sib, float4 slo,
                                            float4 shi, uint32_t here, uint32_t g, uint32_t off, uint32_t cnt,
-                                           uint32_t nb, uint32_t n, uint32_t epoch, const uint8_t* __restrict__ D,
-                                           Node* nodes, const uint8_t* hgt) {
+                                           uint32_t nb, uint32_t n, uint32_t epoch, uint32_t mark,
+                                           const uint8_t* __restrict__ D, Node* nodes, const uint8_t* hgt) {
   const uint32_t other = (uint32_t)old;
   if (here) clear_padding(nodes, nb + (uint32_t)c.my);
   if (LEFT) c.l = other;
   else c.f = other;
   if ((old >> 32) & 1u) {
     const float4* sp = reinterpret_cast<const float4*>(nodes + nb + sib);
-    for (uint32_t spins = 0;
-         __float_as_uint(slo.w) != epoch || __float_as_uint(shi.w) >> 16 != ((epoch >> 6) & 0xffffu); ++spins) {
+    for (uint32_t spins = 0; !climb_whole(__float_as_uint(slo.w), __float_as_uint(shi.w), epoch, mark); ++spins) {
       if (spins >= kClimbSpins) return false;
       slo = ld_relaxed16(sp);
       shi = ld_relaxed16(sp + 1);
     }
     clear_padding(nodes, nb + sib);
     const uint32_t w = __float_as_uint(shi.w);
-    dfar = (w >> 8) & 0xffu;
+    dfar = climb_delta(w);
     Box sb;
     sb.lo = make_float4(slo.x, slo.y, slo.z, 0.f);
     sb.hi = make_float4(shi.x, shi.y, shi.z, 0.f);
-    climb_merge<PLUS>(c, LEFT, (int32_t)sib, sb, w & 0xffu);
+    climb_merge<PLUS>(c, LEFT, (int32_t)sib, sb, climb_height(w));
     return true;
   }
   const bool leaf = other == g + off + (LEFT ? 1u : 0u);
@@ -390,10 +398,11 @@ __device__ __forceinline__ bool climb_join(Climb& c, uint32_t& dfar, unsigned lo
 //
 // What bounds it is the chain of one round trip after another, a dozen or more levels from the tiles to
 // the root.  A node is therefore its own message: while its parent is missing, the padding of its two
-// corners (each written and read as 16 bytes at once) holds the build's epoch and, beside it, the delta
-// byte past its far end and its height.  No fence orders the node's stores before its announcement: the
-// sibling, which reads the node while its own announcement is under way, sees by the epoch whether it has
-// it, and otherwise reads again.  Both paddings are 0 again once the parent is complete.  A rendezvous word is
+// corners (each written and read as 16 bytes at once) holds the build's epoch and a mark of it and, beside
+// that, the delta byte past its far end and its height (climb_message.h).  No fence orders the node's
+// stores before its announcement: the sibling, which reads the node while its own announcement is under way,
+// sees by epoch and mark whether it has it, and otherwise reads again.  Both paddings are 0 before (see
+// Workspace::nodes, and k_emit's CLEAR) and again once the parent is complete.  A rendezvous word is
 // (epoch | written in this kernel) << 32 | far end; a node written by k_emit (bit 0 clear) carries
 // no epoch and needs none.
 // With a fence before the exchange, and the sibling's box and delta byte read after it, emission took 43 us of
@@ -408,6 +417,7 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
   after_previous();
   const uint32_t count = __ldcg(frontier_count);
   const uint32_t epoch = __ldcg(epoch_word);  // (a multiple of kEpochStride)
+  const uint32_t mark = climb_mark(epoch);
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
     const uint2 fl = __ldcg(frontier + e);
     Climb c;
@@ -436,8 +446,8 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
           atom_exch_relaxed(slots + gamma, (unsigned long long)(epoch | here) << 32 | (is_left ? c.f : c.l));
       if ((uint32_t)(old >> 33) != epoch >> 1) break;  // first child to arrive
       const bool ok =
-          is_left ? climb_join<PLUS, true>(c, dr, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, D, nodes, hgt)
-                  : climb_join<PLUS, false>(c, dl, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, D, nodes, hgt);
+          is_left ? climb_join<PLUS, true>(c, dr, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, mark, D, nodes, hgt)
+                  : climb_join<PLUS, false>(c, dl, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, mark, D, nodes, hgt);
       if (!ok) {
         atomicOr(status, kStatusClimbTimeout);
         break;
@@ -453,7 +463,7 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
       float4* np = reinterpret_cast<float4*>(nodes + nb + (uint32_t)c.my);
       st_relaxed16(np, make_float4(c.box.lo.x, c.box.lo.y, c.box.lo.z, __uint_as_float(epoch)));
       st_relaxed16(np + 1, make_float4(c.box.hi.x, c.box.hi.y, c.box.hi.z,
-                                       __uint_as_float((epoch >> 6) << 16 | (is_left ? dl : dr) << 8 | min(c.h, 255u))));
+                                       __uint_as_float(climb_hi_word(mark, is_left ? dl : dr, c.h))));
       __stcg(reinterpret_cast<int4*>(np + 2), PLUS ? make_int4(c.lc, c.rc, __float_as_int(c.al), __float_as_int(c.ar))
                                                    : make_int4(c.lc, c.rc, -1, 0));
       if (PLUS) __stcg(hgt + nb + (uint32_t)c.my, (uint8_t)min(c.h, 255u));

@@ -698,6 +698,7 @@ cudaError_t workspace_reserve(Workspace& ws, uint32_t n, cudaStream_t st) {
   ScratchLayout L = scratch_layout(cap);
   if ((e = cudaMalloc(&ws.scratch, L.total * 4)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(ws.slots, 0, (size_t)cap * 8, st)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(ws.nodes, 0, 2 * (size_t)cap * sizeof(Node), st)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(ws.scratch, 0, L.total * 4, st)) != cudaSuccess) return e;
   ws.scratch_words = L.total;
   ws.cap_n = cap;
@@ -714,23 +715,21 @@ static inline void rec(StageEvents* evs, int k, cudaStream_t st) {
   if (evs && evs->use) cudaEventRecord(evs->ev[k], st);
 }
 
-// Split codes keep their low bits in the node buffer, which emission writes only after the run
-// fix-up: [lows by original index: 4n B][64-bit run scratch: 8n B][long-run list: n/6 words],
-// 16-byte aligned; at most 13n + 48 bytes of the 96n - 48 the nodes take.
+// Split codes keep their low bits in the leaf nodes, which emission writes only after the run fix-up (and
+// reads nothing of): from node n-1 on, [lows by original index: 4n B][long-run list: n/6 words], 16-byte
+// aligned; at most 5n + 32 of the 48n bytes (n >= 1: of the workspace's least size).
 static inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
-static inline uint32_t* split_lows(const Workspace& ws) { return reinterpret_cast<uint32_t*>(ws.nodes); }
-static inline unsigned long long* split_run_scratch(const Workspace& ws, uint32_t n) {
-  return reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(ws.nodes) + align16((size_t)n * 4));
+static inline uint32_t* split_lows(const Workspace& ws, uint32_t n) {
+  return reinterpret_cast<uint32_t*>(ws.nodes + (n ? n - 1 : 0));
 }
 static inline uint32_t* split_long_list(const Workspace& ws, uint32_t n) {
-  return reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(ws.nodes) + align16((size_t)n * 4) +
-                                     align16((size_t)n * 8));
+  return reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(split_lows(ws, n)) + align16((size_t)n * 4));
 }
 
 template <int BITS, typename K>
 static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cudaStream_t st, const ScratchLayout& L,
                                int* final_buf, bool plus) {
-  uint32_t* lows = sizeof(K) == 8 ? split_lows(ws) : nullptr;
+  uint32_t* lows = sizeof(K) == 8 ? split_lows(ws, n) : nullptr;
   const int vec4 = all_aligned16(m) && (reinterpret_cast<uintptr_t>(lows) & 15) == 0 ? 1 : 0;
   // zero only the descriptors the current build's passes use (the passes sort 32-bit keys)
   ScratchLayout Lz = L;
@@ -752,7 +751,7 @@ static cudaError_t lbvh_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, cud
     const int fb = *final_buf;
     // the fix-up also writes the delta bytes of the final order
     e = sort_fix_runs_split(reinterpret_cast<const uint32_t*>(ws.keys[fb]), ws.vals[fb], lows, n, BITS - 32,
-                            reinterpret_cast<unsigned long long*>(ws.keys[fb ^ 1]), split_run_scratch(ws, n),
+                            reinterpret_cast<unsigned long long*>(ws.keys[fb ^ 1]), ws.slots,
                             ws.vals[fb ^ 1], split_long_list(ws, n), ws.scratch + L.counters + kLongRunCounter,
                             ws.delta, st, ws.alone);
   }
@@ -777,9 +776,11 @@ static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchL
   uint2* frontier = reinterpret_cast<uint2*>(ws.keys[fb ^ 1]);  // the sort's other key buffer, 8 B per position
   // delta bytes: computed by k_emit from the 30-bit keys, written by the run fix-up for 60/63 bits
   unsigned long long* stamps = reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps);
-  cudaError_t e = launch_after(ws.alone, k_emit<SegSingle, PLUS, kEmitTile, BITS == 30>, div_up(n, kEmitTile), kEmitTile, 0, st,
-                               ws.delta, keys, ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier,
-                               fcount, emit_max_steps(n), stamps, ws.heights);
+  const auto emit = ws.caller_nodes && !PLUS ? k_emit<SegSingle, false, kEmitTile, BITS == 30, true>
+                                             : k_emit<SegSingle, PLUS, kEmitTile, BITS == 30>;
+  cudaError_t e = launch_after(ws.alone, emit, div_up(n, kEmitTile), kEmitTile, 0, st, ws.delta, keys,
+                               ws.vals[fb], ws.boxes, ws.nodes, n, SegSingle{n}, nullptr, frontier, fcount, emit_max_steps(n),
+                               stamps, ws.heights);
   if (e != cudaSuccess) return e;
   if (ws.leaves_ready && !PLUS) cudaEventRecord(ws.leaves_ready, st);
   return launch_after(ws.alone, k_emit_climb<SegSingle, PLUS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,

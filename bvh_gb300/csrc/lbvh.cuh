@@ -25,8 +25,14 @@ struct Workspace {
   void* keys[2] = {nullptr, nullptr};
   uint32_t* vals[2] = {nullptr, nullptr};
   Box* boxes = nullptr;      // per-triangle AABB in input order
-  Node* nodes = nullptr;     // 2n-1 output nodes
-  unsigned long long* slots = nullptr;  // n-1 rendezvous words (epoch | flag) << 32 | endpoint
+  // 2n-1 output nodes.  The padding of the inner nodes' corners is 0 between builds -- cleared when allocated,
+  // left so by every build that ends well -- because emission reads it (climb_message.h); so no build keeps
+  // other data there.  caller_nodes: the memory is a caller's, and the build clears what it reads.
+  Node* nodes = nullptr;
+  bool caller_nodes = false;
+  // n-1 rendezvous words (epoch | flag) << 32 | endpoint; before the emission, the run fix-up's second buffer of
+  // low key bits, which are below 2^32: no word of theirs carries an epoch
+  unsigned long long* slots = nullptr;
   uint32_t* scratch = nullptr;          // histograms, look-back descriptors, counters
   uint8_t* delta = nullptr;             // n-1 adjacent common-prefix lengths (+1)
   uint8_t* heights = nullptr;           // LBVH+: n-1 inner nodes' heights (at most 255)
@@ -252,10 +258,11 @@ constexpr uint32_t kSegChunk = 4096;
 struct BatchedSort {
   int fb = 0;              // ping-pong buffer holding the sorted keys (high 32 bits) and indices
   int shift0 = 0;          // key bits below the sorted high 32
-  uint32_t* lows = nullptr;  // those low bits by original index (inside the node buffer)
+  uint32_t* lows = nullptr;  // those low bits by original index (in the output indices, until emission or cluster start)
 };
 cudaError_t batched_prefix(Workspace& ws, const MeshPtrs& m, uint32_t n, uint32_t count, const SegItem* d_items,
-                           uint32_t n_items, float* d_mbox, cudaStream_t st, StageEvents* evs, BatchedSort* out);
+                           uint32_t n_items, float* d_mbox, uint32_t* d_indices, cudaStream_t st,
+                           StageEvents* evs, BatchedSort* out);
 
 // Batched PLOC(radius) over the same layout: every mesh's tree equals its single build.  d_mbox
 // (8 words per mesh) holds the per-mesh loop state once the keys are made.

@@ -95,6 +95,7 @@ extern "C" bvh_status bvh_build_lbvh_static(const bvh_mesh_soa* mesh, int32_t mo
   ws.delta = base + o; o += kDeltaBytes;
   ws.scratch = reinterpret_cast<uint32_t*>(base + o);
   ws.nodes = reinterpret_cast<Node*>(nodes);
+  ws.caller_nodes = true;
   ws.cap_n = kStaticMaxTris;
   ws.scratch_words = kScratchBytes / 4;
   if (scratch_layout(kStaticMaxTris).total > ws.scratch_words) return BVH_ERR_DEVICE;  // layout guard

@@ -1835,7 +1835,7 @@ cudaError_t batched_ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, con
     }
   }
   BatchedSort bs;
-  if ((e = batched_prefix(ws, m, n, count, d_items, n_items, d_mbox, st, evs, &bs)) != cudaSuccess) return e;
+  if ((e = batched_prefix(ws, m, n, count, d_items, n_items, d_mbox, d_indices, st, evs, &bs)) != cudaSuccess) return e;
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(n_items, 152 * 8));
   k_ploc_init_seg<<<grid, 256, 0, st>>>(ws.vals[bs.fb], ws.boxes, B, S, d_items, n_items, n, cap, d_indices,
                                        reinterpret_cast<unsigned long long*>(ws.scratch + L.stamps));
