@@ -20,6 +20,7 @@ struct BatchGraph {
   uint32_t n = 0, count = 0;
   int32_t algo = -1, radius = 0, max_iter = 0, sort_variant = -1;
   uint32_t shape = 0;
+  uint64_t generation = 0;  // of the workspace whose addresses it holds
   std::vector<uint32_t> offsets;
 };
 
@@ -475,6 +476,7 @@ static cudaError_t reserve_batch(Workspace& ws, uint32_t n, uint32_t count, size
   if (e != cudaSuccess) return e;
   if (ws.bat_words_cap < words || ws.bat_count_cap < count || !ws.bat_offsets) {
     cudaDeviceSynchronize();  // the staging buffer may still be read by queued copies
+    workspace_moves(ws);
     cudaFree(ws.bat_offsets);
     cudaFreeHost(ws.bat_offsets_h);
     cudaFree(ws.bat_mbox);
@@ -490,6 +492,7 @@ static cudaError_t reserve_batch(Workspace& ws, uint32_t n, uint32_t count, size
     ws.bat_words_cap = wcap;
   }
   if (ws.bat_n_cap < n || !ws.bat_indices) {
+    workspace_moves(ws);
     cudaFree(ws.bat_indices);
     ws.bat_indices = nullptr;
     ws.bat_n_cap = 0;
@@ -561,7 +564,7 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
                          !(ploc && params->reserved[1] == BVH_HOST_DRIVEN_LOOPS);
   if (use_graph) {
     BatchGraph& g = ctx->bgraph;
-    bool same = g.exec && !changed && g.n == n && g.count == count && memcmp(g.ptrs, m.v, sizeof(g.ptrs)) == 0 &&
+    bool same = g.exec && !changed && g.generation == ws.generation && g.n == n && g.count == count && memcmp(g.ptrs, m.v, sizeof(g.ptrs)) == 0 &&
                 g.algo == params->algo && g.radius == params->ploc_radius && g.max_iter == params->max_iterations &&
                 g.sort_variant == ws.sort_variant && g.shape == ((uint32_t)ws.ploc_nn_bps << 16 | (uint32_t)ws.ploc_mg_bps);
     if (!same) {
@@ -580,6 +583,7 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) { g.exec = nullptr; return from_cuda(e); }
       memcpy(g.ptrs, m.v, sizeof(g.ptrs));
+      g.generation = ws.generation;
       g.n = n;
       g.count = count;
       g.algo = params->algo;

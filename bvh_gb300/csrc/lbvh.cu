@@ -650,12 +650,9 @@ void workspace_free(Workspace& ws) {
   cudaFree(ws.vals[0]); cudaFree(ws.vals[1]);
   cudaFree(ws.boxes); cudaFree(ws.nodes); cudaFree(ws.slots); cudaFree(ws.scratch); cudaFree(ws.delta);
   cudaFree(ws.heights);
-  if (ws.ploc_exec) cudaGraphExecDestroy(ws.ploc_exec);
-  if (ws.ploc_seg_exec) cudaGraphExecDestroy(ws.ploc_seg_exec);
+  workspace_moves(ws);
   if (ws.aux_stream) cudaStreamDestroy(ws.aux_stream);
   if (ws.ploc_host) cudaFreeHost(ws.ploc_host);
-  for (cudaGraphExec_t x : ws.tl_exec)
-    if (x) cudaGraphExecDestroy(x);
   cudaFree(ws.cbox[0]); cudaFree(ws.cbox[1]); cudaFree(ws.cid[0]); cudaFree(ws.cid[1]); cudaFree(ws.nbr);
   cudaFree(ws.mesh_dev);
   cudaFree(ws.bat_offsets); cudaFreeHost(ws.bat_offsets_h); cudaFree(ws.bat_mbox); cudaFree(ws.bat_indices);
@@ -676,8 +673,17 @@ cudaError_t epoch_tick(Workspace& ws, cudaStream_t st) {
   return e;
 }
 
+void workspace_moves(Workspace& ws) {
+  for (cudaGraphExec_t* x : {&ws.tl_exec[0], &ws.tl_exec[1], &ws.ploc_exec, &ws.ploc_seg_exec}) {
+    if (*x) cudaGraphExecDestroy(*x);
+    *x = nullptr;
+  }
+  ++ws.generation;
+}
+
 cudaError_t workspace_reserve(Workspace& ws, uint32_t n, cudaStream_t st) {
   if (n <= ws.cap_n && ws.scratch) return cudaSuccess;
+  workspace_moves(ws);
   uint32_t cap = std::max<uint32_t>(n, 1024);
   cudaFree(ws.keys[0]); cudaFree(ws.keys[1]); cudaFree(ws.vals[0]); cudaFree(ws.vals[1]);
   cudaFree(ws.boxes); cudaFree(ws.nodes); cudaFree(ws.slots); cudaFree(ws.scratch); cudaFree(ws.delta);

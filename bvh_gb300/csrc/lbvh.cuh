@@ -47,10 +47,7 @@ struct Workspace {
   // LBVH+ loop over heights, valid for the key below: [1] keeps the heights for a further pass
   cudaGraphExec_t tl_exec[2] = {nullptr, nullptr};
   uint32_t tl_key_n = 0;
-  const void* tl_key_nodes = nullptr;
-  const void* tl_key_list = nullptr;
-  const void* tl_key_desc = nullptr;
-  const void* tl_key_ctl = nullptr;
+  const void* tl_key_list = nullptr;  // (either of two buffers)
   bool tl_narrow = false;               // the last treelet pass launched k_tl_narrow
   int tl_dp3 = 0;                       // its launches of the DP at height 3
   // This workspace's builds are not known to share the GPU.  A server's slots (false) build in many streams at
@@ -61,16 +58,15 @@ struct Workspace {
   bool no_cooperative = false;          // run no cooperative kernel (their host-driven fallbacks)
   uint32_t ploc_key_n = 0;
   int ploc_key_r = 0;
-  const void* ploc_key_nodes = nullptr;
-  const void* ploc_key_scratch = nullptr;
   uint32_t ploc_key_shape = 0;  // nn and merge blocks per SM the cached loop graph was made with
   cudaStream_t aux_stream = nullptr;  // a second stream for capturing loop bodies
+  uint64_t generation = 0;             // times a buffer was reallocated (workspace_moves)
   uint64_t epoch_builds = 0;           // builds that bumped this workspace's epoch (epoch_tick)
   // the batched PLOC loop graph and what it was made for
   cudaGraphExec_t ploc_seg_exec = nullptr;
   uint32_t ploc_seg_key_n = 0, ploc_seg_key_count = 0;
   int ploc_seg_key_r = 0;
-  const void* ploc_seg_key[4] = {};
+  const void* ploc_seg_key[2] = {};  // the offsets and mesh boxes it was made with (a caller's, in a server)
   uint32_t ploc_seg_key_shape = 0;
   // device-side mesh copy for host-pointer builds
   float* mesh_dev = nullptr;
@@ -200,6 +196,10 @@ cudaError_t prepare_kernels(bool small = false);
 // counts instead (call it before cudaGraphLaunch).
 cudaError_t epoch_tick(Workspace& ws, cudaStream_t st);
 
+// The workspace's buffers are about to be reallocated: the graphs that hold their addresses go, and
+// ws.generation counts on, for a graph that somebody else keeps.  An address is no key: a buffer may come
+// back at its old address while others that a graph holds have moved.
+void workspace_moves(Workspace& ws);
 // Grow `ws` to hold n triangles (cudaMalloc; synchronising).
 cudaError_t workspace_reserve(Workspace& ws, uint32_t n, cudaStream_t st);
 cudaError_t workspace_reserve_ploc(Workspace& ws, uint32_t n);

@@ -1526,14 +1526,7 @@ cudaError_t workspace_reserve_ploc(Workspace& ws, uint32_t n) {
   }
   if (n <= ws.ploc_cap && ws.nbr) return cudaSuccess;
   uint32_t cap = std::max<uint32_t>(n, 1024);
-  if (ws.ploc_exec) {
-    cudaGraphExecDestroy(ws.ploc_exec);
-    ws.ploc_exec = nullptr;
-  }
-  if (ws.ploc_seg_exec) {  // both loop graphs hold the cluster buffers' addresses
-    cudaGraphExecDestroy(ws.ploc_seg_exec);
-    ws.ploc_seg_exec = nullptr;
-  }
+  workspace_moves(ws);
   cudaFree(ws.cbox[0]); cudaFree(ws.cbox[1]); cudaFree(ws.cid[0]); cudaFree(ws.cid[1]); cudaFree(ws.nbr);
   ws.cbox[0] = ws.cbox[1] = nullptr; ws.cid[0] = ws.cid[1] = nullptr; ws.nbr = nullptr; ws.ploc_cap = 0;
   cudaError_t e;
@@ -1711,16 +1704,13 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
   const PlocShape sh = ploc_shape(ws);
   if (host_loop && !ws.ploc_host && (e = cudaMallocHost(&ws.ploc_host, 64)) != cudaSuccess) return e;
   if (loop && !host_loop) {
-    const bool same = ws.ploc_exec && ws.ploc_key_n == n && ws.ploc_key_r == radius && ws.ploc_key_nodes == ws.nodes &&
-                      ws.ploc_key_scratch == ws.scratch && ws.ploc_key_shape == sh.key();
+    const bool same = ws.ploc_exec && ws.ploc_key_n == n && ws.ploc_key_r == radius && ws.ploc_key_shape == sh.key();
     if (!same) {
       if (ws.ploc_exec) cudaGraphExecDestroy(ws.ploc_exec);
       ws.ploc_exec = nullptr;
       if ((e = make_loop_graph<false>(B, none, n, radius, sh, &ws.ploc_exec)) != cudaSuccess) return e;
       ws.ploc_key_n = n;
       ws.ploc_key_r = radius;
-      ws.ploc_key_nodes = ws.nodes;
-      ws.ploc_key_scratch = ws.scratch;
       ws.ploc_key_shape = sh.key();
     }
   }
@@ -1817,9 +1807,8 @@ cudaError_t batched_ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, con
   if ((e = cudaStreamIsCapturing(st, &cst0)) != cudaSuccess) return e;
   if (loop && !host_loop && cst0 == cudaStreamCaptureStatusNone) {
     const bool same = ws.ploc_seg_exec && ws.ploc_seg_key_n == n && ws.ploc_seg_key_count == count &&
-                      ws.ploc_seg_key_r == radius && ws.ploc_seg_key[0] == ws.nodes &&
-                      ws.ploc_seg_key[1] == ws.scratch && ws.ploc_seg_key[2] == d_offsets &&
-                      ws.ploc_seg_key[3] == d_mbox && ws.ploc_seg_key_shape == sh.key();
+                      ws.ploc_seg_key_r == radius && ws.ploc_seg_key[0] == d_offsets &&
+                      ws.ploc_seg_key[1] == d_mbox && ws.ploc_seg_key_shape == sh.key();
     if (!same) {
       if (ws.ploc_seg_exec) cudaGraphExecDestroy(ws.ploc_seg_exec);
       ws.ploc_seg_exec = nullptr;
@@ -1828,10 +1817,8 @@ cudaError_t batched_ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, con
       ws.ploc_seg_key_n = n;
       ws.ploc_seg_key_count = count;
       ws.ploc_seg_key_r = radius;
-      ws.ploc_seg_key[0] = ws.nodes;
-      ws.ploc_seg_key[1] = ws.scratch;
-      ws.ploc_seg_key[2] = d_offsets;
-      ws.ploc_seg_key[3] = d_mbox;
+      ws.ploc_seg_key[0] = d_offsets;
+      ws.ploc_seg_key[1] = d_mbox;
     }
   }
   BatchedSort bs;

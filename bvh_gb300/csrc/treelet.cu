@@ -1169,9 +1169,7 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
   const auto kept = [&](int round) { return round + 1 < rounds ? ws.heights : nullptr; };
   // one loop graph per choice of keeping the heights: [1] for a pass that another follows
   for (int keep = rounds > 1 ? 1 : 0; keep >= 0 && !host_loop; --keep) {
-    const bool same = ws.tl_exec[keep] && ws.tl_key_n == n && ws.tl_key_nodes == ws.nodes && ws.tl_key_list == list &&
-                      ws.tl_key_desc == A.desc && ws.tl_key_ctl == ctl;
-    if (same) continue;
+    if (ws.tl_exec[keep] && ws.tl_key_n == n && ws.tl_key_list == list) continue;
     for (cudaGraphExec_t& x : ws.tl_exec) {
       if (x) cudaGraphExecDestroy(x);
       x = nullptr;
@@ -1182,10 +1180,7 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
         return e;
     }
     ws.tl_key_n = n;
-    ws.tl_key_nodes = ws.nodes;
     ws.tl_key_list = list;
-    ws.tl_key_desc = A.desc;
-    ws.tl_key_ctl = ctl;
   }
   ws.tl_narrow = narrow != 0;
   for (int r = 0; r < rounds && r + 1 < 0x20; ++r) {
