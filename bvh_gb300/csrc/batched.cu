@@ -284,7 +284,8 @@ cudaError_t batched_build(Workspace& ws, const MeshPtrs& m, uint32_t n, const ui
     return e;
   // launched plainly, as the per-mesh kernels: with 29M triangles emission takes 1,357 us, started early 1,434
   k_emit_climb<SegBatch, false><<<std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st>>>(
-      ws.delta, ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount, nullptr, ws.scratch + L.status);
+      ws.delta, ws.nodes, ws.slots, ws.scratch + L.epoch, n, seg, frontier, fcount, nullptr, ws.scratch + L.status,
+      kClimbSpins);
   return cudaGetLastError();
 }
 

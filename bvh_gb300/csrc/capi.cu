@@ -290,11 +290,18 @@ extern "C" bvh_status bvh_selftest_bounded_wait(int device, uint32_t polls) {
       polls > kSpinLimit)
     return BVH_ERR_INVALID_ARG;
   cudaSetDevice(device);
-  uint32_t status = 0, grid_status = 0;
+  uint32_t status = 0, grid_status = 0, climb_status = 0;
+  bool clean_stops = true, stops = false;
   cudaError_t e = wait_selftest(polls, &status);
   if (e != cudaSuccess) return from_cuda(e);
   if ((e = grid_wait_selftest(polls, &grid_status)) != cudaSuccess) return from_cuda(e);
-  return (status & kStatusSortTimeout) && (grid_status & kStatusGridTimeout) ? BVH_ERR_TIMEOUT : BVH_ERR_DEVICE;
+  if ((e = climb_wait_selftest(polls, &climb_status)) != cudaSuccess) return from_cuda(e);
+  if ((e = treelet_stop_selftest(0, &clean_stops)) != cudaSuccess) return from_cuda(e);
+  if ((e = treelet_stop_selftest(climb_status, &stops)) != cudaSuccess) return from_cuda(e);
+  return (status & kStatusSortTimeout) && (grid_status & kStatusGridTimeout) && (climb_status & kStatusClimbTimeout) &&
+                 stops && !clean_stops
+             ? BVH_ERR_TIMEOUT
+             : BVH_ERR_DEVICE;
 }
 
 extern "C" bvh_status bvh_sync(bvh_ctx* ctx) {

@@ -362,7 +362,7 @@ constexpr uint32_t kClimbSpins = 1u << 22;  // re-reads of a node whose writer h
 template <bool PLUS, bool LEFT>
 __device__ __forceinline__ bool climb_join(Climb& c, uint32_t& dfar, unsigned long long old, uint32_t sib, float4 slo,
                                            float4 shi, uint32_t here, uint32_t g, uint32_t off, uint32_t cnt,
-                                           uint32_t nb, uint32_t n, uint32_t epoch, uint32_t mark,
+                                           uint32_t nb, uint32_t n, uint32_t epoch, uint32_t mark, uint32_t limit,
                                            const uint8_t* __restrict__ D, Node* nodes, const uint8_t* hgt) {
   const uint32_t other = (uint32_t)old;
   if (here) clear_padding(nodes, nb + (uint32_t)c.my);
@@ -371,7 +371,7 @@ __device__ __forceinline__ bool climb_join(Climb& c, uint32_t& dfar, unsigned lo
   if ((old >> 32) & 1u) {
     const float4* sp = reinterpret_cast<const float4*>(nodes + nb + sib);
     for (uint32_t spins = 0; !climb_whole(__float_as_uint(slo.w), __float_as_uint(shi.w), epoch, mark); ++spins) {
-      if (spins >= kClimbSpins) return false;
+      if (spins >= limit) return false;
       slo = ld_relaxed16(sp);
       shi = ld_relaxed16(sp + 1);
     }
@@ -413,7 +413,8 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
                                                     const uint32_t* epoch_word, uint32_t n, Seg seg,
                                                     const uint2* __restrict__ frontier,
                                                     const uint32_t* __restrict__ frontier_count,
-                                                    uint8_t* __restrict__ hgt, uint32_t* __restrict__ status) {
+                                                    uint8_t* __restrict__ hgt, uint32_t* __restrict__ status,
+                                                    uint32_t limit) {
   after_previous();
   const uint32_t count = __ldcg(frontier_count);
   const uint32_t epoch = __ldcg(epoch_word);  // (a multiple of kEpochStride)
@@ -446,10 +447,11 @@ __global__ void __launch_bounds__(256) k_emit_climb(const uint8_t* __restrict__ 
           atom_exch_relaxed(slots + gamma, (unsigned long long)(epoch | here) << 32 | (is_left ? c.f : c.l));
       if ((uint32_t)(old >> 33) != epoch >> 1) break;  // first child to arrive
       const bool ok =
-          is_left ? climb_join<PLUS, true>(c, dr, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, mark, D, nodes, hgt)
-                  : climb_join<PLUS, false>(c, dl, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, mark, D, nodes, hgt);
-      if (!ok) {
+          is_left ? climb_join<PLUS, true>(c, dr, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, mark, limit, D, nodes, hgt)
+                  : climb_join<PLUS, false>(c, dl, old, sib, slo, shi, here, g, off, cnt, nb, n, epoch, mark, limit, D, nodes, hgt);
+      if (!ok) {  // nothing above is completed by anyone: the root becomes a leaf, so that no walk meets what is missing
         atomicOr(status, kStatusClimbTimeout);
+        store_node(nodes, nb, c.box, (int32_t)kLeafBit, -1, -1);
         break;
       }
       if (dl == 0 && dr == 0) {

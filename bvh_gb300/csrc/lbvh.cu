@@ -622,6 +622,59 @@ cudaError_t wait_selftest(uint32_t limit, uint32_t* status_out) {
   return e != cudaSuccess ? e : e2;
 }
 
+// Emission's wait for a node that was announced but does not arrive: two pairs of leaves, the left pair's node
+// written by its tile, the right pair's announced as written above the tiles, its padding still clear.
+struct ClimbSelfTest {
+  Node nodes[7];
+  unsigned long long slots[4];
+  uint2 frontier;
+  uint32_t frontier_count, epoch, status;
+  uint8_t D[4];
+};
+__device__ ClimbSelfTest g_climb_selftest;
+
+__global__ void k_climb_selftest_setup(int32_t* root) {
+  ClimbSelfTest& T = g_climb_selftest;
+  if (!root) {
+    for (uint32_t k = 0; k < sizeof(T) / 4; ++k) reinterpret_cast<uint32_t*>(&T)[k] = 0;
+    T.epoch = kEpochStride;
+    T.D[0] = T.D[2] = 9;
+    T.D[1] = 3;
+    T.frontier = make_uint2(0u, 1u);
+    T.frontier_count = 1;
+    T.slots[1] = (unsigned long long)(kEpochStride | 1u) << 32 | 3u;
+    T.nodes[0].left = 1;
+    T.nodes[0].right = 2;
+  } else {
+    root[0] = (int32_t)T.status;
+    root[1] = T.nodes[0].left;
+  }
+}
+
+cudaError_t climb_wait_selftest(uint32_t limit, uint32_t* status_out) {
+  *status_out = 0;
+  void* p = nullptr;
+  int32_t* out = nullptr;  // in the test's own memory, past what it uses: the second pair's slot
+  cudaError_t e = cudaGetSymbolAddress(&p, g_climb_selftest);
+  cudaStream_t st = nullptr;
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  ClimbSelfTest* T = static_cast<ClimbSelfTest*>(p);
+  out = reinterpret_cast<int32_t*>(&T->slots[3]);
+  k_climb_selftest_setup<<<1, 1, 0, st>>>(nullptr);
+  k_emit_climb<SegSingle, false><<<1, 32, 0, st>>>(T->D, T->nodes, T->slots, &T->epoch, 4u, SegSingle{4u}, &T->frontier,
+                                                   &T->frontier_count, nullptr, &T->status, limit);
+  k_climb_selftest_setup<<<1, 1, 0, st>>>(out);
+  int32_t got[2] = {0, 0};
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(got, out, sizeof(got), cudaMemcpyDeviceToHost, st);
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  // the root has to be a leaf, so that nothing walks the unfinished tree
+  *status_out = got[1] < 0 ? (uint32_t)got[0] : 0u;
+  return e != cudaSuccess ? e : e2;
+}
+
 // ---------------------------------------------------------------------------------------
 // end of a build
 // ---------------------------------------------------------------------------------------
@@ -790,7 +843,8 @@ static cudaError_t launch_emit(Workspace& ws, int fb, uint32_t n, const ScratchL
   if (e != cudaSuccess) return e;
   if (ws.leaves_ready && !PLUS) cudaEventRecord(ws.leaves_ready, st);
   return launch_after(ws.alone, k_emit_climb<SegSingle, PLUS>, std::min<uint32_t>(div_up(n, 256), 152 * 16), 256, 0, st,
-                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount, ws.heights, ws.scratch + L.status);
+                      ws.delta, ws.nodes, ws.slots, epoch, n, SegSingle{n}, frontier, fcount, ws.heights, ws.scratch + L.status,
+                      kClimbSpins);
 }
 
 bool one_block_build(uint32_t n) { return n <= kSmallMax; }

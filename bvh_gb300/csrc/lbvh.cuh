@@ -186,6 +186,12 @@ cudaError_t wait_selftest(uint32_t limit, uint32_t* status_out);
 // after `limit` polls per block; *status_out = the status word it left (kStatusGridTimeout).
 cudaError_t grid_wait_selftest(uint32_t limit, uint32_t* status_out);
 
+// Runs emission's climb against a sibling that is announced but never arrives (kStatusClimbTimeout expected; 0
+// where the root was not left a leaf).
+cudaError_t climb_wait_selftest(uint32_t limit, uint32_t* status_out);
+// The status bits under which the treelet passes of a build leave its tree alone: given `status`, whether they do.
+cudaError_t treelet_stop_selftest(uint32_t status, bool* stops);
+
 // Kernel attributes (dynamic shared memory limits), set once per device before any capture.
 // small: those of the one-block builds too (14 kernels to load, 0.2 ms), which a workspace otherwise sets
 // when it first needs each.
@@ -237,7 +243,7 @@ cudaError_t sort_fix_runs_split(const uint32_t* hkeys, uint32_t* vals, const uin
 // (the other one is scratch).
 cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream_t st, int fb,
                                bool host_loop = false);
-// Treelet control words (scratch + L.hist + kTlCtlWord): [0] too high, [1] tree height.
+// Treelet control words (scratch + L.hist + kTlCtlWord): [0] flags (too high, stopped), [1] tree height.
 constexpr size_t kTlCtlWord = 256 + 264 + 256;
 
 // Stable sort of the 32-bit keys in ws.keys[0] with implicit indices over `passes` 8-bit digits;

@@ -345,6 +345,7 @@ __device__ void treelet_rebuild(Node* nodes, int32_t* parents, int32_t root, Lan
 // three passes 19.0 -> 12.1 ms, one pass at 200k 880 -> 542 us.
 // ---------------------------------------------------------------------------------------
 constexpr int kTlMaxHeight = 254;
+constexpr uint32_t kTlTooHigh = 1u, kTlStop = 2u;  // flags of the first control word
 constexpr int kLvThreads = 32;  // one warp per block; its DP table is 16 KB of shared memory
 
 // A lane's treelet in registers (all indexing below is unrolled to constant indices).
@@ -632,7 +633,7 @@ __device__ __forceinline__ void reg_build(Node* nodes, uint8_t* hgt, int32_t fir
 }
 
 // Nodes per height (block histograms in shared memory, one global add per nonzero bin).
-// A height past kTlMaxHeight hands this pass and the following ones to the fallback (flags[0]).
+// A height past kTlMaxHeight hands this pass and the following ones to the fallback (kTlTooHigh in flags[0]).
 __global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hgt, uint32_t m, uint32_t* __restrict__ cnt,
                                                   uint32_t* __restrict__ flags) {
   after_previous();
@@ -644,13 +645,14 @@ __global__ void __launch_bounds__(256) k_tl_count(const uint8_t* __restrict__ hg
   __syncthreads();
   const uint32_t c = s_cnt[threadIdx.x];
   if (c) atomicAdd(cnt + threadIdx.x, c);
-  if (c && threadIdx.x > kTlMaxHeight) atomicOr(flags, 1u);
+  if (c && threadIdx.x > kTlMaxHeight) atomicOr(flags, kTlTooHigh);
 }
 
 // off[h] = first list position of height h (exclusive scan of cnt over 256 heights), cursor
-// copy for the scatter, off[256] = total, flags[1] = the largest height.  A total other than
-// the m internal nodes (a malformed tree) hands the pass to the fallback.
-__global__ void __launch_bounds__(256) k_tl_offsets(const uint32_t* __restrict__ cnt, uint32_t m,
+// copy for the scatter, off[256] = total, flags[1] = the largest height.  A build that has given up
+// (any status bit: its tree may be unfinished, and growth would follow whatever its nodes hold) stops
+// here: this pass and the following ones, the fallback too, leave the tree alone (kTlStop in flags[0]).
+__global__ void __launch_bounds__(256) k_tl_offsets(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ status,
                                                     uint32_t* __restrict__ off, uint32_t* __restrict__ cursor,
                                                     uint32_t* __restrict__ flags) {
   after_previous();
@@ -672,10 +674,8 @@ __global__ void __launch_bounds__(256) k_tl_offsets(const uint32_t* __restrict__
   for (int k = 0; k < w; ++k) before += s_w[k];
   off[t] = before + x - v;
   cursor[t] = before + x - v;
-  if (t == 255) {
-    off[256] = before + x;
-    if (before + x != m) atomicOr(flags, 2u);
-  }
+  if (t == 255) off[256] = before + x;
+  if (t == 0 && __ldcg(status) != 0u) atomicOr(flags, kTlStop);
   __syncthreads();
   if (t == 0) {
     flags[1] = s_maxh;
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(256) k_tl_scatter(const uint8_t* __restrict__ 
 // treelet and writes a descriptor; k_tl_dp (compute-bound) loads the leaf boxes, runs the DP and
 // rebuilds.  Descriptors are structure-of-arrays, kTlDescWords words per
 // node at stride `stride` (>= the largest height's node count): [0] n | n_avail << 8,
-// [1..7] leaf ids, [8..13] reused internal ids in order.  ctl: [0] too high, [1] largest
+// [1..7] leaf ids, [8..13] reused internal ids in order.  ctl: [0] flags, [1] largest
 // height, [2] current height.  at: the height, 0 for the current one.
 constexpr int kGrowThreads = 128;
 
@@ -724,7 +724,7 @@ struct TlArgs {
 __global__ void __launch_bounds__(kGrowThreads, 8) k_tl_grow(TlArgs A, const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ ctl, uint32_t at) {
   after_previous();
-  if (__ldcg(ctl) != 0u) return;  // too high: the fallback pass does the work
+  if (__ldcg(ctl) != 0u) return;  // too high (the fallback pass does the work) or stopped
   const uint32_t h = at ? at : __ldcg(ctl + 2);
   const uint32_t b = __ldcg(A.off + h), e = __ldcg(A.off + h + 1);
   const bool wild = __ldcg(A.wild) != 0u;
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(kNarrowThreads) k_tl_narrow(TlArgs A, const ui
   __shared__ NarrowWarp s_warp[kNarrowThreads / 32];
   __shared__ uint32_t s_ok;
   // every block reads the same words (nothing writes them in this kernel)
-  if (__ldcg(ctl) != 0u) return;  // too high: the fallback pass does the work
+  if (__ldcg(ctl) != 0u) return;  // too high (the fallback pass does the work) or stopped
   const uint32_t h0 = __ldcg(ctl + 2), h1 = __ldcg(ctl + 1);
   const bool wild = __ldcg(A.wild) != 0u;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -996,11 +996,11 @@ __global__ void k_tl_step(uint32_t* __restrict__ ctl, const uint32_t* __restrict
   if constexpr (GRAPH) cudaGraphSetConditional(handle, go ? 1u : 0u);
 }
 
-// Parent links for the fallback; returns at once unless flags[0] is set.
+// Parent links for the fallback; returns at once unless flags[0] is kTlTooHigh.
 __global__ void __launch_bounds__(256) k_tl_parents(const Node* __restrict__ nodes, uint32_t m,
                                                     int32_t* __restrict__ parents, const uint32_t* __restrict__ flags) {
   after_previous();
-  if (__ldcg(flags) == 0u) return;
+  if (__ldcg(flags) != kTlTooHigh) return;
   for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) {
     const int2 ch = ldcg_children(nodes, (int32_t)x);
     parents[ch.x] = (int32_t)x;
@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(256) k_tl_parents(const Node* __restrict__ nod
 }
 
 // The climb-ordered pass as a fallback for trees higher than kTlMaxHeight: persistent warps
-// take groups of 32 leaves.  Launched every pass; returns at once unless flags[0] is set, which it
+// take groups of 32 leaves.  Launched every pass; returns at once unless flags[0] is kTlTooHigh, which it
 // stays for the following passes (this kernel keeps neither heights nor areas).
 __global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ nodes, int32_t* __restrict__ parents,
                                                          unsigned long long* __restrict__ slots,
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(64) k_treelet_fallback(Node* __restrict__ node
   after_previous();
   __shared__ LaneTreelet S[64];
   __shared__ float s_cost[2][1 << kTlMax], s_area[2][1 << kTlMax];
-  if (__ldcg(flags) == 0u) return;
+  if (__ldcg(flags) != kTlTooHigh) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned long long tag = (unsigned long long)(__ldcg(epoch_word) + 0x20u + round) << 32;
   LaneTreelet& mine = S[threadIdx.x];
@@ -1153,7 +1153,7 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
   uint32_t* cnt = ws.scratch + L.hist;       // 256
   uint32_t* off = cnt + 256;                 // 257
   uint32_t* cursor = off + 264;              // 256
-  uint32_t* ctl = cursor + 256;              // [0] too high, [1] largest height, [2] current height
+  uint32_t* ctl = cursor + 256;              // [0] flags, [1] largest height, [2] current height
   static_assert(kTlCtlWord == 256 + 264 + 256, "control words of the treelet pass");
   static_assert(kTlCtlWord + 8 <= (size_t)kMaxPasses * 256, "treelet words fit the histogram area");
   TlArgs A;
@@ -1200,7 +1200,7 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
     const auto launch = [&](auto kernel, uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, auto... args) {
       return launch_after(ws.alone && n < 2000000u, kernel, grid, block, smem, s, args...);
     };
-    e = launch(k_tl_offsets, 1, 256, 0, st, cnt, n - 1, off, cursor, ctl);
+    e = launch(k_tl_offsets, 1, 256, 0, st, cnt, ws.scratch + L.status, off, cursor, ctl);
     if (e == cudaSuccess) e = launch(k_tl_scatter, div_up(n - 1, 256), 256, 0, st, ws.heights, n - 1, cursor, list);
     // heights 1 to 3 first: every height-1 treelet has two leaves and is finished by the growth
     // kernel (in the first pass by the emission); height 2 holds at most 4 leaves and takes the smaller
@@ -1274,6 +1274,29 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
+}
+
+// k_tl_offsets over counts of zero and the given status word.
+__device__ uint32_t g_tl_selftest[256 + 264 + 256 + 8 + 8];
+
+cudaError_t treelet_stop_selftest(uint32_t status, bool* stops) {
+  *stops = false;
+  void* p = nullptr;
+  cudaStream_t st = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&p, g_tl_selftest);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  uint32_t *cnt = static_cast<uint32_t*>(p), *off = cnt + 256, *cursor = off + 264, *ctl = cursor + 256, *word = ctl + 8;
+  uint32_t flags = 0;
+  e = cudaMemsetAsync(p, 0, sizeof(g_tl_selftest), st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(word, &status, 4, cudaMemcpyHostToDevice, st);
+  k_tl_offsets<<<1, 256, 0, st>>>(cnt, word, off, cursor, ctl);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, ctl, 4, cudaMemcpyDeviceToHost, st);
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  *stops = (flags & kTlStop) != 0;
+  return e != cudaSuccess ? e : e2;
 }
 
 }  // namespace bvhgb

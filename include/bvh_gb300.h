@@ -193,11 +193,13 @@ bvh_status bvh_tree_download(bvh_ctx* ctx, const bvh_tree* tree, void* stream, b
                              uint32_t* host_indices);
 
 /* Self-test of the device-side bounded waits (no reference counterpart): the radix sort's
- * look-back wait is run on `device` against a predecessor that never publishes, and the grid
- * barrier of the cooperative PLOC kernel against a block that never arrives, each giving up after
- * `polls` polls (1 .. 16,777,216).  Returns BVH_ERR_TIMEOUT -- the expected outcome: both waits
- * ended and reported it, and the device is still usable -- or BVH_ERR_DEVICE / another error if
- * either did not.  Synchronous; allocates nothing. */
+ * look-back wait is run on `device` against a predecessor that never publishes, the grid barrier
+ * of the cooperative PLOC kernel against a block that never arrives, and the emission's wait
+ * against a node that is announced and never written, each giving up after `polls` polls (1 ..
+ * 16,777,216).  Returns BVH_ERR_TIMEOUT -- the expected outcome: all waits ended and reported it,
+ * the unfinished tree's root was left a leaf, LBVH+'s passes would leave such a tree alone, and the
+ * device is still usable -- or BVH_ERR_DEVICE / another error if one did not.  Synchronous;
+ * allocates nothing. */
 bvh_status bvh_selftest_bounded_wait(int device, uint32_t polls);
 
 /* Timing of the last build; waits for it to finish.  Also reports device-side errors. */
