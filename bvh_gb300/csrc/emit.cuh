@@ -112,6 +112,12 @@ static __global__ void __launch_bounds__(256)
   D[k] = (uint8_t)(d + 1);
 }
 
+// Delta bytes increase strictly from a node to its inner children and take at most 63 values from the code (one
+// per bit) and 32 from the index that ties are broken by, so no node of an emitted tree is higher than
+// this: it fits the byte that carries it.
+constexpr uint32_t kMaxTreeHeight = 63 + 32;
+static_assert(kMaxTreeHeight < 255, "a height takes one byte, 255 means higher");
+
 // Climb state of one lane: the node it currently owns covers sorted positions [f, l].  al, ar (its
 // children's areas) and h (its height) are kept for LBVH+ alone.
 struct Climb {
@@ -305,7 +311,7 @@ __global__ void __launch_bounds__(T, 2048 / T) k_emit(uint8_t* __restrict__ D, c
     const int side = is_left ? 0 : 1;
     s_lo[side][k] = make_float4(c.box.lo.x, c.box.lo.y, c.box.lo.z, __int_as_float(c.my));
     s_hi[side][k] = make_float4(c.box.hi.x, c.box.hi.y, c.box.hi.z, __uint_as_float(is_left ? c.f : c.l));
-    if (PLUS) s_h[side][k] = (uint8_t)c.h;  // (at most T)
+    if (PLUS) s_h[side][k] = (uint8_t)c.h;  // (at most kMaxTreeHeight)
     // release: the slot is visible before the flag bit; acquire: the sibling's slot is read after
     const uint32_t prev = atom_or_acq_rel_cta(&s_flag[k], 1u << side);
     if (pending) write_internal<PLUS>(nodes, hgt, nb, c.my, c);

@@ -90,7 +90,8 @@ struct Workspace {
   uint32_t small_ready = 0;  // one-block kernels whose attributes are set, by variant
 };
 
-// First epoch value; every build adds kEpochStride (emission uses E, treelet round r uses E+1+r).
+// First epoch value; every build adds kEpochStride.  Rendezvous words of build E carry E and E + 1 (emission)
+// and E + 32 + r (the fallback of treelet pass r < 31).
 constexpr uint32_t kEpochStride = 64;
 // The 32-bit epoch repeats after this many builds (it wraps to kEpochStride); the build that
 // reuses an epoch first clears the rendezvous slots (epoch_tick).

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       const int side = is_left ? 0 : 1;
       S.climb.lo[side][gamma] = make_float4(c.box.lo.x, c.box.lo.y, c.box.lo.z, __int_as_float(c.my));
       S.climb.hi[side][gamma] = make_float4(c.box.hi.x, c.box.hi.y, c.box.hi.z, __uint_as_float(is_left ? c.f : c.l));
-      if (PLUS) S.climb.h[side][gamma] = (uint8_t)c.h;  // (at most 95: the code's bits and 32)
+      if (PLUS) S.climb.h[side][gamma] = (uint8_t)c.h;  // (at most kMaxTreeHeight)
       const uint32_t prev = atom_or_acq_rel_cta(&S.climb.flag[gamma], 1u << side);
       if (pending) write_internal<PLUS>(nodes, hgt, 0, c.my, c);
       if (prev == 0u) break;  // first to arrive
