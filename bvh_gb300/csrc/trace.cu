@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(128) k_trace_pinhole(const Node* __restrict__ 
 // Packed traversal.  A ray's loop is a chain of dependent loads, and a warp's 32 rays load from 32
 // places: k_trace above fetches a 48-byte node per visit (two sectors each, then its children's
 // indices, then nine separate triangle arrays) and spends most of its time waiting for them.  For
-// a trace of many rays, two kernels first rewrite tree and mesh as 64-byte records -- per inner node
+// a trace of many rays, a kernel first rewrites tree and mesh as 64-byte records -- per inner node
 // both children's boxes and references, per triangle its vertex and edges -- so that
 //   - one 64-byte load decides both children: half the steps and half the bytes per visited node,
 //     a child that misses is counted without being fetched or pushed;
@@ -210,62 +210,138 @@ __device__ __forceinline__ void ld_record(const void* p, float (&w)[16]) {  // t
                  : "l"(reinterpret_cast<const char*>(p) + 32 * h));
 }
 
-// One record per inner node, read by two gathers of its children (neighbours in Karras numbering);
-// bound by DRAM traffic (20M nodes and 10M triangles: 2.6 GB in 0.50 ms).
-__global__ void __launch_bounds__(256) k_pack_nodes(const Node* __restrict__ nodes, int n_nodes,
-                                                    PackNode* __restrict__ rec) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_nodes; i += (int64_t)gridDim.x * blockDim.x) {
-    const int2 ch = __ldg(reinterpret_cast<const int2*>(reinterpret_cast<const float4*>(nodes + i) + 2));
-    if (ch.x < 0) continue;  // a leaf has no record
-    float4 b[2][2];
-    int32_t ref[2];
+// The record of inner node i, whose children are ch.
+__device__ __forceinline__ void node_record(const Node* __restrict__ nodes, int n_nodes, int2 ch, float (&w)[16]) {
+  float4 b[2][2];
+  int32_t ref[2];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int c = s ? ch.y : ch.x;
-      ref[s] = kPackNone;
-      b[s][0] = b[s][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c >= 0 && c < n_nodes) {
-        const float4* p = reinterpret_cast<const float4*>(nodes + c);
-        b[s][0] = __ldg(p);
-        b[s][1] = __ldg(p + 1);
-        const int32_t l = __ldg(reinterpret_cast<const int32_t*>(p + 2));
-        ref[s] = l < 0 ? l : c;
-      }
+  for (int s = 0; s < 2; ++s) {
+    const int c = s ? ch.y : ch.x;
+    ref[s] = kPackNone;
+    b[s][0] = b[s][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c >= 0 && c < n_nodes) {
+      const float4* p = reinterpret_cast<const float4*>(nodes + c);
+      b[s][0] = __ldg(p);
+      b[s][1] = __ldg(p + 1);
+      const int32_t l = __ldg(reinterpret_cast<const int32_t*>(p + 2));
+      ref[s] = l < 0 ? l : c;
     }
+  }
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    w[6 * s] = b[s][0].x; w[6 * s + 1] = b[s][0].y; w[6 * s + 2] = b[s][0].z;
+    w[6 * s + 3] = b[s][1].x; w[6 * s + 4] = b[s][1].y; w[6 * s + 5] = b[s][1].z;
+    w[12 + s] = __int_as_float(ref[s]);
+  }
+  w[14] = w[15] = 0.f;
+}
+__device__ __forceinline__ int2 node_children(const Node* __restrict__ nodes, int64_t i) {
+  return __ldg(reinterpret_cast<const int2*>(reinterpret_cast<const float4*>(nodes + i) + 2));
+}
+
+// The first nine words of triangle p's record.
+__device__ __forceinline__ void tri_record(const MeshPtrs& m, uint64_t p, float (&w)[16]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    w[k] = __ldg(m.v[k] + p);
+    w[3 + k] = __fsub_rn(__ldg(m.v[3 + k] + p), w[k]);
+    w[6 + k] = __fsub_rn(__ldg(m.v[6 + k] + p), w[k]);
+  }
+}
+
+// The rays of a trace: given ones, or the pixels of an image.
+struct GivenRays {
+  RayPtrs p;
+  __device__ __forceinline__ void get(uint32_t r, float3& o, float3& d) const {
+    o = make_float3(__ldg(p.o[0] + r), __ldg(p.o[1] + r), __ldg(p.o[2] + r));
+    d = make_float3(__ldg(p.d[0] + r), __ldg(p.d[1] + r), __ldg(p.d[2] + r));
+  }
+};
+struct PixelRays {
+  PinholeCam cam;
+  __device__ __forceinline__ void get(uint32_t r, float3& o, float3& d) const {
+    o = make_float3(cam.eye[0], cam.eye[1], cam.eye[2]);
+    d = pinhole_dir(cam, (int)(r % (uint32_t)cam.width), (int)(r / (uint32_t)cam.width));
+  }
+};
+
+// Whether one of 256 rays spread over the nr, one per thread of the block, enters the root's box.  Each is taken
+// at an odd place of its own 256th, so that the pixels of an image are not all of one column.
+template <typename Rays>
+__device__ __forceinline__ bool some_ray_enters(const Rays& rays, uint32_t nr, const Node* __restrict__ nodes) {
+  const uint32_t k = threadIdx.x, width = nr >> 8;
+  float3 o, d;
+  rays.get((uint32_t)(((uint64_t)k * nr) >> 8) + (k * 0x9e3779b1u >> 8) % width, o, d);
+  const float4* np = reinterpret_cast<const float4*>(nodes);
+  return __syncthreads_or(hit_box(o, make_float3(inv_dir(d.x), inv_dir(d.y), inv_dir(d.z)), __ldg(np), __ldg(np + 1), 1e30f));
+}
+
+// One record per inner node, read by two gathers of its children (neighbours in Karras numbering), and
+// one per triangle; bound by DRAM traffic (20M nodes and 10M triangles: 2.6 GB in 0.50 ms).
+// Where rays enter the scene at all, a trace waits for its longest chains and the records pay from the first few on:
+// with 2 in 100 entering, 16,384 rays over 16,000 nodes take 50 us packed and 82 plain, 262,144 over 4M 1,161
+// and 1,580.  A trace of which no ray enters is over in 5 us, which the records made 17 to 146.  So every block
+// looks at the same 256 rays first; where none of them enters, nothing is packed and *packed is 0 (12 to 21
+// us then, most of it the call's; with one ray in 2,000 entering 4M nodes 577 -> 323).
+template <typename Rays>
+__global__ void __launch_bounds__(256, 5) k_pack(const Node* __restrict__ nodes, int n_nodes, MeshPtrs m, uint32_t n_tris,
+                                              Rays rays, uint32_t nr, PackNode* __restrict__ rec,
+                                              PackTri* __restrict__ tris, uint32_t* __restrict__ packed) {
+  const bool enters = some_ray_enters(rays, nr, nodes);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *packed = enters ? 1u : 0u;
+  if (!enters) return;
+  const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 1
+  for (int64_t i = first; i < n_nodes; i += step) {
+    const int2 ch = node_children(nodes, i);
+    if (ch.x < 0) continue;  // a leaf has no record
+    float w[16];
+    node_record(nodes, n_nodes, ch, w);
     float4* o = reinterpret_cast<float4*>(rec + i);
-    o[0] = make_float4(b[0][0].x, b[0][0].y, b[0][0].z, b[0][1].x);
-    o[1] = make_float4(b[0][1].y, b[0][1].z, b[1][0].x, b[1][0].y);
-    o[2] = make_float4(b[1][0].z, b[1][1].x, b[1][1].y, b[1][1].z);
-    reinterpret_cast<int4*>(o)[3] = make_int4(ref[0], ref[1], 0, 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k] = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+  }
+#pragma unroll 1
+  for (int64_t p = first; p < n_tris; p += step) {
+    float w[16];
+    tri_record(m, (uint64_t)p, w);
+    float4* o = reinterpret_cast<float4*>(tris + p);
+    o[0] = make_float4(w[0], w[1], w[2], w[3]);
+    o[1] = make_float4(w[4], w[5], w[6], w[7]);
+    o[2] = make_float4(w[8], 0.f, 0.f, 0.f);
   }
 }
 
-__global__ void __launch_bounds__(256) k_pack_tris(MeshPtrs m, uint32_t n, PackTri* __restrict__ out) {
-  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < n; p += (uint64_t)gridDim.x * blockDim.x) {
-    const float v0x = __ldg(m.v[0] + p), v0y = __ldg(m.v[1] + p), v0z = __ldg(m.v[2] + p);
-    float4* o = reinterpret_cast<float4*>(out + p);
-    o[0] = make_float4(v0x, v0y, v0z, __fsub_rn(__ldg(m.v[3] + p), v0x));
-    o[1] = make_float4(__fsub_rn(__ldg(m.v[4] + p), v0y), __fsub_rn(__ldg(m.v[5] + p), v0z),
-                       __fsub_rn(__ldg(m.v[6] + p), v0x), __fsub_rn(__ldg(m.v[7] + p), v0y));
-    o[2] = make_float4(__fsub_rn(__ldg(m.v[8] + p), v0z), 0.f, 0.f, 0.f);
-  }
-}
+// The tree and its records, and whether these were made.
+struct PackedTree {
+  const Node* nodes;
+  int n_nodes;
+  MeshPtrs m;
+  uint32_t n_tris;
+  const PackNode* rec;
+  const PackTri* tris;
+  const uint32_t* packed;
+};
 
-__device__ __forceinline__ void trace_packed(bool live, const float3 o, const float3 d, const Node* __restrict__ nodes,
-                                             const PackNode* __restrict__ rec, const PackTri* __restrict__ tris,
-                                             uint32_t n_tris, uint32_t r, const HitOut& out) {
-  __shared__ int2 s_entry[kPackStack][kPackThreads];  // reference, entry distance
-  __shared__ uint8_t s_vs[kPackStack][kPackThreads];
-  int2 l_entry[kStack - kPackStack];
-  uint8_t l_vs[kStack - kPackStack];
+struct RayStack {  // what lies above the shared part
+  int2 entry[kStack - kPackStack];
+  uint8_t vs[kStack - kPackStack];
+};
+
+// PACKED: from the records; otherwise each is put together from the tree and the mesh when it is met.
+template <bool PACKED>
+__device__ __forceinline__ void trace_records(bool live, const float3 o, const float3 d, const PackedTree& T, uint32_t r,
+                                              const HitOut& out, int2 (*s_entry)[kPackThreads],
+                                              uint8_t (*s_vs)[kPackThreads], RayStack& local) {
   const int tid = threadIdx.x;
+  const uint32_t n_tris = T.n_tris;
   const float3 inv = make_float3(inv_dir(d.x), inv_dir(d.y), inv_dir(d.z));
   float best = 1e30f;
   int32_t prim = -1, vis = 0, tt = 0;
   int vs = 0, sp = 0;
   int32_t cur = kPackNone;
   if (live) {
-    const float4* np = reinterpret_cast<const float4*>(nodes);
+    const float4* np = reinterpret_cast<const float4*>(T.nodes);
     vis = 1;
     if (hit_box(o, inv, __ldg(np), __ldg(np + 1), best)) {
       const int32_t x = __ldg(reinterpret_cast<const int32_t*>(np + 2));
@@ -276,7 +352,12 @@ __device__ __forceinline__ void trace_packed(bool live, const float3 o, const fl
     const bool leaf = cur < 0;
     const uint32_t id = (uint32_t)cur & ~kLeafBit;
     float w[16];
-    ld_record(leaf ? static_cast<const void*>(tris + min(id, n_tris - 1)) : static_cast<const void*>(rec + id), w);
+    if (PACKED)
+      ld_record(leaf ? static_cast<const void*>(T.tris + min(id, n_tris - 1)) : static_cast<const void*>(T.rec + id), w);
+    else if (leaf)
+      tri_record(T.m, min(id, n_tris - 1), w);
+    else
+      node_record(T.nodes, T.n_nodes, node_children(T.nodes, id), w);
     bool pop;
     if (leaf) {
       tt++;
@@ -301,8 +382,8 @@ __device__ __forceinline__ void trace_packed(bool live, const float3 o, const fl
           s_entry[sp][tid] = e;
           s_vs[sp][tid] = (uint8_t)vs;
         } else {
-          l_entry[sp - kPackStack] = e;
-          l_vs[sp - kPackStack] = (uint8_t)vs;
+          local.entry[sp - kPackStack] = e;
+          local.vs[sp - kPackStack] = (uint8_t)vs;
         }
         sp++;
       }
@@ -321,8 +402,8 @@ __device__ __forceinline__ void trace_packed(bool live, const float3 o, const fl
         e = s_entry[sp][tid];
         vs = s_vs[sp][tid];
       } else {
-        e = l_entry[sp - kPackStack];
-        vs = l_vs[sp - kPackStack];
+        e = local.entry[sp - kPackStack];
+        vs = local.vs[sp - kPackStack];
       }
       cur = e.x;
       pop = !(__int_as_float(e.y) < best);
@@ -337,16 +418,23 @@ __device__ __forceinline__ void trace_packed(bool live, const float3 o, const fl
   }
 }
 
+__device__ __forceinline__ void trace_packed(bool live, const float3 o, const float3 d, const PackedTree& T, uint32_t r,
+                                             const HitOut& out) {
+  __shared__ int2 s_entry[kPackStack][kPackThreads];  // reference, entry distance
+  __shared__ uint8_t s_vs[kPackStack][kPackThreads];
+  RayStack local;
+  if (__ldcg(T.packed)) trace_records<true>(live, o, d, T, r, out, s_entry, s_vs, local);
+  else trace_records<false>(live, o, d, T, r, out, s_entry, s_vs, local);
+}
+
 // 20 blocks of 64 threads per SM (48 registers): smaller blocks end as soon as their own rays do.
 __global__ void __launch_bounds__(kPackThreads, 20)
-    k_trace_packed(const Node* __restrict__ nodes, const PackNode* __restrict__ rec, const PackTri* __restrict__ tris,
-                   uint32_t n_tris, RayPtrs rays, uint32_t nr, HitOut out) {
+    k_trace_packed(PackedTree T, GivenRays rays, uint32_t nr, HitOut out) {
   const uint32_t r = blockIdx.x * kPackThreads + threadIdx.x;
   const bool live = r < nr;
-  const uint32_t q = live ? r : nr - 1;
-  const float3 o = make_float3(__ldg(rays.o[0] + q), __ldg(rays.o[1] + q), __ldg(rays.o[2] + q));
-  const float3 d = make_float3(__ldg(rays.d[0] + q), __ldg(rays.d[1] + q), __ldg(rays.d[2] + q));
-  trace_packed(live, o, d, nodes, rec, tris, n_tris, r, out);
+  float3 o, d;
+  rays.get(live ? r : nr - 1, o, d);
+  trace_packed(live, o, d, T, r, out);
 }
 
 // A warp takes two 4x4 pixel tiles from opposite halves of the image: coherent within a tile, and
@@ -355,16 +443,14 @@ __global__ void __launch_bounds__(kPackThreads, 20)
 // tiles of 4x2: 6.8 and 0.35 ms.
 __host__ __device__ inline uint32_t pinhole_tiles(int w, int h) { return div_up((uint32_t)w, 4) * div_up((uint32_t)h, 4); }
 __global__ void __launch_bounds__(kPackThreads, 20)
-    k_trace_pinhole_packed(const Node* __restrict__ nodes, const PackNode* __restrict__ rec,
-                           const PackTri* __restrict__ tris, uint32_t n_tris, PinholeCam cam, HitOut out) {
+    k_trace_pinhole_packed(PackedTree T, PinholeCam cam, HitOut out) {
   const uint32_t warp = (blockIdx.x * kPackThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const uint32_t tiles = pinhole_tiles(cam.width, cam.height), half = div_up(tiles, 2);
   const uint32_t tile = warp + (lane >> 4) * half, across = div_up((uint32_t)cam.width, 4);
   const uint32_t x = (tile % across) * 4 + (lane & 3), y = (tile / across) * 4 + ((lane >> 2) & 3);
   const bool live = warp < half && tile < tiles && x < (uint32_t)cam.width && y < (uint32_t)cam.height;
   const float3 o = make_float3(cam.eye[0], cam.eye[1], cam.eye[2]);
-  trace_packed(live, o, pinhole_dir(cam, (int)x, (int)y), nodes, rec, tris, n_tris,
-               y * (uint32_t)cam.width + x, out);
+  trace_packed(live, o, pinhole_dir(cam, (int)x, (int)y), T, y * (uint32_t)cam.width + x, out);
 }
 
 void trace_pool_free(TracePool& p) {
@@ -372,22 +458,18 @@ void trace_pool_free(TracePool& p) {
   p = TracePool{p.device};
 }
 
-// The records of one trace, on its stream: allocated, filled, and given back by unpack().
-struct Packed {
-  PackNode* rec = nullptr;
-  PackTri* tris = nullptr;
-};
-
-// Whether a trace repacks: repacking costs ~0.025 ns per node and ~10 us of launches; it gains 0.85 ns
-// per ray on the cheapest tree measured (100 visits per ray, 1.3M triangles) and 7 to 14 ns on deep
-// ones.  At 16 nodes per ray and 16,384 rays the least gain is about twice the cost.  Not while the
-// stream is being captured (a graph of the trace stays free of allocations), and where the pool has
-// no room the trace runs on the tree as it is.
-static bool pack(TracePool* tp, const Node* nodes, int n_nodes, const MeshPtrs& m, uint32_t n_tris, uint32_t nr,
-                 cudaStream_t st, Packed* pk) {
+// Whether a trace repacks (if its rays enter the scene: k_pack): repacking costs ~0.025 ns per node and ~10 us of
+// launches; it gains 0.85 ns per ray on the cheapest tree measured (100 visits per ray, 1.3M triangles)
+// and 7 to 14 ns on deep ones.  At 16 nodes per ray and 16,384 rays the least gain is about twice the
+// cost.  Not while the stream is being captured (a graph of the trace stays free of allocations), and
+// where the pool has no room the trace runs on the tree as it is.  T: its records, allocated on the stream,
+// filled there, and given back by unpack().
+template <typename Rays>
+static bool pack(TracePool* tp, const Node* nodes, int n_nodes, const MeshPtrs& m, uint32_t n_tris, const Rays& rays,
+                 uint32_t nr, cudaStream_t st, PackedTree* T) {
   if (!tp || nr < 16384u || n_nodes < 3 || n_tris == 0 || (uint64_t)n_nodes > 16ull * nr) return false;
   const uint64_t node_bytes = (uint64_t)n_nodes * sizeof(PackNode);
-  const uint64_t bytes = node_bytes + (uint64_t)n_tris * sizeof(PackTri);
+  const uint64_t bytes = sizeof(PackNode) + node_bytes + (uint64_t)n_tris * sizeof(PackTri);  // *packed first
   if (bytes > kPackMaxBytes) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   bool ok = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
@@ -408,15 +490,16 @@ static bool pack(TracePool* tp, const Node* nodes, int n_nodes, const MeshPtrs& 
     cudaGetLastError();  // not the caller's error: the trace still runs
     return false;
   }
-  pk->rec = static_cast<PackNode*>(buf);
-  pk->tris = reinterpret_cast<PackTri*>(static_cast<char*>(buf) + node_bytes);
-  k_pack_nodes<<<std::min<uint32_t>(div_up((uint32_t)n_nodes, 256), 152 * 8), 256, 0, st>>>(nodes, n_nodes, pk->rec);
-  k_pack_tris<<<std::min<uint32_t>(div_up(n_tris, 256), 152 * 8), 256, 0, st>>>(m, n_tris, pk->tris);
+  PackNode* rec = static_cast<PackNode*>(buf) + 1;
+  PackTri* tris = reinterpret_cast<PackTri*>(rec + n_nodes);
+  *T = PackedTree{nodes, n_nodes, m, n_tris, rec, tris, static_cast<uint32_t*>(buf)};
+  k_pack<<<std::min<uint32_t>(div_up(std::max((uint32_t)n_nodes, n_tris), 256), 152 * 8), 256, 0, st>>>(
+      nodes, n_nodes, m, n_tris, rays, nr, rec, tris, static_cast<uint32_t*>(buf));
   return true;
 }
-static cudaError_t unpack(const Packed& pk, cudaStream_t st) {
+static cudaError_t unpack(const PackedTree& T, cudaStream_t st) {
   const cudaError_t e = cudaGetLastError();
-  const cudaError_t f = cudaFreeAsync(pk.rec, st);
+  const cudaError_t f = cudaFreeAsync(const_cast<uint32_t*>(T.packed), st);
   return e != cudaSuccess ? e : f;
 }
 
@@ -635,10 +718,12 @@ cudaError_t rgb_to_bytes(const float* rgb, uint32_t nv, uint8_t* out, cudaStream
 cudaError_t trace_rays(const Node* nodes, int n_nodes, const MeshPtrs& m, uint32_t n_tris, const RayPtrs& rays,
                        uint32_t nr, const HitOut& out, TracePool* pool, cudaStream_t st) {
   if (nr == 0) return cudaSuccess;
-  Packed pk;
-  if (pack(pool, nodes, n_nodes, m, n_tris, nr, st, &pk)) {
-    k_trace_packed<<<div_up(nr, kPackThreads), kPackThreads, 0, st>>>(nodes, pk.rec, pk.tris, n_tris, rays, nr, out);
-    return unpack(pk, st);
+  PackedTree T;
+  const GivenRays given{rays};
+  if (pack(pool, nodes, n_nodes, m, n_tris, given, nr, st, &T)) {
+    // (launched plainly: started early, its blocks crowd the first SMs that k_pack leaves, 65,536 rays 448 -> 665 us)
+    k_trace_packed<<<div_up(nr, kPackThreads), kPackThreads, 0, st>>>(T, given, nr, out);
+    return unpack(T, st);
   }
   k_trace<<<div_up(nr, 128), 128, 0, st>>>(nodes, n_nodes, m, n_tris, rays, nr, out);
   return cudaGetLastError();
@@ -708,12 +793,11 @@ cudaError_t trace_pinhole(const Node* nodes, int n_nodes, const MeshPtrs& m, uin
                           const HitOut& out, TracePool* pool, cudaStream_t st) {
   uint32_t total = (uint32_t)cam.width * (uint32_t)cam.height;
   if (total == 0) return cudaSuccess;
-  Packed pk;
-  if (pack(pool, nodes, n_nodes, m, n_tris, total, st, &pk)) {
+  PackedTree T;
+  if (pack(pool, nodes, n_nodes, m, n_tris, PixelRays{cam}, total, st, &T)) {
     const uint32_t warps = div_up(pinhole_tiles(cam.width, cam.height), 2);
-    k_trace_pinhole_packed<<<div_up(warps, kPackThreads / 32), kPackThreads, 0, st>>>(nodes, pk.rec, pk.tris, n_tris,
-                                                                                      cam, out);
-    return unpack(pk, st);
+    k_trace_pinhole_packed<<<div_up(warps, kPackThreads / 32), kPackThreads, 0, st>>>(T, cam, out);
+    return unpack(T, st);
   }
   k_trace_pinhole<<<div_up(total, 128), 128, 0, st>>>(nodes, n_nodes, m, n_tris, cam, out);
   return cudaGetLastError();

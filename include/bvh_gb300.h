@@ -363,8 +363,8 @@ typedef struct bvh_eval_stats {
 bvh_status bvh_evaluate(bvh_ctx* ctx, const bvh_node* nodes, uint32_t n_nodes, void* stream, bvh_eval_stats* out);
 
 /* Closest-hit traversal of explicit rays (device pointers).  Asynchronous.  From 16,384 rays on (and
- * at most 16 nodes per ray) the tree is first repacked on `stream` into 64 bytes per node and per
- * triangle of scratch, which the context keeps for its next trace; where that memory is not to be had,
+ * at most 16 nodes per ray), if any of a sample of the rays enters the root's box, the tree is first
+ * repacked on `stream` into 64 bytes per node and per triangle of scratch, which the context keeps for its next trace; where that memory is not to be had,
  * or `stream` is being captured, the tree is walked as it is.  The hits do not depend on it. */
 bvh_status bvh_trace(bvh_ctx* ctx, const bvh_node* nodes, uint32_t n_nodes, const bvh_mesh_soa* mesh,
                      const bvh_rays* rays, const bvh_hits* hits, void* stream);
