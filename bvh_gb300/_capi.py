@@ -116,6 +116,7 @@ SIGNATURES = {
     "bvh_ctx_destroy": (c_int, [c_void_p]),
     "bvh_ctx_reserve": (c_int, [c_void_p, c_uint32, c_int32]),
     "bvh_ctx_device_bytes": (c_int, [c_void_p, POINTER(c_uint64)]),
+    "bvh_ctx_trim": (c_int, [c_void_p]),
     "bvh_default_params": (Params, [c_int32]),
     "bvh_build_device": (c_int, [c_void_p, POINTER(MeshSoA), POINTER(Params), c_void_p, POINTER(Tree)]),
     "bvh_build_host": (c_int, [c_void_p, POINTER(MeshSoA), POINTER(Params), c_void_p, c_void_p, c_void_p,

@@ -168,6 +168,16 @@ class Context:
     def reserve(self, n: int, algo: int = C.ALGO_LBVH):
         C.check(self.lib.bvh_ctx_reserve(self.handle, n, algo), "bvh_ctx_reserve")
 
+    def device_bytes(self) -> int:
+        """Device memory that the context holds."""
+        b = ctypes.c_uint64(0)
+        C.check(self.lib.bvh_ctx_device_bytes(self.handle, ctypes.byref(b)), "bvh_ctx_device_bytes")
+        return b.value
+
+    def trim(self):
+        """Give back the scratch that large traces leave with the context (waits for the device)."""
+        C.check(self.lib.bvh_ctx_trim(self.handle), "bvh_ctx_trim")
+
     def build_device(self, ptrs: Sequence[int], n: int, params: C.Params, stream: int = 0) -> C.Tree:
         """Build from nine device addresses; asynchronous on `stream` (a cudaStream_t value)."""
         m = C.mesh_struct(ptrs, n)

@@ -146,12 +146,33 @@ extern "C" bvh_status bvh_ctx_destroy(bvh_ctx* ctx) {
   return BVH_OK;
 }
 
+// An allocation of the context; where the device has no room, once more without the traces' kept records.
+template <typename F>
+static cudaError_t with_room(bvh_ctx* ctx, const F& allocate) {
+  cudaError_t e = allocate();
+  if (e == cudaErrorMemoryAllocation && trace_pool_trim(ctx->trace_pool)) {
+    cudaGetLastError();
+    e = allocate();
+  }
+  return e;
+}
+static cudaError_t reserve(bvh_ctx* ctx, uint32_t n, bool ploc, cudaStream_t st) {
+  const cudaError_t e = with_room(ctx, [&] { return workspace_reserve(ctx->ws, n, st); });
+  return e != cudaSuccess || !ploc ? e : with_room(ctx, [&] { return workspace_reserve_ploc(ctx->ws, n); });
+}
+
+extern "C" bvh_status bvh_ctx_trim(bvh_ctx* ctx) {
+  if (!ctx) return BVH_ERR_INVALID_ARG;
+  cudaSetDevice(ctx->device);
+  trace_pool_trim(ctx->trace_pool);
+  return from_cuda(cudaGetLastError());
+}
+
 extern "C" bvh_status bvh_ctx_reserve(bvh_ctx* ctx, uint32_t n, int32_t algo) {
   if (!ctx) return BVH_ERR_INVALID_ARG;
   cudaSetDevice(ctx->device);
   // zero on the legacy stream and wait, so that builds on any stream see the cleared buffers
-  cudaError_t e = workspace_reserve(ctx->ws, n, nullptr);
-  if (e == cudaSuccess && algo == BVH_ALGO_PLOC) e = workspace_reserve_ploc(ctx->ws, n);
+  cudaError_t e = reserve(ctx, n, algo == BVH_ALGO_PLOC, nullptr);
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   return from_cuda(e);
 }
@@ -160,9 +181,12 @@ extern "C" bvh_status bvh_ctx_device_bytes(const bvh_ctx* ctx, uint64_t* bytes) 
   if (!ctx || !bytes) return BVH_ERR_INVALID_ARG;
   const Workspace& w = ctx->ws;
   uint64_t b = 0;
-  if (w.cap_n) b += (uint64_t)w.cap_n * (8 * 2 + 4 * 2 + sizeof(Box) + 2 * sizeof(Node) + 8) + w.scratch_words * 4;
+  if (w.cap_n)  // with the delta bytes and the heights
+    b += (uint64_t)w.cap_n * (8 * 2 + 4 * 2 + sizeof(Box) + 2 * sizeof(Node) + 8 + 1 + 1) + 32 + w.scratch_words * 4;
   if (w.ploc_cap) b += (uint64_t)w.ploc_cap * (2 * sizeof(Box) + 8 + 4) + (w.ploc_cap / 2048 + 8) * 8;
   b += (uint64_t)w.mesh_cap * 36;
+  b += (uint64_t)w.bat_words_cap * 4 + (uint64_t)w.bat_count_cap * 32 + (uint64_t)w.bat_n_cap * 4;
+  b += ctx->eval_bytes + (ctx->heat_buf ? heatmap_scratch_bytes() : 0) + trace_pool_bytes(ctx->trace_pool);
   *bytes = b;
   return BVH_OK;
 }
@@ -244,7 +268,8 @@ static bvh_status build_impl(bvh_ctx* ctx, const bvh_mesh_soa* mesh, const bvh_p
   if (n == 0) return BVH_OK;  // empty mesh: empty tree
   MeshPtrs m = mesh_ptrs(mesh);
   uint32_t* idx = nullptr;
-  cudaError_t e;
+  cudaError_t e = reserve(ctx, n, params->algo == BVH_ALGO_PLOC, st);
+  if (e != cudaSuccess) return from_cuda(e);
   if (params->algo == BVH_ALGO_PLOC) {
     e = ploc_build(ctx->ws, m, n, params->ploc_radius, params->max_iterations, st, &ctx->evs, &idx,
                    params->reserved[1] == BVH_HOST_DRIVEN_LOOPS);
@@ -392,7 +417,7 @@ extern "C" bvh_status bvh_build_host(bvh_ctx* ctx, const bvh_mesh_soa* mesh, con
     ws.mesh_cap = 0;
     // nine arrays, each padded to a multiple of 4 floats so that all stay 16-byte aligned
     size_t stride = ((size_t)n + 3) & ~size_t(3);
-    cudaError_t e = cudaMalloc(&ws.mesh_dev, stride * 9 * sizeof(float));
+    cudaError_t e = with_room(ctx, [&] { return cudaMalloc(&ws.mesh_dev, stride * 9 * sizeof(float)); });
     if (e != cudaSuccess) return from_cuda(e);
     ws.mesh_cap = n;
   }
@@ -547,10 +572,10 @@ extern "C" bvh_status bvh_build_batched(bvh_ctx* ctx, const bvh_batch* batch, co
   apply_tuning(ctx, params->algo + 256, n);
   const uint32_t n_items = count_items(batch->offsets, count);
   const size_t words = items_at(count) + 4 * (size_t)n_items;
-  cudaError_t e = reserve_batch(ws, n, count, words, st);
+  cudaError_t e = with_room(ctx, [&] { return reserve_batch(ws, n, count, words, st); });
   if (e != cudaSuccess) return from_cuda(e);
   if (ploc) {  // everything a capture may not do: allocations, kernel attributes
-    if ((e = workspace_reserve_ploc(ws, n)) != cudaSuccess) return from_cuda(e);
+    if ((e = reserve(ctx, n, true, st)) != cudaSuccess) return from_cuda(e);
     if ((e = ploc_prepare(params->ploc_radius)) != cudaSuccess) return from_cuda(e);
     if (params->reserved[1] == BVH_HOST_DRIVEN_LOOPS && !ws.ploc_host &&
         (e = cudaMallocHost(&ws.ploc_host, 64)) != cudaSuccess)
@@ -631,7 +656,7 @@ extern "C" bvh_status bvh_evaluate(bvh_ctx* ctx, const bvh_node* nodes, uint32_t
     cudaFree(ctx->eval_buf);
     ctx->eval_buf = nullptr;
     ctx->eval_bytes = 0;
-    cudaError_t e = cudaMalloc(&ctx->eval_buf, need);
+    cudaError_t e = with_room(ctx, [&] { return cudaMalloc(&ctx->eval_buf, need); });
     if (e != cudaSuccess) return from_cuda(e);
     ctx->eval_bytes = need;
   }

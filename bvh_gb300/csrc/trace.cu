@@ -458,6 +458,28 @@ void trace_pool_free(TracePool& p) {
   p = TracePool{p.device};
 }
 
+uint64_t trace_pool_bytes(const TracePool& p) {
+  uint64_t bytes = 0;
+  if (p.pool && cudaMemPoolGetAttribute(p.pool, cudaMemPoolAttrReservedMemCurrent, &bytes) != cudaSuccess) bytes = 0;
+  return bytes;
+}
+
+// The pool's memory comes in pieces of 32 MiB; a threshold in the midst of one gives that piece back at every
+// synchronisation.
+constexpr uint64_t kPoolPiece = 32ull << 20;
+static cudaError_t trace_pool_keep(TracePool& p, uint64_t bytes) {
+  p.keep = bytes;
+  uint64_t threshold = (bytes + kPoolPiece - 1) / kPoolPiece * kPoolPiece;
+  return cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &threshold);
+}
+
+bool trace_pool_trim(TracePool& p) {
+  if (trace_pool_bytes(p) == 0) return false;
+  p.recent = p.traces = 0;
+  return trace_pool_keep(p, 0) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess &&
+         cudaMemPoolTrimTo(p.pool, 0) == cudaSuccess;
+}
+
 // Whether a trace repacks (if its rays enter the scene: k_pack): repacking costs ~0.025 ns per node and ~10 us of
 // launches; it gains 0.85 ns per ray on the cheapest tree measured (100 visits per ray, 1.3M triangles)
 // and 7 to 14 ns on deep ones.  At 16 nodes per ray and 16,384 rays the least gain is about twice the
@@ -481,9 +503,13 @@ static bool pack(TracePool* tp, const Node* nodes, int n_nodes, const MeshPtrs& 
     ok = cudaMemPoolCreate(&tp->pool, &props) == cudaSuccess;
     if (!ok) tp->pool = nullptr;
   }
-  if (ok && tp->keep < bytes) {
-    tp->keep = bytes;
-    ok = cudaMemPoolSetAttribute(tp->pool, cudaMemPoolAttrReleaseThreshold, &tp->keep) == cudaSuccess;
+  if (ok) {
+    tp->recent = std::max(tp->recent, bytes);
+    if (tp->keep < bytes) ok = trace_pool_keep(*tp, bytes) == cudaSuccess;
+    if (ok && ++tp->traces == kTraceWindow) {
+      if (tp->recent < tp->keep) ok = trace_pool_keep(*tp, tp->recent) == cudaSuccess && cudaMemPoolTrimTo(tp->pool, tp->recent) == cudaSuccess;
+      tp->recent = tp->traces = 0;
+    }
   }
   void* buf = nullptr;
   if (!ok || cudaMallocFromPoolAsync(&buf, bytes, tp->pool, st) != cudaSuccess) {

@@ -33,14 +33,21 @@ struct ShadeIn {
   const int32_t* vis;
 };
 
-// Stream-ordered scratch of the packed traversal (see trace.cu): a pool of the context's own, made at
-// its first use, which keeps at most one trace's records between calls.
+// Stream-ordered scratch of the packed traversal (see trace.cu): a pool of the context's own, made at its first
+// use, which keeps at most one trace's records between calls (new pages for 1.9 GB cost a trace 4 ms):
+// as many bytes as the largest of the last kTraceWindow to 2 kTraceWindow - 1 traces took, none after a trim.
 struct TracePool {
   int device = 0;
   cudaMemPool_t pool = nullptr;
-  uint64_t keep = 0;  // the pool's release threshold: the largest trace so far
+  uint64_t keep = 0;    // bytes that it keeps (its release threshold, in whole pieces)
+  uint64_t recent = 0;  // the largest trace of this window, and the traces in it
+  uint32_t traces = 0;
 };
+constexpr uint32_t kTraceWindow = 16;
 void trace_pool_free(TracePool& p);
+uint64_t trace_pool_bytes(const TracePool& p);  // device memory that it holds
+// Gives back what no trace is using; waits for the device.  False where it held nothing.
+bool trace_pool_trim(TracePool& p);
 
 // `pool` (may be NULL) lets a trace of enough rays repack the tree first; the hits are the same.
 cudaError_t trace_rays(const Node* nodes, int n_nodes, const MeshPtrs& m, uint32_t n_tris, const RayPtrs& rays,

@@ -170,8 +170,12 @@ bvh_status bvh_ctx_create(bvh_ctx** out, int device);
 bvh_status bvh_ctx_destroy(bvh_ctx* ctx);
 /* Pre-allocate workspace for meshes of up to n triangles (optional; builds grow it). */
 bvh_status bvh_ctx_reserve(bvh_ctx* ctx, uint32_t n, int32_t algo);
-/* Bytes of device memory the context currently holds. */
+/* Bytes of device memory the context currently holds, kept scratch of its traces included. */
 bvh_status bvh_ctx_device_bytes(const bvh_ctx* ctx, uint64_t* bytes);
+/* Give back the scratch that large traces leave with the context (bvh_trace: up to 64 bytes per node and per
+ * triangle of the largest recent tree, 16 GB at most); waits for the device.  The context does so by
+ * itself where an allocation of its own finds no room. */
+bvh_status bvh_ctx_trim(bvh_ctx* ctx);
 
 /* Defaults: LBVH, 30-bit, 1 treelet round, radius 25. */
 bvh_params bvh_default_params(int32_t algo);
@@ -364,8 +368,10 @@ bvh_status bvh_evaluate(bvh_ctx* ctx, const bvh_node* nodes, uint32_t n_nodes, v
 
 /* Closest-hit traversal of explicit rays (device pointers).  Asynchronous.  From 16,384 rays on (and
  * at most 16 nodes per ray), if any of a sample of the rays enters the root's box, the tree is first
- * repacked on `stream` into 64 bytes per node and per triangle of scratch, which the context keeps for its next trace; where that memory is not to be had,
- * or `stream` is being captured, the tree is walked as it is.  The hits do not depend on it. */
+ * repacked on `stream` into 64 bytes per node and per triangle of scratch.  The context keeps the
+ * scratch for its next traces (bvh_ctx_trim gives it back, as do 16 to 31 traces that need less);
+ * where that memory is not to be had, or `stream` is being captured, the tree is walked as it is.
+ * The hits do not depend on it. */
 bvh_status bvh_trace(bvh_ctx* ctx, const bvh_node* nodes, uint32_t n_nodes, const bvh_mesh_soa* mesh,
                      const bvh_rays* rays, const bvh_hits* hits, void* stream);
 /* Primary pinhole rays (generateRay, src/render_engine.cu:155-188) for a width x height
