@@ -14,7 +14,6 @@ from __future__ import annotations
 
 import abc
 import ctypes
-import weakref
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -67,12 +66,26 @@ class TriangleMesh:
 
 class _Lease:
     """What an array handed out by _HostArrays refers to: numpy keeps it as the array's base, so it is gone when
-    the last array, view or buffer of that memory is."""
+    the last array, view or buffer of that memory is, and then gives the memory back."""
 
-    __slots__ = ("__array_interface__", "__weakref__")
+    __slots__ = ("__array_interface__", "_owner", "_piece")
 
-    def __init__(self, piece: np.ndarray, size: int):
-        self.__array_interface__ = dict(piece.__array_interface__, shape=(size,))
+    def __init__(self, owner: "_HostArrays", piece: "_Piece"):
+        self.__array_interface__ = piece.interface
+        self._owner = owner
+        self._piece = piece
+
+    def __del__(self):
+        self._owner._give_back(self._piece)
+
+
+class _Piece:
+    __slots__ = ("memory", "size", "interface")
+
+    def __init__(self, size: int):
+        self.memory = np.empty(size, np.uint8)
+        self.size = size
+        self.interface = self.memory.__array_interface__
 
 
 class _HostArrays:
@@ -80,23 +93,22 @@ class _HostArrays:
     copying a tree into it does, so memory that nobody refers to any more (every array made from it is
     gone) serves the next result.  At most `keep` idle pieces stay, none more than twice as large as asked for.
 
-    A piece is in `_pieces` only while it is idle; the finalizer of its lease puts it back, on whatever thread
-    drops the last reference (append and pop of a list are atomic)."""
+    A piece is in `_pieces` only while it is idle; its lease puts it back, on whatever thread drops the last
+    reference (append and pop of a list are atomic).  take() costs 3 us."""
 
     def __init__(self, keep: int = 2):
         self._keep = keep
         self._pieces: list = []
 
-    @staticmethod
-    def _give_back(pieces: list, keep: int, piece: np.ndarray):
-        pieces.append(piece)
-        while len(pieces) > keep:  # the oldest goes
+    def _give_back(self, piece: _Piece):
+        self._pieces.append(piece)
+        while len(self._pieces) > self._keep:  # the oldest goes
             try:
-                pieces.pop(0)
+                self._pieces.pop(0)
             except IndexError:  # another thread took the rest
                 return
 
-    def _idle(self, need: int) -> Optional[np.ndarray]:
+    def _idle(self, need: int) -> Optional[_Piece]:
         others, found = [], None
         while found is None:
             try:
@@ -116,12 +128,7 @@ class _HostArrays:
         need = count * dtype.itemsize
         if need < 1 << 20:
             return np.empty(count, dtype)
-        piece = self._idle(need)
-        if piece is None:
-            piece = np.empty(need, np.uint8)
-        lease = _Lease(piece, need)
-        weakref.finalize(lease, self._give_back, self._pieces, self._keep, piece).atexit = False
-        return np.asarray(lease).view(dtype)
+        return np.asarray(_Lease(self, self._idle(need) or _Piece(need)))[:need].view(dtype)
 
 
 class Context:
