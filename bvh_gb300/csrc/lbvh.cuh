@@ -56,6 +56,7 @@ struct Workspace {
   // 7.7 ms with plain launches, 9.3 with early ones, 9.9 with small meshes in one block).
   bool alone = true;
   bool no_cooperative = false;          // run no cooperative kernel (their host-driven fallbacks)
+  bool cooperative_refused = false;     // the device has refused one of k_ploc_grid's launches
   uint32_t ploc_key_n = 0;
   int ploc_key_r = 0;
   uint32_t ploc_key_shape = 0;  // nn and merge blocks per SM the cached loop graph was made with

@@ -1661,6 +1661,9 @@ static uint32_t ploc_grid_blocks() {
   return (uint32_t)std::min<long long>((long long)sms * occ, kGridMaxBlocks);
 }
 
+constexpr uint32_t kHostGridMin = 65536;
+constexpr uint32_t kLoopTailPairs = 100000;
+
 // The blocks that a build of n triangles takes of the `all` that fit the GPU.  A cooperative grid starts when all of its
 // blocks have room, so builds in several streams take turns unless their grids fit side by side; and a
 // block has no use for less than 512 clusters or 25,600 pairs to search (20,000 triangles, r = 25: 40 blocks
@@ -1692,13 +1695,19 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
   if ((e = set_tail_smem()) != cudaSuccess) return e;
   // every iteration that makes progress removes at least one cluster, so n bounds the loop
   const uint32_t cap = max_iter > 0 ? (uint32_t)max_iter : n;
-  const uint32_t tail = ploc_tail_threshold(radius, ws.ploc_tail_pairs);
   // k_ploc_grid: from grid_at live clusters down to the tail hand-over (its per-block totals
-  // live in the ballot words)
+  // live in the ballot words).  Where no cooperative kernel runs, its iterations would be driven from the host
+  // (20,000 triangles 890 us); below kHostGridMin the loop graph runs them all (552 us, and a build that only
+  // has the tail can be captured), and the tail takes over earlier, since an iteration of the loop
+  // costs four launches: so it does for radii that k_ploc_grid does not take.
+  const bool cooperative = !ws.no_cooperative && !ws.cooperative_refused;
   const uint32_t grid_blocks = ploc_grid_share(ploc_grid_blocks(), n, radius);
   uint32_t grid_at = 0;
-  if (grid_blocks && radius <= kGridMaxR)
+  if (grid_blocks && radius <= kGridMaxR && (cooperative || n >= kHostGridMin))
     grid_at = std::min<uint32_t>(ws.ploc_grid_max, grid_blocks * kGridPerBlock);
+  uint32_t pairs = ws.ploc_tail_pairs;
+  if (pairs && (!grid_at || !cooperative)) pairs = std::max(pairs, kLoopTailPairs);
+  const uint32_t tail = ploc_tail_threshold(radius, pairs);
   if (grid_at <= tail || n <= tail) grid_at = 0;
   const bool loop = n > 1 && n > std::max(tail, grid_at);  // else the one-launch kernels do every iteration
   const PlocShape sh = ploc_shape(ws);
@@ -1748,12 +1757,13 @@ cudaError_t ploc_build(Workspace& ws, const MeshPtrs& m, uint32_t n, int radius,
       attr[0].val.cooperative = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      e = ws.no_cooperative ? cudaErrorNotSupported : cudaLaunchKernelEx(&cfg, k_ploc_grid, B, radius);
+      e = cooperative ? cudaLaunchKernelEx(&cfg, k_ploc_grid, B, radius) : cudaErrorNotSupported;
       if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
         // no co-resident grid (a client limited to part of the GPU, or asked for): the same
         // iterations as one launch per kernel each, driven from the host, down to the tail
         // hand-over; the loop above stopped at grid_at live clusters or for good
         (void)cudaGetLastError();
+        if (cooperative) ws.cooperative_refused = true;
         if (!ws.ploc_host && (e = cudaMallocHost(&ws.ploc_host, 64)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(B.ctrl + 14, 0, 4, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(ws.ploc_host, B.ctrl, 8 * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
