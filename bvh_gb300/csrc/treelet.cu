@@ -1117,11 +1117,9 @@ cudaError_t treelet_rounds_run(Workspace& ws, uint32_t n, int rounds, cudaStream
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   if (!g_dp_grid[dev]) {
     int per_sm = 0;
-    // Seven blocks of shared memory per SM in place of eight leave L1 the lines that the boxes' loads need while
-    // in flight: one pass over 10M 2,888 us with the default (72% of the memory shared), 2,822 with 58%, 2,716
-    // with the boxes read through L1; twelve blocks in fewer registers took 3,350, all memory shared 3,339.
-    if ((e = cudaFuncSetAttribute(k_tl_dp<kTlMax>, cudaFuncAttributePreferredSharedMemoryCarveout, 58)) != cudaSuccess)
-      return e;
+    // Registers (241) leave k_tl_dp<7> eight blocks per SM; the carve-out that comes with them is 164 KB and leaves L1
+    // the rest for the lines of the boxes' loads.  132 KB, seven blocks, take longer (one pass over 10M 3,836 ->
+    // 3,913 us); all memory shared, or twelve blocks in fewer registers, longer still.
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tl_dp<kTlMax>, kLvThreads, 0)) != cudaSuccess)
       return e;
     g_dp_grid[dev] = std::max(1, per_sm * sms);
