@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import abc
 import ctypes
+import weakref
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -64,71 +65,50 @@ class TriangleMesh:
         return v.min(0), v.max(0)
 
 
-class _Lease:
-    """What an array handed out by _HostArrays refers to: numpy keeps it as the array's base, so it is gone when
-    the last array, view or buffer of that memory is, and then gives the memory back."""
-
-    __slots__ = ("__array_interface__", "_owner", "_piece")
-
-    def __init__(self, owner: "_HostArrays", piece: "_Piece"):
-        self.__array_interface__ = piece.interface
-        self._owner = owner
-        self._piece = piece
-
-    def __del__(self):
-        self._owner._give_back(self._piece)
-
-
-class _Piece:
-    __slots__ = ("memory", "size", "interface")
-
-    def __init__(self, size: int):
-        self.memory = np.empty(size, np.uint8)
-        self.size = size
-        self.interface = self.memory.__array_interface__
-
-
 class _HostArrays:
     """Memory for the arrays that builds return.  The pages of a new 100 MB array cost three times what
     copying a tree into it does, so memory that nobody refers to any more (every array made from it is
     gone) serves the next result.  At most `keep` idle pieces stay, none more than twice as large as asked for.
 
-    A piece is in `_pieces` only while it is idle; its lease puts it back, on whatever thread drops the last
-    reference (append and pop of a list are atomic).  take() costs 3 us."""
+    An array handed out is made over a memoryview, which is no array, so it is itself the base that numpy keeps for
+    all its views; a weak reference to it tells whether the memory is in use.  take() costs a microsecond."""
 
     def __init__(self, keep: int = 2):
         self._keep = keep
-        self._pieces: list = []
+        self._pieces: list = []  # (memoryview, weak reference to the array last made over it)
 
-    def _give_back(self, piece: _Piece):
-        self._pieces.append(piece)
-        while len(self._pieces) > self._keep:  # the oldest goes
+    def _trim(self, _=None):
+        """Drops the oldest idle pieces but `keep`."""
+        pieces = self._pieces
+        idle = [p for p in pieces if p[1]() is None]
+        for p in idle[:max(0, len(idle) - self._keep)]:
             try:
-                self._pieces.pop(0)
-            except IndexError:  # another thread took the rest
-                return
-
-    def _idle(self, need: int) -> Optional[_Piece]:
-        others, found = [], None
-        while found is None:
-            try:
-                piece = self._pieces.pop()
-            except IndexError:
-                break
-            if need <= piece.size <= 2 * need:
-                found = piece
-            else:
-                others.append(piece)
-        self._pieces.extend(reversed(others))
-        return found
+                pieces.remove(p)
+            except ValueError:  # another thread took it
+                pass
 
     def take(self, dtype, count: int) -> np.ndarray:
         """An array of `count` items, uninitialised."""
-        dtype = np.dtype(dtype)
-        need = count * dtype.itemsize
+        need = count * dtype.itemsize if isinstance(dtype, np.dtype) else count * np.dtype(dtype).itemsize
         if need < 1 << 20:
             return np.empty(count, dtype)
-        return np.asarray(_Lease(self, self._idle(need) or _Piece(need)))[:need].view(dtype)
+        pieces, self._pieces = self._pieces, []  # (of two threads, one starts anew)
+        memory = None
+        for k, (m, array) in enumerate(pieces):
+            if need <= m.nbytes <= 2 * need and array() is None:
+                memory = m
+                del pieces[k]
+                break
+        if memory is None:
+            memory = memoryview(np.empty(need, np.uint8))
+        array = np.frombuffer(memory, dtype, count)
+        # one result in use and one idle, two arrays each, are ordinary; beyond that, memory goes when it gets idle
+        many = len(pieces) >= 4
+        pieces.append((memory, weakref.ref(array, self._trim if many else None)))
+        self._pieces = pieces
+        if many:
+            self._trim()
+        return array
 
 
 class Context:
